@@ -165,28 +165,40 @@ int launch_slice_extract_batch(const SliceView* d_views, int number_of_views, lo
 int tensor_sum_available(const SumRequest& req, int form);
 
 // One job of the persistent tensor-core kernel: a separable group summed over
-// a lattice of rows (a, b) and columns c >= 0 into its work items' slots.  Its
+// row representatives (a, b) and columns c into its work items' slots.  Its
 // work items are (split ks, m tile, n tile), local index (ks * n_mtiles +
 // m_tile) * n_ntiles + n_tile.  Device-resident.
 //
-// Frequencies: a = a_idx + a_base, b = b_idx + b_base, c = c_idx + c_base.
-// A group's planes c < Kz/2 are one job (a_base = -Kx/2, b_base = -Ky/2,
-// c_base = 0).  Its Nyquist plane c = Kz/2 is two transposed jobs over the
-// same particles with x and z exchanged, so that their one row index a_idx = 0
-// carries the frequency of z and their columns the frequencies of x:
-//   a >= 0: a_base = Kz/2, rows b (b_base = -Ky/2), columns 0 .. Kx/2 - 1;
-//   a < 0:  F(a, b, Kz/2) = conj F(-a, -b, -Kz/2), so a_base = -Kz/2, rows
-//           b' = -b (b_base = 1 - Ky/2), columns -a = 1 .. Kx/2 (c_base = 1).
-// Every column frequency is >= 0: the B chains only rise.
+// With A = w gx gy e^{-i alpha} the row factor of a particle and B = gz
+// e^{-i beta} its column factor, the four real products (Re A, Im A) x (Re B,
+// Im B) give two elements of the spectrum, A B and conj(A) B:
+//   plus  = (cc - ss) + i (cs + sc),   minus = (cc + ss) + i (cs - sc).
+// So a job holds half of its row lattice, each representative as a Re row and
+// an Im row of the MMA, and one real K entry per particle: two real
+// multiply-adds per element, where a complex product takes four.  conj(A) is
+// the row factor at the point mirrored in the centre of the row lattice:
+//   - groups of pure phases are mirrored in (-1/2, -F/2), the middle of the
+//     lattice a in [-Kx/2, Kx/2), b in [-Ky/2, Ky/2) (rows F apart): the half
+//     step's phase is added to every row and taken back by the columns (offa,
+//     offb of the particle constants), and the representatives are a >= 0,
+//     with mirrors (-1 - a, -F - b + bl) for every b offset bl;
+//   - Gaussian factors are even about 0 only: representatives a = 0 .. Kx/2,
+//     mirrors (-a, -b); a = Kx/2 is there for its mirror -Kx/2, and b = -Ky/2
+//     has no mirror on the lattice, so the elements (a < 0, -Ky/2) come from a
+//     job of their own (the face: rows a, columns c, y fixed).
+//
+// Frequencies: a = a_idx + a_base, b = F b_idx + b_base, c = c_idx + c_base.
+// The Nyquist plane c = Kz/2 is one more job over rows b (with their mirrors)
+// and columns a in [-Kx/2, Kx/2), z's fixed frequency joining the offsets.
 //
 // B-operand images: where a job's B stages are read by many m-tiles, they are
 // computed once (tc_bimg_kernel) into `bimg` in the exact swizzled layout of
-// the stage buffer, [n_tile][CTA half][32-particle block][img_stride bytes],
+// the stage buffer, [n_tile][CTA half][64-particle block][img_stride bytes],
 // each image its hi rows then its lo rows (2 x 2 bnc rows of 128 bytes), and
 // the loader copies them; otherwise (bimg null) producer warps compute them
 // per stage.
 struct TcJob {
-    const unsigned char* blocks;  // the job's per-particle constants, 32-particle blocks
+    const unsigned char* blocks;  // the job's per-particle constants, 64-particle blocks
     // Item results: each work item owns slot [local item * slot_stride ..] of
     // `slots`: per CTA of the item (rank r at r * 128 * 2 nc_tile elements)
     // its 128 rows of every accumulator column n.  A job whose items span at
@@ -201,17 +213,19 @@ struct TcJob {
     int n_splits;     // particle chunks (items per tile)
     int ctas;         // 2 for the CTA-pair tiles
     double wmax;
-    int kx, ky, lz_tc;  // row extents (a_idx < kx, b_idx < ky); columns c_idx < lz_tc
+    int kx, ky, lz_tc;  // representatives (a_idx < kx, b_idx < ky); columns c_idx < lz_tc
     int n_mtiles, n_ntiles;
     int n;        // particles
-    int k_chunk;  // particles per item (multiple of 32)
+    int flush;    // pipeline stages (64 particles) per TMEM accumulation chain
+    int unit_col; // column 0's factors are exactly 1 (frequency 0, no offset: a Gaussian group's planes)
+    int k_chunk;  // particles per item (multiple of 64)
     int gauss;    // per-particle Gaussian factors (GAUSSIAN_DECAYING with radii)
     int nc_tile;  // c values per n-tile (a multiple of 8; the last tile may be narrower)
     int a_base;   // frequency of row index a_idx = 0
-    int b_base;   // frequency of row index b_idx = 0 (-Ky/2 or 1 - Ky/2: 8-row chunks never hold both signs)
-    int c_base;   // frequency of column c_idx = 0 (>= 0)
+    int b_base;   // frequency of row index b_idx = 0 (0 or -Ky/2: Gaussian 8-row chunks never hold both signs)
+    int c_base;   // frequency of column c_idx = 0 (0 or -Kx/2: Gaussian 8-column chunks never hold both signs)
     const unsigned char* bimg;  // B-operand images, or null
-    int n_blocks;    // 32-particle blocks
+    int n_blocks;    // 64-particle blocks
     int img_stride;  // bytes per image: 512 x (c values per CTA of a full n-tile)
     // h-binned jobs (period > 0): the job's lz_tc = P x period columns are P
     // blocks of `period` frequency columns, block q weighted on the B side by
@@ -236,14 +250,29 @@ struct TcJob {
     // (N = 256 instead of 64 or 128 on small lattices) and less A work per
     // term.  0 or 1: no fold.
     int fold;
-    // Axis-exchanged jobs (exch = 1; groups whose amplitudes separate per
-    // axis, on lattices with more b values than tensor planes): rows (a,
-    // c_idx) with ky = the planes Kz/2 and b_base = 0, columns b_idx with
-    // lz_tc = Ky and c_base = -Ky/2 (B chains of negative b fall away from
-    // 0); the particle constants carry y and z exchanged.  192 planes with
-    // Ky = 384 then run 3 n-tiles of 128 b values (N = 256 MMAs) instead of
-    // two of 96 planes.
+    // Axis-exchanged jobs (exch = 1; Gaussian groups on lattices with more b
+    // values than tensor planes): rows (a, c_idx) with ky = the planes Kz/2
+    // and b_base = 0, all a, columns b_idx < Ky/2; the particle constants
+    // carry y and z exchanged.  The mirror is along the columns instead: A
+    // conj(B) is the element (a, -b, c), and b = -Ky/2 comes from the face job.
+    // 256 x 256 x 64 then runs N = 256 MMAs over 128 b values instead of N =
+    // 64 over 32 planes.
     int exch;
+};
+
+// How the jobs of one part of an output class lie in the spectrum
+// (tc_reduce_kernel; TcJob).
+enum TcPartKind : int { kPartPlanes = 0, kPartExchanged = 1, kPartNyquist = 2, kPartFace = 3 };
+struct TcPart {
+    int kind;
+    int n_reps;   // row representatives
+    int rows;     // b_idx values per a_idx
+    int fold, a_base, b_base, c_base;
+    int columns;  // frequency columns per block
+    int mirror_a, mirror_b;  // the mirror's frequencies: mirror - frequency
+    int min_minus;   // smallest mirrored frequency (a, exchanged: b, else the row) whose mirror is stored
+    int write_plus;  // whether the representatives themselves are stored
+    int fixed;       // Nyquist: z's frequency; face: y's
 };
 
 // The h-bins of one binned group on one lattice (tensor_plan): consecutive
@@ -291,10 +320,13 @@ struct TensorPlan {
         double h;
         bool factored;
         double scale;
-        bool nyquist;  // the Nyquist plane is summed by the groups' transposed jobs
-        // the class's jobs (indices into jobs): planes, Nyquist a >= 0, Nyquist a < 0
-        std::vector<int> jobs, nyq_pos, nyq_neg;
-        size_t list_offset = 0;  // those three lists in meta (ints)
+        // the class's parts: planes, Nyquist plane, face (those with jobs)
+        struct Part {
+            TcPart geometry;
+            std::vector<int> jobs;   // indices into TensorPlan::jobs
+            size_t list_offset = 0;  // that list in meta (ints)
+        };
+        Part parts[3];
     };
     std::vector<TcJob> jobs;
     std::vector<int2> items;  // 128x128-tile items (n_narrow), narrow CTA-pair items (n_pair_narrow),
@@ -302,10 +334,10 @@ struct TensorPlan {
     int n_narrow = 0, n_pair_narrow = 0, n_pair = 0, n_pair_db = 0;
     std::vector<Class> classes;
     std::vector<int> group_class, job_of_group;
-    std::vector<int> nyq_job_of_group;  // the transposed Nyquist-plane jobs (a >= 0 here, a < 0 next), or -1
+    std::vector<int> nyq_job_of_group;  // the Nyquist-plane job (h-binned: the first bin's), or -1
+    std::vector<int> face_job_of_group; // Gaussian groups: the b = -Ky/2 job, or -1
     std::vector<int> group_binned;      // index into binned, or -1
     // per job: its particle constants (offset into the particles workspace),
-    // accumulator class and part (0 planes, 1 Nyquist a >= 0, 2 Nyquist a < 0),
     // coefficient table (offset in floats into coef, SIZE_MAX for none)
     std::vector<size_t> job_tp, job_coef, job_slot;  // job_slot: byte offset into slots
     std::vector<size_t> job_colmap;                 // the job's column map: index into colmaps
@@ -314,16 +346,13 @@ struct TensorPlan {
     std::vector<int> img_jobs;                      // the jobs with B-operand images
     std::vector<long long> img_first;               // their first images (and the total last)
     size_t img_jobs_offset = 0, img_first_offset = 0;  // both in meta
-    std::vector<int> job_class, job_acc;
     size_t slot_bytes = 0;
-    std::vector<size_t> tp_offset, tp_nyq_offset;
+    std::vector<size_t> tp_offset, tp_nyq_offset;  // per group: particle constants, the Nyquist jobs'
     std::vector<size_t> bimg_offset;  // per job: its B-operand images in the workspace, or SIZE_MAX
     size_t bimg_bytes = 0;
     size_t tp_bytes = 0, meta_bytes = 0;
     const void* d_jobs = nullptr;
     const void* d_items = nullptr;
-    int flush = 16;        // stages per TMEM accumulation chain of the kWide / kPair tiles, as planned
-    int flush_narrow = 8;  // the same for the kNarrow tile
 };
 
 struct TensorWorkspace {

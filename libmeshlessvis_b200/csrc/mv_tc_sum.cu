@@ -21,18 +21,23 @@
 // lattices with more b values than planes exchange the axes (rows (a, c),
 // columns b; TcJob::exch).
 //
-// Real embedding with re/im interleaved along K (k = 2j + {0,1}):
-//   A'[m, 2j..2j+1] = (Re A, Im A),  B'_re[2j..2j+1, n] = (Re B, -Im B),
-//   B'_im[2j..2j+1, n] = (Im B, Re B);  C = A' [B'_re | B'_im] = [Re F | Im F].
+// Real rows.  The operands hold the real and imaginary parts of A and of B as
+// rows of their own, one K entry per particle, and the four real products give
+// two elements of the spectrum, A B and conj(A) B (TcJob): half the row
+// lattice covers all of it, at two real multiply-adds per element.  The
+// complex embedding this replaces (re and im interleaved along K, four
+// multiply-adds per element) took 167 ms on 2^20 Gaussians and 256^3, this
+// form 84 ms; 38.4 and 20.1 ms on 16 particle sets of 64^3 to 192^3.
 // Split precision: operands are scaled by 2^12 (exact) and split as
 // x 2^12 = hi + lo with hi, lo FP16; the scale keeps lo a normal FP16 number
 // for every |x| >= 2^-15 (below that the absolute error is < 2^-36).  The three
 // products hi*hi + hi*lo + lo*hi (error ~2^-22 relative) accumulate into ONE
-// TMEM accumulator (FP32, units of 2^24; 256 columns).  Every flush_stages
-// stages (a chain of flush_stages x 12 MMAs; the tensor core's FP32
-// accumulation loses accuracy with chain length: 1.6e-6 rel-L2 at 4 stages,
-// 2.4e-6 at 8, 4.1e-6 at 16) the MMA pauses while the flush warps add the
-// accumulator into an FP32 total in the other 256 TMEM columns.  A work item
+// TMEM accumulator (FP32, units of 2^24; 256 columns).  Every TcJob::flush
+// stages (a chain of 12 MMAs a stage) the MMA pauses while the flush warps add
+// the accumulator into an FP32 total in the other 256 TMEM columns, with the
+// mean of what the tensor core's truncation took from it (kChainGain: the
+// error then does not grow with the chain as it did, 4.1e-6 rel-L2 at 16
+// stages; now 0.4-1.5e-6 at the 8 and 16 stages in use).  A work item
 // (one particle range of one tile) owns a slot of global memory: at its end
 // an item of at most kMaxItemChains chains stores its FP32 total there once,
 // and a longer item adds its FP32 total of every kMaxItemChains chains into
@@ -43,26 +48,25 @@
 // spectrum, so results are bitwise reproducible.
 //
 // The Nyquist plane c = Kz/2 is the same kind of GEMM with the axes
-// exchanged: rows b with the fixed frequency Kz/2 on z, columns a on x (two
-// jobs, a >= 0 and, by F(-a, b, c) = conj F(a, -b, -c), a < 0; see TcJob), so
-// it runs as 1/Kx of the other planes' tiles in the same launch instead of a
-// plain-form pass.
+// exchanged: rows b, columns a, the fixed frequency Kz/2 on z in the phase
+// offsets (see TcJob), so it runs as about 1/Kx of the other planes' tiles
+// instead of a plain-form pass; likewise the Gaussians' face b = -Ky/2.
 //
-// CTA tile: M = 128 rows (a, b) (8-row chunks of constant a), N = up to 128 c
-// values (256 real columns), K = 32 particles (64 real) per pipeline stage;
-// CTA pairs run M = 256 over both CTAs (tile kinds and operand rings at
-// TileMode and Shape below).
+// CTA tile: M = 128 rows (the Re and Im rows of 64 representatives (a, b), in
+// 8-row chunks of constant a), N = up to 128 c values (256 real columns), K =
+// 64 particles per pipeline stage; CTA pairs run M = 256 over both CTAs (tile
+// kinds and operand rings at TileMode and Shape below).
 // Warp roles:
 //   warp 0       allocates TMEM, one thread issues tcgen05.mma / commit;
 //   warps 1-4    flush TMEM (warp w reads lanes 32 (w % 4) .. +31);
 //   warps 5-16   generate operands straight into shared memory (8 warps of A
-//                row chunks, 4 of B c chunks, two chunks per thread) in the
-//                128-byte swizzled K-major layout (one 128-byte row of 64 FP16
-//                per operand row and stage; the swizzle lets the tensor core
-//                read at full rate and keeps the stores free of bank
-//                conflicts), by recurrences along b and
-//                c (8 steps from an exact fixed-point start, moving away from
-//                the axis origin so Gaussian factors only shrink along a chain);
+//                chunks, one each, 4 of B c chunks) in the 128-byte swizzled
+//                K-major layout (one 128-byte row of 64 FP16 per operand row
+//                and stage; the swizzle lets the tensor core read at full
+//                rate; a warp's 32 particle pairs store one whole row at a
+//                time, free of bank conflicts), by recurrences along b and
+//                c (8 steps from an exact fixed-point start; Gaussian chains
+//                move away from the axis origin so their factors only shrink);
 //   warp 17      lane 0 streams the per-particle constants of each stage into
 //                shared memory with cp.async.bulk (global -> own CTA, no
 //                multicast), up to the pipeline depth ahead; lane 1, once the
@@ -70,7 +74,7 @@
 //                jobs with B-operand images together with the bulk copy of the
 //                stage's B image (the B warps then idle).
 // Per-particle constants (fixed-point positions, unit rotations, Gaussian
-// ratios) are computed once per launch by tc_prep_kernel into 32-particle
+// ratios) are computed once per launch by tc_prep_kernel into 64-particle
 // field-by-field blocks.  B-operand images (the B stages of a job whose m-tiles
 // all read the same ones) are computed once per launch by tc_bimg_kernel, with
 // the producers' own arithmetic, and read from L2 by every m-tile.
@@ -102,29 +106,35 @@
 namespace mv {
 
 // Per-particle constants of one group, computed once per launch by
-// tc_prep_kernel, in blocks of 32 particles laid out field by field (1280
+// tc_prep_kernel, in blocks of 64 particles laid out field by field (3072
 // bytes per block) so that a producer reads the constants of its particle
 // pair with conflict-free 64-bit shared-memory loads, and the loader moves one
 // whole block per pipeline stage:
-//   qx[32], qy[32], qz[32]  u32 fixed-point turns of step * position
-//   amp[32]                 2^12 w / W
-//   gam[32]                 -pi log2(e) step^2 h^2 (GAUSSIAN_DECAYING), else 0
-//   rho2[32]                exp2(2 gam): ratio of successive Gaussian step factors
-//   ry[32], rz[32]          float2 exp(-2 pi i Q / 2^32), accurate
+//   qx[64], qy[64], qz[64]  u32 fixed-point turns of step * position (row a,
+//                           row b and column axes of the job)
+//   amp[64]                 2^12 w / W
+//   gam[64]                 -pi log2(e) step^2 h^2 (GAUSSIAN_DECAYING), else 0
+//   rho2[64]                exp2(2 gam): ratio of successive Gaussian step factors
+//   offa[64], offb[64]      u32 turns added to every row and column phase
+//   ry[64], rz[64]          float2 exp(-2 pi i Q / 2^32), accurate
 // Particles past the group's end (up to the block boundary) have amp = 0.
-constexpr int kBlockParticles = 32;
-constexpr int kBlockBytes = 6 * 4 * kBlockParticles + 2 * 8 * kBlockParticles;  // 1280
-constexpr int kOffQx = 0, kOffQy = 128, kOffQz = 256, kOffAmp = 384, kOffGam = 512, kOffRho2 = 640, kOffRy = 768,
-              kOffRz = 1024;
+constexpr int kBlockParticles = 64;
+constexpr int kFieldBytes = 4 * kBlockParticles;
+constexpr int kBlockBytes = 8 * kFieldBytes + 2 * 2 * kFieldBytes;  // 3072
+constexpr int kOffQx = 0, kOffQy = kFieldBytes, kOffQz = 2 * kFieldBytes, kOffAmp = 3 * kFieldBytes,
+              kOffGam = 4 * kFieldBytes, kOffRho2 = 5 * kFieldBytes, kOffOa = 6 * kFieldBytes,
+              kOffOb = 7 * kFieldBytes, kOffRy = 8 * kFieldBytes, kOffRz = 10 * kFieldBytes;
 
 namespace {
 
 constexpr int kM = 128;
-constexpr int kKp = 32;
-constexpr int kKr = 2 * kKp;
+constexpr int kReps = kM / 2;  // row representatives of a CTA tile: a cos and a sin row each
+constexpr int kKp = kBlockParticles;
+constexpr int kKr = kKp;       // one real K entry per particle
 constexpr int kRowBytes = 2 * kKr;                 // one operand row: 64 FP16 along K = one 128-byte swizzle row
 constexpr int kAtomBytes = 8 * kRowBytes;           // 8-row swizzle atom
-constexpr int kABytes = kM * kRowBytes;             // A operand: 128 rows
+constexpr int kABytes = kM * kRowBytes;             // A operand: 128 rows (64 cos rows, then their 64 sin rows)
+constexpr int kSinGap = kReps * kRowBytes;          // from a representative's cos row to its sin row
 constexpr int kSlotBytes = kBlockBytes;            // particle constants of one stage
 constexpr int kProducerWarps = 12;  // 8 warps of A units + 4 warps of B units
 constexpr int kFlushWarps = 4;
@@ -134,6 +144,17 @@ constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kColTotal = 256;  // FP32 total: columns [256, 256 + accumulator columns)
 constexpr float kOperandScale = 4096.f;                     // 2^12 per operand
 constexpr double kInvProductScale = 1.0 / (4096.0 * 4096.0);  // 2^-24
+// The tensor core's FP32 accumulation truncates toward zero, so a chain's total
+// comes out low by a part that grows with the chain: per 64 particles 2.1e-7
+// of the total where the terms' phases are random, up to 4.3e-7 where they
+// agree and the total approaches the number of particles (the spectrum near
+// its peak), measured against FP64 on 64^3 and 128^3 (uniform and clustered
+// sets of 2^12 to 2^18 particles, chains of 2 to 32 stages).  The flush adds
+// it back: a part kChainGain per particle, growing with |total| / (particles
+// x operand scale^2) up to kChainGainMost times that.  A unit column (the
+// frequency 0 of a Gaussian job's columns, whose factors are exactly 1, so
+// that many low bits are 0) loses 0.8e-7: kChainGainUnit.
+constexpr float kChainGain = 2.1e-7f / 64, kChainAgree = 4.f, kChainGainMost = 2.f, kChainGainUnit = 0.4f;
 // An FP32 total in TMEM sums at most this many accumulation chains (random-walk
 // rounding of about 2^-24 sqrt(64) of the total) before it goes to the item's
 // slot.
@@ -145,11 +166,10 @@ constexpr unsigned long long kWaitLimitNs = 2000000000ull;
 constexpr unsigned long long kAbortGraceNs = 200000ull;
 
 // Tile kinds (template parameter MODE):
-//   kNarrow (lattices with at most 64 tensor planes): 128x128 MMA, two
-//       alternating 128-column TMEM accumulators (the MMAs never wait for a
-//       flush), 3 stages of 64 KB;
+//   kNarrow (at most 64 columns): 128x128 MMA, two alternating 128-column
+//       TMEM accumulators (the MMAs never wait for a flush);
 //   kWide: 128x256 MMA, one 256-column accumulator (the MMA waits while a
-//       flush reads it), 2 stages of 96 KB;
+//       flush reads it), two stages of each operand;
 //   kPair: a CTA pair (cluster of 2) runs one 256x256 MMA (tcgen05
 //       cta_group::2): each CTA holds 128 rows of A and the B rows of half the
 //       n-tile's c values, and its 128 accumulator rows of all 256 columns in
@@ -180,14 +200,13 @@ struct Shape {
     static constexpr int kN = narrow_mode(MODE) ? 128 : 256;  // accumulator columns: the MMA's N at most
     static constexpr int kNc = kN / 2;                       // c values per n-tile (at most)
     static constexpr int kBRows = kN / kCtas;                // B operand rows held by one CTA
-    static constexpr int kMTile = kM * kCtas;                // lattice rows per m-tile
-    // Rings: A operands (kAStages), B operands (kBStages: deeper where B may
-    // come as a copied image, whose copy starts only once the MMA has read
-    // the B buffer it overwrites), particle constants (kSlots).  One full
-    // barrier per stage, in a ring as deep as the deeper operand ring (an
-    // arrival for stage S + kFull then waits for the MMA to be past stage S).
-    static constexpr int kAStages = 3;
-    static constexpr int kBStages = MODE == kWide ? 2 : 4;
+    static constexpr int kMTile = kReps * kCtas;             // row representatives per m-tile
+    // Rings: A operands (kAStages), B operands (kBStages), particle constants
+    // (kSlots).  One full barrier per stage, in a ring as deep as the deeper
+    // operand ring (an arrival for stage S + kFull then waits for the MMA to
+    // be past stage S).
+    static constexpr int kAStages = MODE == kWide ? 2 : 3;
+    static constexpr int kBStages = MODE == kWide ? 2 : 3;
     static constexpr int kSlots = 2;
     static constexpr int kFull = kAStages > kBStages ? kAStages : kBStages;
     static constexpr bool kDB = MODE == kPairDB;              // totals in the slot, no TMEM total
@@ -195,7 +214,7 @@ struct Shape {
     static constexpr int kBBytes = kBRows * kRowBytes;
     static constexpr int kAStageBytes = 2 * kABytes;  // A_hi, A_lo
     static constexpr int kBStageBytes = 2 * kBBytes;  // B_hi, B_lo (2 bnc rows each, packed)
-    static constexpr int kChunksPerThread = kBRows > 128 ? kBRows / 128 : 1;  // 8-c chunks per B producer thread
+    static constexpr int kChunksPerThread = kBRows / (2 * 8 * 4);  // 8-c chunks per B producer warp
     static constexpr size_t kBOffset = (size_t)kAStages * kAStageBytes;
     static constexpr size_t kSlotOffset = kBOffset + (size_t)kBStages * kBStageBytes;
     static constexpr size_t kBarrierOffset = kSlotOffset + (size_t)kSlots * kSlotBytes;
@@ -215,7 +234,6 @@ struct TcArgs {
     const TcJob* jobs;
     const int2* items;  // (job, local item), longest first
     int n_items;
-    int flush_stages;  // stages per TMEM accumulation chain (12 MMAs each)
     int* error_flag;
     unsigned long long wait_limit_ns;  // bound of every mbarrier wait (kWaitLimitNs unless a test shortens it)
     int withhold_first_arrival;        // test hook: CTA 0's loader skips its arrival on the first full barrier
@@ -227,12 +245,14 @@ struct TcItem {
     int m_tile, n_tile;
     int kb, ke;
     int n_stages, n_chunks;
+    int flush;     // stages per TMEM accumulation chain (12 MMAs each)
     int c0, nc;    // the n-tile's first c and c values (a multiple of 8); the MMA's N is 2 nc
     int bc0, bnc;  // the c values whose B rows this CTA produces: all of them, or one half (kPair)
-    int row0;      // this CTA's first lattice row
+    int row0;      // this CTA's first row representative
     int a_base, b_base, c_base;  // the job's frequency offsets, in registers for the stage loops
     int period;                  // h-binned or row-folded job: frequency columns per column block (else 0)
     int fold;                    // row-folded job: b steps per row (TcJob::fold), else 1
+    bool unit_col;               // accumulator column 0 holds column factors of exactly 1 (TcJob::unit_col)
     const unsigned char* bimg;   // this CTA's B-operand images of the item's n-tile (one per block), or null
     int img_stride, img_bytes;   // bytes between images; bytes of one image (512 bnc)
     void* slot;                  // this CTA's part of the item's slot (TcJob::slots)
@@ -252,17 +272,19 @@ __device__ __forceinline__ TcItem tc_item(const TcArgs& a, int it, int rank) {
     r.kb = ks * r.job->k_chunk;
     r.ke = min(r.job->n, r.kb + r.job->k_chunk);
     r.n_stages = max(0, (r.ke - r.kb + kKp - 1) / kKp);
-    r.n_chunks = (r.n_stages + a.flush_stages - 1) / a.flush_stages;
+    r.flush = r.job->flush;
+    r.n_chunks = (r.n_stages + r.flush - 1) / r.flush;
     r.c0 = r.n_tile * r.job->nc_tile;
     r.nc = min(r.job->nc_tile, r.job->lz_tc - r.c0);
     r.bnc = r.nc / Shape<MODE>::kCtas;
     r.bc0 = r.c0 + rank * r.bnc;
-    r.row0 = r.m_tile * Shape<MODE>::kMTile + rank * kM;
+    r.row0 = r.m_tile * Shape<MODE>::kMTile + rank * kReps;
     r.a_base = r.job->a_base;
     r.b_base = r.job->b_base;
     r.c_base = r.job->c_base;
     r.period = r.job->period;
     r.fold = r.job->fold > 1 ? r.job->fold : 1;
+    r.unit_col = r.job->unit_col && r.n_tile == 0;
     r.img_stride = r.job->img_stride;
     r.img_bytes = 4 * r.bnc * kRowBytes;
     r.bimg = r.job->bimg ? r.job->bimg + (size_t)(r.n_tile * Shape<MODE>::kCtas + rank) * r.job->n_blocks *
@@ -486,16 +508,13 @@ __device__ __forceinline__ float2 unit_phase(uint32_t q) {
 __device__ __forceinline__ uint32_t h2_bits(__half2 h) { return *reinterpret_cast<const uint32_t*>(&h); }
 
 // A producer's two particles as packed pairs: X = (Re z0, Re z1), Y = (Im z0,
-// Im z1), already scaled by 2^12.  split_pair: FP16 hi and lo of (Re, Im) for
-// each particle (x: particle 0, y: particle 1); the residuals are packed FMAs.
-__device__ __forceinline__ void split_pair(float2 X, float2 Y, uint2& hi, uint2& lo) {
-    const __half2 h0 = __floats2half2_rn(X.x, Y.x), h1 = __floats2half2_rn(X.y, Y.y);
-    const float2 f0 = __half22float2(h0), f1 = __half22float2(h1);
-    const float2 m1 = make_float2(-1.f, -1.f);
-    const float2 dx = __ffma2_rn(make_float2(f0.x, f1.x), m1, X);
-    const float2 dy = __ffma2_rn(make_float2(f0.y, f1.y), m1, Y);
-    hi = make_uint2(h2_bits(h0), h2_bits(h1));
-    lo = make_uint2(h2_bits(__floats2half2_rn(dx.x, dy.x)), h2_bits(__floats2half2_rn(dx.y, dy.y)));
+// Im z1), already scaled by 2^12.  split_two: FP16 hi and lo of one such pair
+// (the two particles are neighbours along K); the residual is a packed FMA.
+__device__ __forceinline__ void split_two(float2 V, uint32_t& hi, uint32_t& lo) {
+    const __half2 h = __floats2half2_rn(V.x, V.y);
+    const float2 d = __ffma2_rn(__half22float2(h), make_float2(-1.f, -1.f), V);
+    hi = h2_bits(h);
+    lo = h2_bits(__floats2half2_rn(d.x, d.y));
 }
 
 // One step of both particles' chains: z <- z R, with R = (RX, RY) (NRY =
@@ -515,46 +534,19 @@ __device__ __forceinline__ void rotate_pair(float2& X, float2& Y, float2& RX, fl
     }
 }
 
-__device__ __forceinline__ uint32_t h2_swap_negate(uint32_t h, bool negate_second) {
-    // (re, im) -> (re, -im) when negate_second, else (im, re)
-    if (negate_second) return h ^ 0x80000000u;
-    return (h >> 16) | (h << 16);
-}
-
 // Swizzled offsets: row r (a multiple of 8 plus K, K < 8) of an operand,
-// pair column col = 8 pp: r * 128 + ((col >> 4) ^ K) * 16 + (col & 15).  With
+// pair column col = 4 pp: r * 128 + ((col >> 4) ^ K) * 16 + (col & 15).  With
 // base = 128 * (r - K) + (col & 15) and c16 = col & ~15 fixed per thread, a
-// chain's step K adds K * 128 + (c16 ^ 16 K): one XOR and one add per step.
+// chain's step K adds K * 128 + (c16 ^ 16 K): one XOR and one add per step.  A
+// warp's 32 pairs fill one 128-byte row per store.
 __device__ __forceinline__ int sw_step(int c16, int K) { return K * kRowBytes + (c16 ^ (K << 4)); }
 
-// An A unit's 8 rows for its two particles (b moving away from 0: K = i when
-// UP, 7 - i otherwise), from the chain start (X, Y); lo goes kABytes after hi.
+// A unit's 8 chain steps for its two particles (away from 0: K = i when UP,
+// 7 - i otherwise), from the chain start (X, Y): Re to the row at re_base, Im
+// to the row at im_base; lo goes lo_gap after hi.
 template <bool GAUSS, bool UP>
-__device__ __forceinline__ void a_chain(uint8_t* base, int c16, float2 X, float2 Y, float2 RX, float2 RY, float2 NRY,
-                                        float2 Q, float2 RHO) {
-    if constexpr (GAUSS) {  // the first step's ratio q0 = Q
-        RX = __fmul2_rn(RX, Q);
-        RY = __fmul2_rn(RY, Q);
-        NRY = __fmul2_rn(NRY, Q);
-    }
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        uint8_t* p = base + sw_step(c16, UP ? i : 7 - i);
-        uint2 hi, lo;
-        split_pair(X, Y, hi, lo);
-        *reinterpret_cast<uint2*>(p) = hi;
-        *reinterpret_cast<uint2*>(p + kABytes) = lo;
-        if (i < 7) rotate_pair<GAUSS>(X, Y, RX, RY, NRY, RHO);
-    }
-}
-
-// A B unit's 8 c values for its two particles: (Re B, -Im B) at re_base (a
-// Re F row), (Im B, Re B) at im_base (the Im F row); lo goes lo_gap after hi.
-// UP: the chain starts at the unit's first column and rises; otherwise it
-// starts at the last and falls (negative frequencies, moving away from 0).
-template <bool GAUSS, bool UP>
-__device__ __forceinline__ void b_chain(uint8_t* re_base, uint8_t* im_base, int lo_gap, int c16, float2 X, float2 Y,
-                                        float2 RX, float2 RY, float2 NRY, float2 Q, float2 RHO) {
+__device__ __forceinline__ void unit_chain(uint8_t* re_base, uint8_t* im_base, int lo_gap, int c16, float2 X, float2 Y,
+                                           float2 RX, float2 RY, float2 NRY, float2 Q, float2 RHO) {
     if constexpr (GAUSS) {  // the first step's ratio q0 = Q
         RX = __fmul2_rn(RX, Q);
         RY = __fmul2_rn(RY, Q);
@@ -563,14 +555,13 @@ __device__ __forceinline__ void b_chain(uint8_t* re_base, uint8_t* im_base, int 
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         const int off = sw_step(c16, UP ? i : 7 - i);
-        uint2 hi, lo;
-        split_pair(X, Y, hi, lo);
-        *reinterpret_cast<uint2*>(re_base + off) = make_uint2(h2_swap_negate(hi.x, true), h2_swap_negate(hi.y, true));
-        *reinterpret_cast<uint2*>(re_base + off + lo_gap) =
-            make_uint2(h2_swap_negate(lo.x, true), h2_swap_negate(lo.y, true));
-        *reinterpret_cast<uint2*>(im_base + off) = make_uint2(h2_swap_negate(hi.x, false), h2_swap_negate(hi.y, false));
-        *reinterpret_cast<uint2*>(im_base + off + lo_gap) =
-            make_uint2(h2_swap_negate(lo.x, false), h2_swap_negate(lo.y, false));
+        uint32_t hi, lo;
+        split_two(X, hi, lo);
+        *reinterpret_cast<uint32_t*>(re_base + off) = hi;
+        *reinterpret_cast<uint32_t*>(re_base + off + lo_gap) = lo;
+        split_two(Y, hi, lo);
+        *reinterpret_cast<uint32_t*>(im_base + off) = hi;
+        *reinterpret_cast<uint32_t*>(im_base + off + lo_gap) = lo;
         if (i < 7) rotate_pair<GAUSS>(X, Y, RX, RY, NRY, RHO);
     }
 }
@@ -588,22 +579,23 @@ __device__ __forceinline__ float chebyshev_t(int q, float t) {
 }
 
 // One B unit: the job's columns c_col .. c_col + 7 of a particle pair
-// (fixed-point z turns pqz, Gaussian exponents pgam -- for h-binned jobs the
-// particles' normalised radii t in their bin; unit rotations RX, RY, NRY = -RY
-// and Gaussian ratios RHO as in rotate_pair), into a B operand of bnc c values
-// at bhi: rows chunk*8 .. +7 of its Re F half and of its Im F half, hi rows
-// then lo rows 2 bnc rows later.  Column c_col is frequency c_col + c_base; in
+// (fixed-point z turns pqz, column offsets pob, Gaussian exponents pgam -- for
+// h-binned jobs the particles' normalised radii t in their bin; unit rotations
+// RX, RY, NRY = -RY and Gaussian ratios RHO as in rotate_pair), into a B
+// operand of bnc c values at bhi: rows chunk*8 .. +7 of its Re B half and of
+// its Im B half, hi rows then lo rows 2 bnc rows later.  Column c_col is
+// frequency c_col + c_base; in
 // an h-binned job (period > 0) it is frequency c_col % period + c_base of
 // column block k = c_col / period: in a row-folded job (fold = F > 1) the b
 // offset bl = k mod F, whose phase bl Qy (fixed-point y turns pqy) joins the
 // chain's start; in an h-binned job (cheb_blocks) Chebyshev block q = k / F,
-// weighted by T_q(t).  The chain's 8
-// frequencies c_s .. c_s + 7 rise from c_s >= 0 and never cross a block (the
+// weighted by T_q(t).  The chain's 8 frequencies never cross a block (the
 // period is a multiple of 8).  The producer warps run it into the stage
 // buffer and tc_bimg_kernel into global memory: one arithmetic for both.
 __device__ __forceinline__ void b_unit(uint8_t* bhi, int bnc, int chunk, int col, int c_col, int c_base, int period,
                                        int fold, bool cheb_blocks, const uint32_t* pqz, const uint32_t* pqy,
-                                       const float* pgam, bool gauss, float2 RX, float2 RY, float2 NRY, float2 RHO) {
+                                       const uint32_t* pob, const float* pgam, bool gauss, float2 RX, float2 RY,
+                                       float2 NRY, float2 RHO) {
     int c_s = c_col + c_base, cheb = -1;
     uint32_t bl = 0u;
     if (period > 0) {
@@ -612,15 +604,15 @@ __device__ __forceinline__ void b_unit(uint8_t* bhi, int bnc, int chunk, int col
         bl = (uint32_t)(blk % fold);
         if (cheb_blocks) cheb = blk / fold;
     }
-    // a unit of negative frequencies (the axis-exchanged jobs' b columns)
-    // starts at its top and falls
-    const bool down = c_s < 0;
+    // a Gaussian unit of negative frequencies (the Nyquist plane's columns)
+    // starts at its top and falls, so its factors only shrink
+    const bool down = gauss && c_s < 0;
     const int c_t = down ? c_s + 7 : c_s;
     float v[2][3];
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
         float sn, cs;
-        __sincosf(turns_to_radians((uint32_t)c_t * pqz[e] + bl * pqy[e]), &sn, &cs);
+        __sincosf(turns_to_radians((uint32_t)c_t * pqz[e] + bl * pqy[e] + pob[e]), &sn, &cs);
         float g = kOperandScale, q = 1.f;
         if (gauss) {
             g *= exp2f(pgam[e] * (float)(c_t * c_t));
@@ -636,17 +628,12 @@ __device__ __forceinline__ void b_unit(uint8_t* bhi, int bnc, int chunk, int col
     const float2 Y = make_float2(v[0][1], v[1][1]);
     // bnc and chunk * 8 are multiples of 8: row K of the chain is K within its atom
     uint8_t* re_base = bhi + chunk * 8 * kRowBytes + (col & 15);
-    uint8_t* im_base = bhi + (bnc + chunk * 8) * kRowBytes + (col & 15);
-    const int c16 = col & ~15;
-    const float2 Q = gauss ? make_float2(v[0][2], v[1][2]) : make_float2(1.f, 1.f);
-    // falling: the conjugate rotation
-    if (down) {
-        if (gauss) b_chain<true, false>(re_base, im_base, 2 * bnc * kRowBytes, c16, X, Y, RX, NRY, RY, Q, RHO);
-        else b_chain<false, false>(re_base, im_base, 2 * bnc * kRowBytes, c16, X, Y, RX, NRY, RY, Q, RHO);
-    } else {
-        if (gauss) b_chain<true, true>(re_base, im_base, 2 * bnc * kRowBytes, c16, X, Y, RX, RY, NRY, Q, RHO);
-        else b_chain<false, true>(re_base, im_base, 2 * bnc * kRowBytes, c16, X, Y, RX, RY, NRY, Q, RHO);
-    }
+    uint8_t* im_base = re_base + bnc * kRowBytes;
+    const int c16 = col & ~15, lo_gap = 2 * bnc * kRowBytes;
+    const float2 Q = make_float2(v[0][2], v[1][2]);
+    if (!gauss) unit_chain<false, true>(re_base, im_base, lo_gap, c16, X, Y, RX, RY, NRY, Q, RHO);
+    else if (down) unit_chain<true, false>(re_base, im_base, lo_gap, c16, X, Y, RX, NRY, RY, Q, RHO);  // conjugate
+    else unit_chain<true, true>(re_base, im_base, lo_gap, c16, X, Y, RX, RY, NRY, Q, RHO);
 }
 
 // Persistent: CTA (or CTA pair) b walks items b, b + grid, ... of the
@@ -686,7 +673,6 @@ __global__ void __launch_bounds__(kThreads, 1) tc_sum_kernel(TcArgs a) {
     const int tid = threadIdx.x;
     const int warp = tid >> 5;
     const int lane = tid & 31;
-    const int flush_stages = a.flush_stages;
     const int rank = kCtas == 2 ? (int)cluster_rank() : 0;
     const int unit = blockIdx.x / kCtas, n_units = gridDim.x / kCtas;  // CTA or CTA pair
 
@@ -750,9 +736,9 @@ __global__ void __launch_bounds__(kThreads, 1) tc_sum_kernel(TcArgs a) {
                 const uint32_t idesc = mma_idesc(kM * kCtas, 2 * I.nc);
                 for (int s = 0; s < I.n_stages; ++s, ++S) {
                     const int fb = S % kFull, ab = S % kAStages, bb = S % kBStages;
-                    const int k = C + s / flush_stages;  // chain index
+                    const int k = C + s / I.flush;  // chain index
                     const int b = k % kBufs, u = k / kBufs;  // accumulator and its use count
-                    const bool first = (s % flush_stages) == 0;
+                    const bool first = (s % I.flush) == 0;
                     // a chain starts once the flush of the accumulator's previous chain has read it
                     if (first && u >= 1 && !mbar_wait(&acc_empty[b], (u - 1) & 1, abort_flag, a.error_flag, a.wait_limit_ns, 1)) break;
                     if (!mbar_wait(&full[fb], (S / kFull) & 1, abort_flag, a.error_flag, a.wait_limit_ns, 2)) break;
@@ -772,7 +758,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_sum_kernel(TcArgs a) {
                     }
                     mma_commit<kCtas>(&a_empty[ab]);
                     mma_commit<kCtas>(&b_empty[bb]);
-                    if ((s % flush_stages) == flush_stages - 1 || s == I.n_stages - 1) mma_commit<kCtas>(&acc_full[b]);
+                    if ((s % I.flush) == I.flush - 1 || s == I.n_stages - 1) mma_commit<kCtas>(&acc_full[b]);
                 }
                 C += I.n_chunks;
             }
@@ -818,6 +804,18 @@ __global__ void __launch_bounds__(kThreads, 1) tc_sum_kernel(TcArgs a) {
                 // warp-uniform outcome: the warp arrives as one below
                 if (!__all_sync(0xffffffffu, mbar_wait(&acc_full[b], u & 1, abort_flag, a.error_flag, a.wait_limit_ns, 4))) break;
                 tc_fence_after();
+                // the chain's total, with its mean truncation added back
+                // (kChainGain)
+                const int chain_n = min(I.flush * kKp, I.ke - I.kb - kk * I.flush * kKp);
+                const float gain_n = kChainGain * (float)chain_n;
+                const float agree = kChainAgree * kChainGain / (kOperandScale * kOperandScale);
+                auto chain_gain = [&](float v) {
+                    return 1.f + fminf(fmaf(fabsf(v), agree, gain_n), kChainGainMost * gain_n);
+                };
+                // accumulator column 0, where it may be a job's unit column
+                auto chain_gain0 = [&](float v, int cc) {
+                    return cc == 0 && I.unit_col ? 1.f + kChainGainUnit * gain_n : chain_gain(v);
+                };
                 if constexpr (SH::kDB) {
                     // the item's FP32 total is its slot: the first chain stores
                     // it, later ones add to it (the slot's loads are issued
@@ -837,8 +835,10 @@ __global__ void __launch_bounds__(kThreads, 1) tc_sum_kernel(TcArgs a) {
 #pragma unroll
                         for (int i = 0; i < 4; ++i)
                             __stcg(reinterpret_cast<float4*>(slot32 + (size_t)(cc + 4 * i) * kM),
-                                   make_float4(sv[i].x + dv[4 * i], sv[i].y + dv[4 * i + 1], sv[i].z + dv[4 * i + 2],
-                                               sv[i].w + dv[4 * i + 3]));
+                                   make_float4(fmaf(dv[4 * i], chain_gain0(dv[4 * i], cc + i), sv[i].x),
+                                               fmaf(dv[4 * i + 1], chain_gain(dv[4 * i + 1]), sv[i].y),
+                                               fmaf(dv[4 * i + 2], chain_gain(dv[4 * i + 2]), sv[i].z),
+                                               fmaf(dv[4 * i + 3], chain_gain(dv[4 * i + 3]), sv[i].w)));
                     }
                     tc_fence_before();
                     __syncwarp();
@@ -873,8 +873,8 @@ __global__ void __launch_bounds__(kThreads, 1) tc_sum_kernel(TcArgs a) {
                         tmem_wait_ld();
 #pragma unroll
                         for (int i = 0; i < 4; ++i) {
-                            const float t0 = restart ? dv[2 * i] : tv[2 * i] + dv[2 * i];
-                            const float t1 = restart ? dv[2 * i + 1] : tv[2 * i + 1] + dv[2 * i + 1];
+                            const float t0 = fmaf(dv[2 * i], chain_gain0(dv[2 * i], cc + i), restart ? 0.f : tv[2 * i]);
+                            const float t1 = fmaf(dv[2 * i + 1], chain_gain(dv[2 * i + 1]), restart ? 0.f : tv[2 * i + 1]);
                             __stcg(reinterpret_cast<double2*>(slot64 + (size_t)(cc + 2 * i) * kM),
                                    make_double2(sv[i].x + (double)t0, sv[i].y + (double)t1));
                         }
@@ -890,6 +890,8 @@ __global__ void __launch_bounds__(kThreads, 1) tc_sum_kernel(TcArgs a) {
                         if (restart) {
                             tmem_ld32(acc_col + cc, tt);
                             tmem_wait_ld();
+#pragma unroll
+                            for (int i = 0; i < 32; ++i) tt[i] *= i == 0 ? chain_gain0(tt[0], cc) : chain_gain(tt[i]);
                         } else {
                             float dv[32];
                             tmem_ld32(acc_col + cc, dv);
@@ -897,8 +899,9 @@ __global__ void __launch_bounds__(kThreads, 1) tc_sum_kernel(TcArgs a) {
                             tmem_wait_ld();
 #pragma unroll
                             for (int i = 0; i < 32; i += 2) {
-                                const float2 t2 =
-                                    __fadd2_rn(make_float2(tt[i], tt[i + 1]), make_float2(dv[i], dv[i + 1]));
+                                const float2 t2 = __ffma2_rn(make_float2(dv[i], dv[i + 1]), make_float2(i == 0 ? chain_gain0(dv[0], cc) : chain_gain(dv[i]),
+                                                                         chain_gain(dv[i + 1])),
+                                                             make_float2(tt[i], tt[i + 1]));
                                 tt[i] = t2.x;
                                 tt[i + 1] = t2.y;
                             }
@@ -979,67 +982,57 @@ __global__ void __launch_bounds__(kThreads, 1) tc_sum_kernel(TcArgs a) {
         __syncwarp();
     } else {
         // -------------------------------------------------------- producers
-        const int p = tid - 32 * (1 + kFlushWarps);
-        const int pp = p & 15;  // particle pair within the stage
-        const bool has_a = p < 256;  // A unit: 8-row chunk rc; else B unit: c chunks cb, cb + 8
-        const int rc = (p >> 4) & 15;
-        const int cb = (p >> 4) & 7;
+        const int pw = warp - 1 - kFlushWarps;  // producer warp: 0-7 A units, 8-11 B units
+        const bool has_a = pw < 8;   // A unit: chunk pw of 8 representatives; else B unit: c chunks cb, cb + 4, ...
+        const int cb = pw - 8;
         int S = 0;
         for (int it = unit; it < a.n_items && !__any_sync(0xffffffffu, *abort_flag != 0); it += n_units) {
             const TcItem I = tc_item<MODE>(a, it, rank);
             const int ky = I.job->ky;
             const bool gauss = I.job->gauss != 0;
-            const int rho0 = I.row0 + rc * 8;
+            const int rho0 = I.row0 + pw * 8;
             const int a_x = rho0 / ky + I.a_base;
-            // the chunk's 8 rows have b = b0, b0 + fold, ..., b0 + 7 fold (the
-            // constants' y rotation is the one of fold steps)
+            // the chunk's 8 representatives have b = b0, b0 + fold, ..., b0 + 7
+            // fold (the constants' y rotation is the one of fold steps);
+            // Gaussian chains run away from b = 0
             const int b0 = (rho0 % ky) * I.fold + I.b_base;
-            const bool a_up = b0 >= 0;
+            const bool a_up = !gauss || b0 >= 0;
             const int b_s = a_up ? b0 : b0 + 7 * I.fold;
             for (int s = 0; s < I.n_stages; ++s, ++S) {
                 const int buf = S % kSlots;
                 if (!__all_sync(0xffffffffu, mbar_wait(&pdata[buf], (S / kSlots) & 1, abort_flag, a.error_flag, a.wait_limit_ns, 64)))
                     break;
-                uint32_t pqx[2], pqy[2], pqz[2];
-                float pamp[2], pgam[2], prho2[2];
-                float2 pry[2], prz[2];
+                // the pair's constants: particles 2 lane, 2 lane + 1 of the
+                // stage's block (row side for A warps, column side for B warps)
+                uint32_t pq[2], pqy[2], po[2];
+                float pamp[2] = {0.f, 0.f}, pgam[2] = {0.f, 0.f}, prho2[2] = {1.f, 1.f};
+                float2 pr[2];
                 {
-                    // the pair's constants: particles 2pp, 2pp+1 of the stage's block
                     const uint8_t* blk = slots + buf * kSlotBytes;
-                    const uint2 gq = *reinterpret_cast<const uint2*>(blk + kOffGam + 8 * pp);
-                    const uint2 rq = *reinterpret_cast<const uint2*>(blk + kOffRho2 + 8 * pp);
+                    const uint2 x = *reinterpret_cast<const uint2*>(blk + (has_a ? kOffQx : kOffQz) + 8 * lane);
+                    const uint2 y = *reinterpret_cast<const uint2*>(blk + kOffQy + 8 * lane);
+                    const uint2 o = *reinterpret_cast<const uint2*>(blk + (has_a ? kOffOa : kOffOb) + 8 * lane);
+                    const uint2 gq = *reinterpret_cast<const uint2*>(blk + kOffGam + 8 * lane);
+                    const float4 r = *reinterpret_cast<const float4*>(blk + (has_a ? kOffRy : kOffRz) + 16 * lane);
+                    pq[0] = x.x;
+                    pq[1] = x.y;
+                    pqy[0] = y.x;  // B, row-folded jobs: the phase of a column block's b offset
+                    pqy[1] = y.y;
+                    po[0] = o.x;
+                    po[1] = o.y;
                     pgam[0] = __uint_as_float(gq.x);
                     pgam[1] = __uint_as_float(gq.y);
-                    prho2[0] = __uint_as_float(rq.x);
-                    prho2[1] = __uint_as_float(rq.y);
+                    pr[0] = make_float2(r.x, r.y);
+                    pr[1] = make_float2(r.z, r.w);
                     if (has_a) {
-                        const uint2 x = *reinterpret_cast<const uint2*>(blk + kOffQx + 8 * pp);
-                        const uint2 y = *reinterpret_cast<const uint2*>(blk + kOffQy + 8 * pp);
-                        const uint2 w = *reinterpret_cast<const uint2*>(blk + kOffAmp + 8 * pp);
-                        const float4 r = *reinterpret_cast<const float4*>(blk + kOffRy + 16 * pp);
-                        pqx[0] = x.x;
-                        pqx[1] = x.y;
-                        pqy[0] = y.x;
-                        pqy[1] = y.y;
+                        const uint2 w = *reinterpret_cast<const uint2*>(blk + kOffAmp + 8 * lane);
                         pamp[0] = __uint_as_float(w.x);
                         pamp[1] = __uint_as_float(w.y);
-                        pry[0] = make_float2(r.x, r.y);
-                        pry[1] = make_float2(r.z, r.w);
-                        pqz[0] = pqz[1] = 0u;
-                        prz[0] = prz[1] = make_float2(1.f, 0.f);
-                    } else {
-                        const uint2 zq = *reinterpret_cast<const uint2*>(blk + kOffQz + 8 * pp);
-                        const uint2 yq = *reinterpret_cast<const uint2*>(blk + kOffQy + 8 * pp);
-                        const float4 r = *reinterpret_cast<const float4*>(blk + kOffRz + 16 * pp);
-                        pqz[0] = zq.x;
-                        pqz[1] = zq.y;
-                        prz[0] = make_float2(r.x, r.y);
-                        prz[1] = make_float2(r.z, r.w);
-                        pqy[0] = yq.x;  // row-folded jobs: the phase of a column block's b offset
-                        pqy[1] = yq.y;
-                        pqx[0] = pqx[1] = 0u;
-                        pamp[0] = pamp[1] = 0.f;
-                        pry[0] = pry[1] = make_float2(1.f, 0.f);
+                    }
+                    if (gauss) {
+                        const uint2 rq = *reinterpret_cast<const uint2*>(blk + kOffRho2 + 8 * lane);
+                        prho2[0] = __uint_as_float(rq.x);
+                        prho2[1] = __uint_as_float(rq.y);
                     }
                 }
                 // the slot's constants are in registers: release it to the loader
@@ -1053,16 +1046,15 @@ __global__ void __launch_bounds__(kThreads, 1) tc_sum_kernel(TcArgs a) {
                 if (!__all_sync(0xffffffffu, waited)) break;
                 uint8_t* st = has_a ? a_ring + (S % kAStages) * SH::kAStageBytes
                                     : b_ring + (S % kBStages) * SH::kBStageBytes;
-                // the thread's two particles as packed pairs (see split_pair)
-                float2 X, Y, RX, RY, Q = make_float2(1.f, 1.f), RHO = make_float2(1.f, 1.f);
-                const int col = 8 * pp;  // byte offset of the pair within a 128-byte operand row
+                const int col = 4 * lane;  // byte offset of the pair within a 128-byte operand row
+                const float2 RHO = make_float2(prho2[0], prho2[1]);
                 if (has_a) {
-                    // ---- A: rows rc*8 .. rc*8+7, particles 2pp, 2pp+1 (amp includes 2^12)
-                    float v[2][5];
+                    // ---- A: representatives pw*8 .. pw*8+7 (amp includes 2^12)
+                    float v[2][3];
 #pragma unroll
                     for (int e = 0; e < 2; ++e) {
                         float sn, cs;
-                        __sincosf(turns_to_radians((uint32_t)a_x * pqx[e] + (uint32_t)b_s * pqy[e]), &sn, &cs);
+                        __sincosf(turns_to_radians((uint32_t)a_x * pq[e] + (uint32_t)b_s * pqy[e] + po[e]), &sn, &cs);
                         float g = pamp[e], q = 1.f;
                         if (gauss) {
                             g *= exp2f(pgam[e] * (float)(a_x * a_x + b_s * b_s));
@@ -1070,43 +1062,30 @@ __global__ void __launch_bounds__(kThreads, 1) tc_sum_kernel(TcArgs a) {
                         }
                         v[e][0] = g * cs;
                         v[e][1] = -g * sn;
-                        v[e][2] = pry[e].x;
-                        v[e][3] = a_up ? pry[e].y : -pry[e].y;
-                        v[e][4] = q;
+                        v[e][2] = q;
                     }
-                    X = make_float2(v[0][0], v[1][0]);
-                    Y = make_float2(v[0][1], v[1][1]);
-                    RX = make_float2(v[0][2], v[1][2]);
-                    RY = make_float2(v[0][3], v[1][3]);
+                    const float2 X = make_float2(v[0][0], v[1][0]), Y = make_float2(v[0][1], v[1][1]);
+                    const float2 RX = make_float2(pr[0].x, pr[1].x), RY = make_float2(pr[0].y, pr[1].y);
                     const float2 NRY = make_float2(-RY.x, -RY.y);
-                    uint8_t* base = st + rc * 8 * kRowBytes + (col & 15);
+                    const float2 Q = make_float2(v[0][2], v[1][2]);
+                    uint8_t* base = st + pw * kAtomBytes + (col & 15);
                     const int c16 = col & ~15;
-                    if (gauss) {
-                        Q = make_float2(v[0][4], v[1][4]);
-                        RHO = make_float2(prho2[0], prho2[1]);
-                        if (a_up) a_chain<true, true>(base, c16, X, Y, RX, RY, NRY, Q, RHO);
-                        else a_chain<true, false>(base, c16, X, Y, RX, RY, NRY, Q, RHO);
-                    } else {
-                        if (a_up) a_chain<false, true>(base, c16, X, Y, RX, RY, NRY, Q, RHO);
-                        else a_chain<false, false>(base, c16, X, Y, RX, RY, NRY, Q, RHO);
-                    }
-                } else {
-                    // ---- B: c chunks cb (and cb + 8, kWide) of this CTA's bnc c values
-                    // from bc0 (8 each), scaled by 2^12; rows [0, bnc) hold (Re B, -Im B)
-                    // pairs (Re F columns), rows [bnc, 2 bnc) (Im B, Re B) (Im F columns).
-                    // Chunks at or beyond bnc are not read by the MMA.
-                    uint8_t* bhi = st;
-                    RX = make_float2(prz[0].x, prz[1].x);
-                    RY = make_float2(prz[0].y, prz[1].y);
+                    if (!gauss) unit_chain<false, true>(base, base + kSinGap, kABytes, c16, X, Y, RX, RY, NRY, Q, RHO);
+                    else if (a_up) unit_chain<true, true>(base, base + kSinGap, kABytes, c16, X, Y, RX, RY, NRY, Q, RHO);
+                    else unit_chain<true, false>(base, base + kSinGap, kABytes, c16, X, Y, RX, NRY, RY, Q, RHO);
+                } else if (!I.bimg) {  // the loader copies B images
+                    // ---- B: c chunks cb, cb + 4, ... of this CTA's bnc c values
+                    // from bc0 (8 each), scaled by 2^12; rows [0, bnc) hold Re B,
+                    // rows [bnc, 2 bnc) Im B.  Chunks at or beyond bnc are not
+                    // read by the MMA.
+                    const float2 RX = make_float2(pr[0].x, pr[1].x), RY = make_float2(pr[0].y, pr[1].y);
                     const float2 NRY = make_float2(-RY.x, -RY.y);
-                    if (gauss) RHO = make_float2(prho2[0], prho2[1]);
 #pragma unroll 1
                     for (int h = 0; h < SH::kChunksPerThread; ++h) {
-                        const int chunk = cb + 8 * h;
-                        if (chunk * 8 >= I.bnc || I.bimg) break;  // the loader copies B images
-                        b_unit(bhi, I.bnc, chunk, col, I.bc0 + chunk * 8, I.c_base, I.period, I.fold,
-                               I.job->coef != nullptr, pqz, pqy, pgam, gauss, RX, RY,
-                               NRY, RHO);
+                        const int chunk = cb + 4 * h;
+                        if (chunk * 8 >= I.bnc) break;
+                        b_unit(st, I.bnc, chunk, col, I.bc0 + chunk * 8, I.c_base, I.period, I.fold,
+                               I.job->coef != nullptr, pq, pqy, po, pgam, gauss, RX, RY, NRY, RHO);
                     }
                 }
                 // each thread makes its stores visible to the tensor core; the
@@ -1170,15 +1149,42 @@ struct TcPrepArgs {
     bool gauss;
     int fold;          // the planes' job's row fold (1: none): its y rotation covers fold steps
     int exch;          // the planes' job is axis-exchanged: its blocks carry y and z exchanged
-    uint8_t* out;      // ceil(n / 32) blocks
-    uint8_t* out_nyq;  // the same with x and z exchanged (the Nyquist-plane job's), or null
+    int half_y, half_z;  // Ky/2 and Kz/2
+    uint8_t* out;      // ceil(n / 64) blocks
+    uint8_t* out_nyq;  // the Nyquist plane's job's (rows y, columns x, z fixed at Kz/2), or null
+    uint8_t* out_face; // Gaussian groups: the b = -Ky/2 job's (rows x, columns z, y fixed), or null
 };
+
+// One particle's constants (entry l of block blk): row a, row b and column
+// turns, and the phase offsets.
+__device__ __forceinline__ void put_constants(uint8_t* blk, int l, uint32_t qa, uint32_t qb, uint32_t qc, float amp,
+                                              float gam, float rho2, uint32_t offa, uint32_t offb, float2 rb,
+                                              float2 rc) {
+    reinterpret_cast<uint32_t*>(blk + kOffQx)[l] = qa;
+    reinterpret_cast<uint32_t*>(blk + kOffQy)[l] = qb;
+    reinterpret_cast<uint32_t*>(blk + kOffQz)[l] = qc;
+    reinterpret_cast<float*>(blk + kOffAmp)[l] = amp;
+    reinterpret_cast<float*>(blk + kOffGam)[l] = gam;
+    reinterpret_cast<float*>(blk + kOffRho2)[l] = rho2;
+    reinterpret_cast<uint32_t*>(blk + kOffOa)[l] = offa;
+    reinterpret_cast<uint32_t*>(blk + kOffOb)[l] = offb;
+    reinterpret_cast<float2*>(blk + kOffRy)[l] = rb;
+    reinterpret_cast<float2*>(blk + kOffRz)[l] = rc;
+}
+
+// Half of the row lattice's step (Qx + F Qy) / 2, in turns: the row phases of
+// a pure-phase job are taken about the middle of its lattice, (a, b) =
+// (-1/2, -F/2) (TcJob), and the columns take the offset back.  The odd half
+// unit that is dropped (2^-33 turns) drops from both sides.
+__device__ __forceinline__ uint32_t half_steps(uint32_t qx, uint32_t qy, int fold) {
+    return (qx >> 1) + (uint32_t)(fold >> 1) * qy + ((fold & 1) ? qy >> 1 : 0u);
+}
 
 __global__ void tc_prep_kernel(TcPrepArgs p) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     const int padded = (p.n + kBlockParticles - 1) / kBlockParticles * kBlockParticles;
     if (j >= padded) return;
-    uint8_t* blk = p.out + (size_t)(j / kBlockParticles) * kBlockBytes;
+    const size_t blk = (size_t)(j / kBlockParticles) * kBlockBytes;
     const int l = j % kBlockParticles;
     uint32_t qx = 0, qy = 0, qz = 0;
     float amp = 0.f, gam = 0.f;
@@ -1193,27 +1199,22 @@ __global__ void tc_prep_kernel(TcPrepArgs p) {
             gam = p.gamma_scale * h * h;
         }
     }
-    const uint32_t by = p.exch ? qz : qy, bz = p.exch ? qy : qz;  // the planes job's row and column axes
-    reinterpret_cast<uint32_t*>(blk + kOffQx)[l] = qx;
-    reinterpret_cast<uint32_t*>(blk + kOffQy)[l] = by;
-    reinterpret_cast<uint32_t*>(blk + kOffQz)[l] = bz;
-    reinterpret_cast<float*>(blk + kOffAmp)[l] = amp;
-    reinterpret_cast<float*>(blk + kOffGam)[l] = gam;
-    reinterpret_cast<float*>(blk + kOffRho2)[l] = exp2f(2.f * gam);
-    const float2 ry = unit_phase(qy);
-    reinterpret_cast<float2*>(blk + kOffRy)[l] = unit_phase((uint32_t)p.fold * by);
-    reinterpret_cast<float2*>(blk + kOffRz)[l] = unit_phase(bz);
+    const float rho2 = exp2f(2.f * gam);
+    const uint32_t by = p.exch ? qz : qy, bz = p.exch ? qy : qz;  // the planes job's row b and column axes
+    const uint32_t off = p.gauss ? 0u : half_steps(qx, by, p.fold);
+    const float2 ux = unit_phase(qx), uy = unit_phase(qy), uz = unit_phase(qz);
+    const float2 ry = p.exch ? uz : p.fold > 1 ? unit_phase((uint32_t)p.fold * by) : uy;
+    put_constants(p.out + blk, l, qx, by, bz, amp, gam, rho2, off, 0u - off, ry, p.exch ? uy : uz);
+    // a fixed frequency f joins the column offsets and, for Gaussians, the weight
+    auto fixed_amp = [&](int f) { return p.gauss ? amp * exp2f(gam * (float)(f * f)) : amp; };
     if (p.out_nyq) {
-        uint8_t* t = p.out_nyq + (size_t)(j / kBlockParticles) * kBlockBytes;
-        reinterpret_cast<uint32_t*>(t + kOffQx)[l] = qz;
-        reinterpret_cast<uint32_t*>(t + kOffQy)[l] = qy;
-        reinterpret_cast<uint32_t*>(t + kOffQz)[l] = qx;
-        reinterpret_cast<float*>(t + kOffAmp)[l] = amp;
-        reinterpret_cast<float*>(t + kOffGam)[l] = gam;
-        reinterpret_cast<float*>(t + kOffRho2)[l] = exp2f(2.f * gam);
-        reinterpret_cast<float2*>(t + kOffRy)[l] = ry;
-        reinterpret_cast<float2*>(t + kOffRz)[l] = unit_phase(qx);
+        const uint32_t o = p.gauss ? 0u : qy >> 1;
+        put_constants(p.out_nyq + blk, l, 0u, qy, qx, fixed_amp(p.half_z), gam, rho2, o, (uint32_t)p.half_z * qz - o,
+                      uy, ux);
     }
+    if (p.out_face)
+        put_constants(p.out_face + blk, l, 0u, qx, qz, fixed_amp(p.half_y), gam, rho2, 0u,
+                      0u - (uint32_t)p.half_y * qy, ux, uz);
 }
 
 // h-bins of a group whose Phi^ does not separate per axis (SPH, Wendland with
@@ -1243,7 +1244,8 @@ struct TcBinnedPrepArgs {
     const int4* bins;      // (first block, capacity, coef offset, order)
     const float4* spans;   // (lo, hi, 2^12 / W_b, 0): Chebyshev interval and weight scale
     uint8_t* out;          // the group's blocks, bin by bin
-    uint8_t* out_nyq;      // the same with x and z exchanged, or null
+    uint8_t* out_nyq;      // the Nyquist plane's jobs' (rows y, columns x, z fixed at Kz/2), or null
+    int half_z;            // Kz/2
     const int* first;      // nbins + 1: the bins' first particles in sorted order
     float4* sorted;        // particles sorted by bin (for the branch part)
     float* sorted_radii;
@@ -1289,19 +1291,14 @@ __global__ void tc_prep_binned_kernel(TcBinnedPrepArgs p) {
     const float amp = q.w * sp.z;
     const size_t blk_off = (size_t)(bin.x + slot / kBlockParticles) * kBlockBytes;
     const int l = slot % kBlockParticles;
-    const float2 ry = unit_phase(qy);
-    const float2 ry_fold = p.fold > 1 ? unit_phase((uint32_t)p.fold * qy) : ry;
-    for (int pass = 0; pass < (p.out_nyq ? 2 : 1); ++pass) {
-        uint8_t* blk = (pass == 0 ? p.out : p.out_nyq) + blk_off;
-        const uint32_t ax = pass == 0 ? qx : qz, az = pass == 0 ? qz : qx;
-        reinterpret_cast<uint32_t*>(blk + kOffQx)[l] = ax;
-        reinterpret_cast<uint32_t*>(blk + kOffQy)[l] = qy;
-        reinterpret_cast<uint32_t*>(blk + kOffQz)[l] = az;
-        reinterpret_cast<float*>(blk + kOffAmp)[l] = amp;
-        reinterpret_cast<float*>(blk + kOffGam)[l] = t;
-        reinterpret_cast<float*>(blk + kOffRho2)[l] = 1.f;
-        reinterpret_cast<float2*>(blk + kOffRy)[l] = pass == 0 ? ry_fold : ry;
-        reinterpret_cast<float2*>(blk + kOffRz)[l] = unit_phase(az);
+    const float2 uy = unit_phase(qy);
+    const float2 ry = p.fold > 1 ? unit_phase((uint32_t)p.fold * qy) : uy;
+    const uint32_t off = half_steps(qx, qy, p.fold);
+    put_constants(p.out + blk_off, l, qx, qy, qz, amp, t, 1.f, off, 0u - off, ry, unit_phase(qz));
+    if (p.out_nyq) {
+        const uint32_t o = qy >> 1;
+        put_constants(p.out_nyq + blk_off, l, 0u, qy, qx, amp, t, 1.f, o, (uint32_t)p.half_z * qz - o, uy,
+                      unit_phase(qx));
     }
 }
 
@@ -1354,7 +1351,7 @@ __global__ void tc_coef_kernel(TcCoefArgs c) {
 }
 
 // B-operand images of one job (layout in TcJob): one CTA per image (n-tile,
-// CTA half, 32-particle block); thread (chunk, pair) runs b_unit for 8 c
+// CTA half, 64-particle block); warp (chunk), lane (pair) runs b_unit for 8 c
 // values of 2 particles, exactly as a producer warp would into the stage
 // buffer.  Each image is written once and copied by the tensor kernel's loader
 // for every m-tile of the job.
@@ -1383,39 +1380,38 @@ __global__ void __launch_bounds__(256) tc_bimg_kernel(TcImageArgs g) {
     const int half = nh % J.ctas, n_tile = nh / J.ctas;
     const int c0 = n_tile * J.nc_tile;
     const int bnc = min(J.nc_tile, J.lz_tc - c0) / J.ctas;
-    const int pp = threadIdx.x & 15, chunk = threadIdx.x >> 4;
-    if (chunk * 8 >= bnc) return;
+    const int pp = threadIdx.x & 31;
     const unsigned char* blk = J.blocks + (size_t)block * kBlockBytes;
     const uint2 zq = *reinterpret_cast<const uint2*>(blk + kOffQz + 8 * pp);
     const uint2 yq = *reinterpret_cast<const uint2*>(blk + kOffQy + 8 * pp);
+    const uint2 oq = *reinterpret_cast<const uint2*>(blk + kOffOb + 8 * pp);
     const uint2 gq = *reinterpret_cast<const uint2*>(blk + kOffGam + 8 * pp);
     const uint2 rq = *reinterpret_cast<const uint2*>(blk + kOffRho2 + 8 * pp);
     const float4 r = *reinterpret_cast<const float4*>(blk + kOffRz + 16 * pp);
-    const uint32_t pqz[2] = {zq.x, zq.y}, pqy[2] = {yq.x, yq.y};
+    const uint32_t pqz[2] = {zq.x, zq.y}, pqy[2] = {yq.x, yq.y}, pob[2] = {oq.x, oq.y};
     const float pgam[2] = {__uint_as_float(gq.x), __uint_as_float(gq.y)};
     const float2 RX = make_float2(r.x, r.z), RY = make_float2(r.y, r.w);
     const float2 NRY = make_float2(-RY.x, -RY.y);
     const bool gauss = J.gauss != 0;
     const float2 RHO = gauss ? make_float2(__uint_as_float(rq.x), __uint_as_float(rq.y)) : make_float2(1.f, 1.f);
     uint8_t* out = const_cast<uint8_t*>(J.bimg) + (size_t)img * J.img_stride;
-    b_unit(out, bnc, chunk, 8 * pp, c0 + half * bnc + chunk * 8, J.c_base, J.period, max(1, J.fold), J.coef != nullptr,
-           pqz, pqy, pgam, gauss, RX, RY, NRY, RHO);
+    for (int chunk = threadIdx.x >> 5; chunk * 8 < bnc; chunk += 8)
+        b_unit(out, bnc, chunk, 4 * pp, c0 + half * bnc + chunk * 8, J.c_base, J.period, max(1, J.fold),
+               J.coef != nullptr, pqz, pqy, pob, pgam, gauss, RX, RY, NRY, RHO);
 }
 
 // What the reduction needs of a job, gathered into shared memory once per
 // block (the job table's other fields are not read).
 struct ReduceJob {
     const void* slots;
-    int slot_fp64;
     const int4* colmap;
     const float* coef;  // null unless h-binned
     double scale;       // W x 2^-24
+    int slot_fp64;
     int slot_stride, n_splits, n_mtiles, n_ntiles;
-    int rank_stride;    // floats between the CTAs' parts of a slot: 128 * 2 nc_tile
-    int mrows_log2;     // 7 (one CTA) or 8 (CTA pair)
+    int rank_stride;    // elements between the CTAs' parts of a slot: 128 * 2 nc_tile
+    int reps_log2;      // representatives per m-tile: 6 (one CTA) or 7 (CTA pair)
     int period, blocks, coef_stride;
-    int fold, ky_full;  // row-folded jobs: the fold and the spectrum's Ky (else 1, 0)
-    int exch, rows_a;   // axis-exchanged jobs: 1 and the job rows per a (the planes)
 };
 
 __device__ __forceinline__ ReduceJob reduce_job(const TcJob& J) {
@@ -1430,285 +1426,222 @@ __device__ __forceinline__ ReduceJob reduce_job(const TcJob& J) {
     r.n_mtiles = J.n_mtiles;
     r.n_ntiles = J.n_ntiles;
     r.rank_stride = kM * 2 * J.nc_tile;
-    r.mrows_log2 = J.ctas == 2 ? 8 : 7;
+    r.reps_log2 = J.ctas == 2 ? 7 : 6;
     r.period = J.period;
     r.blocks = J.period > 0 ? J.lz_tc / J.period / (J.fold > 1 ? J.fold : 1) : 1;
     r.coef_stride = J.coef_stride;
-    r.fold = J.fold > 1 ? J.fold : 1;
-    r.ky_full = J.exch ? J.lz_tc : J.ky * r.fold;
-    r.exch = J.exch;
-    r.rows_a = J.ky;
     return r;
 }
 
-// Adds one job's contribution at lattice row rho (the spectrum's a_idx Ky +
-// b_idx; within the job's rows for unfolded jobs) and the kC consecutive
-// frequency columns c0 .. c0 + kC - 1 (c_idx, before the Chebyshev blocks of
-// an h-binned job; they share one n-tile and one CTA half, as n-tiles and
-// halves hold multiples of 8 columns): the totals of all its particle chunks
-// (FP32 or FP64 slots) summed in FP64, each h-binned block weighted by its
-// coefficient at |k|^2 = n2[i] step^2, times W 2^-24.  A row-folded job holds
-// b_idx = fold bh + bl at job row a_idx (Ky / fold) + bh, in column blocks
-// q fold + bl.
 constexpr int kReduceC = 4;
-__device__ __forceinline__ void reduce_add(const ReduceJob& J, int rho, int c0, const int* n2, int nc, double* sr,
-                                           double* si, double sign_im) {
-    if (J.exch) {
-        // axis-exchanged: plane c0 + i of spectrum row (a_idx, b_idx) is job
-        // row a_idx (planes) + c0 + i, job column b_idx; the kC rows share a
-        // 128-row CTA half (c0 is a multiple of kC)
-        const int a_idx = rho / J.ky_full, b_idx = rho - a_idx * J.ky_full;
-        const int4 m = __ldg(J.colmap + b_idx);
-        for (int i = 0; i < nc; ++i) {
-            const int jr = a_idx * J.rows_a + c0 + i;
-            const int m_tile = jr >> J.mrows_log2, within = jr - (m_tile << J.mrows_log2);
-            const int rank = within >> 7, rl = within & (kM - 1);
-            double tr = 0.0, ti = 0.0;
-            for (int ks = 0; ks < J.n_splits; ++ks) {
-                const size_t li = ((size_t)ks * J.n_mtiles + m_tile) * J.n_ntiles + m.x;
-                const size_t base = li * J.slot_stride + (size_t)rank * J.rank_stride;
-                if (J.slot_fp64) {
-                    const double* v = static_cast<const double*>(J.slots) + base + rl * 2;
-                    tr += __ldg(v + (size_t)(m.y & ~1) * kM + (m.y & 1));
-                    ti += __ldg(v + (size_t)(m.z & ~1) * kM + (m.z & 1));
-                } else {
-                    const float* v = static_cast<const float*>(J.slots) + base + rl * 4;
-                    tr += (double)__ldg(v + (size_t)(m.y & ~3) * kM + (m.y & 3));
-                    ti += (double)__ldg(v + (size_t)(m.z & ~3) * kM + (m.z & 3));
-                }
-            }
-            sr[i] = fma(J.scale, tr, sr[i]);
-            si[i] = fma(J.scale * sign_im, ti, si[i]);
-        }
-        return;
-    }
-    int bl = 0;
-    if (J.fold > 1) {
-        const int a_idx = rho / J.ky_full, b_idx = rho - a_idx * J.ky_full;
-        rho = a_idx * (J.ky_full / J.fold) + b_idx / J.fold;
-        bl = b_idx % J.fold;
-    }
-    const int m_tile = rho >> J.mrows_log2, within = rho - (m_tile << J.mrows_log2);
-    const int rank = within >> 7, rl = within & (kM - 1);
-    // FP32 slot layout [column / 4][128 rows][column % 4]: column n of row rl
-    // at (n / 4) * 512 + rl * 4 + n % 4; FP64: [column / 2][128 rows][column %
-    // 2], column n at (n / 2) * 256 + rl * 2 + n % 2
-    const size_t rbase = (size_t)rank * J.rank_stride;
-    const float* row = static_cast<const float*>(J.slots) + rbase + rl * 4;
-    const double* row64 = static_cast<const double*>(J.slots) + rbase + rl * 2;
-    if (!J.slot_fp64 && nc == kReduceC && J.n_splits == 1) {
-        // the common h-bin case (one particle chunk, FP32 slots): two column
-        // blocks per round, so each thread has twice the loads in flight
-        const size_t lbase = (size_t)m_tile * J.n_ntiles;
-        for (int q = 0; q < J.blocks; q += 2) {
-            const bool two = q + 1 < J.blocks;
-            const int4 m0 = __ldg(J.colmap + (q * J.fold + bl) * J.period + c0);
-            const int4 m1 = two ? __ldg(J.colmap + ((q + 1) * J.fold + bl) * J.period + c0) : m0;
-            const float* v0 = row + (lbase + m0.x) * J.slot_stride;
-            const float* v1 = row + (lbase + m1.x) * J.slot_stride;
-            const float4 re0 = __ldg(reinterpret_cast<const float4*>(v0 + (size_t)m0.y * kM));
-            const float4 im0 = __ldg(reinterpret_cast<const float4*>(v0 + (size_t)m0.z * kM));
-            const float4 re1 = two ? __ldg(reinterpret_cast<const float4*>(v1 + (size_t)m1.y * kM)) : make_float4(0.f, 0.f, 0.f, 0.f);
-            const float4 im1 = two ? __ldg(reinterpret_cast<const float4*>(v1 + (size_t)m1.z * kM)) : make_float4(0.f, 0.f, 0.f, 0.f);
-            double w0[kReduceC], w1[kReduceC];
+
+// The four accumulators (Re A, Im A) x (Re B, Im B) of one representative and
+// kReduceC columns in one item's slot.
+struct Quad {
+    double cc[kReduceC], cs[kReduceC], sc[kReduceC], ss[kReduceC];
+};
+
+__device__ __forceinline__ void quad_load(const ReduceJob& J, size_t base, int rl, int4 m, Quad& t) {
+    // FP32 slots: column n (a multiple of 4) of row r at (n / 4) * 512 + 4 r,
+    // four columns in one load, a warp's rows 512 contiguous bytes; FP64:
+    // column n (even) at (n / 2) * 256 + 2 r
+    if (J.slot_fp64) {
+        const double* v = static_cast<const double*>(J.slots) + base + rl * 2;
 #pragma unroll
-            for (int i = 0; i < kReduceC; ++i) {
-                w0[i] = J.coef ? (double)__ldg(J.coef + (size_t)n2[i] * J.coef_stride + q) * J.scale : J.scale;
-                w1[i] = J.coef && two ? (double)__ldg(J.coef + (size_t)n2[i] * J.coef_stride + q + 1) * J.scale
-                                      : (two ? J.scale : 0.0);
-            }
-            const float r0[kReduceC] = {re0.x, re0.y, re0.z, re0.w}, i0[kReduceC] = {im0.x, im0.y, im0.z, im0.w};
-            const float r1[kReduceC] = {re1.x, re1.y, re1.z, re1.w}, i1[kReduceC] = {im1.x, im1.y, im1.z, im1.w};
-#pragma unroll
-            for (int i = 0; i < kReduceC; ++i) {
-                sr[i] = fma(w1[i], (double)r1[i], fma(w0[i], (double)r0[i], sr[i]));
-                si[i] = fma(w1[i] * sign_im, (double)i1[i], fma(w0[i] * sign_im, (double)i0[i], si[i]));
-            }
+        for (int h = 0; h < 2; ++h) {
+            const double* re = v + (size_t)(m.y + 2 * h) * kM;
+            const double* im = v + (size_t)(m.z + 2 * h) * kM;
+            const double2 a = __ldg(reinterpret_cast<const double2*>(re));
+            const double2 b = __ldg(reinterpret_cast<const double2*>(im));
+            const double2 c = __ldg(reinterpret_cast<const double2*>(re + 2 * kReps));
+            const double2 d = __ldg(reinterpret_cast<const double2*>(im + 2 * kReps));
+            t.cc[2 * h] += a.x; t.cc[2 * h + 1] += a.y;
+            t.cs[2 * h] += b.x; t.cs[2 * h + 1] += b.y;
+            t.sc[2 * h] += c.x; t.sc[2 * h + 1] += c.y;
+            t.ss[2 * h] += d.x; t.ss[2 * h + 1] += d.y;
         }
-        return;
+    } else {
+        const float* re = static_cast<const float*>(J.slots) + base + rl * 4 + (size_t)m.y * kM;
+        const float* im = static_cast<const float*>(J.slots) + base + rl * 4 + (size_t)m.z * kM;
+        const float4 a = __ldg(reinterpret_cast<const float4*>(re));
+        const float4 b = __ldg(reinterpret_cast<const float4*>(im));
+        const float4 c = __ldg(reinterpret_cast<const float4*>(re + 4 * kReps));
+        const float4 d = __ldg(reinterpret_cast<const float4*>(im + 4 * kReps));
+        t.cc[0] += a.x; t.cc[1] += a.y; t.cc[2] += a.z; t.cc[3] += a.w;
+        t.cs[0] += b.x; t.cs[1] += b.y; t.cs[2] += b.z; t.cs[3] += b.w;
+        t.sc[0] += c.x; t.sc[1] += c.y; t.sc[2] += c.z; t.sc[3] += c.w;
+        t.ss[0] += d.x; t.ss[1] += d.y; t.ss[2] += d.z; t.ss[3] += d.w;
     }
+}
+
+// Sums of one representative's kReduceC columns: [column] of F at the
+// representative (plus) and at its mirror (minus), see TcJob.
+struct PairSum {
+    double pr[kReduceC], pi[kReduceC], mr[kReduceC], mi[kReduceC];
+};
+
+// Adds one job's contribution at row representative rep and the kReduceC
+// columns from c0 of every Chebyshev block's b offset bl (they share one
+// n-tile and one CTA half, as n-tiles and halves hold multiples of 8
+// columns): the totals of all its particle chunks (FP32 or FP64 slots) summed
+// in FP64, each h-binned block weighted by its coefficients at the two
+// elements' |k|^2 = np[i] step^2 and nm[i] step^2, times W 2^-24.
+__device__ __forceinline__ void reduce_add(const ReduceJob& J, int rep, int fold, int bl, int c0, const int* np,
+                                           const int* nm, PairSum& f) {
+    const int m_tile = rep >> J.reps_log2, within = rep - (m_tile << J.reps_log2);
+    const int rl = within & (kReps - 1);
+    const size_t rbase = (size_t)(within / kReps) * J.rank_stride;
     for (int q = 0; q < J.blocks; ++q) {
-        // column block q F + bl: Chebyshev block q (h-binned), b offset bl (folded)
-        const int4 m = __ldg(J.colmap + (q * J.fold + bl) * J.period + c0);  // the same for a warp's rows
-        double tr[kReduceC] = {}, ti[kReduceC] = {};
+        const int4 m = __ldg(J.colmap + (q * fold + bl) * J.period + c0);  // the same for a warp's rows
+        float wp[kReduceC], wm[kReduceC];
+        if (J.coef) {
+#pragma unroll
+            for (int i = 0; i < kReduceC; ++i) {
+                wp[i] = __ldg(J.coef + (size_t)np[i] * J.coef_stride + q);
+                wm[i] = __ldg(J.coef + (size_t)nm[i] * J.coef_stride + q);
+            }
+        }
+        Quad t = {};
         for (int ks = 0; ks < J.n_splits; ++ks) {
             const size_t li = ((size_t)ks * J.n_mtiles + m_tile) * J.n_ntiles + m.x;
-            if (J.slot_fp64) {
-                const double* v = row64 + li * J.slot_stride;
-                if (nc == kReduceC) {
-                    // two columns per load (m.y, m.z are multiples of 4)
-                    const double2 r0 = __ldg(reinterpret_cast<const double2*>(v + (size_t)m.y * kM));
-                    const double2 r1 = __ldg(reinterpret_cast<const double2*>(v + (size_t)(m.y + 2) * kM));
-                    const double2 i0 = __ldg(reinterpret_cast<const double2*>(v + (size_t)m.z * kM));
-                    const double2 i1 = __ldg(reinterpret_cast<const double2*>(v + (size_t)(m.z + 2) * kM));
-                    tr[0] += r0.x; tr[1] += r0.y; tr[2] += r1.x; tr[3] += r1.y;
-                    ti[0] += i0.x; ti[1] += i0.y; ti[2] += i1.x; ti[3] += i1.y;
-                } else {
-                    tr[0] += __ldg(v + (size_t)(m.y & ~1) * kM + (m.y & 1));
-                    ti[0] += __ldg(v + (size_t)(m.z & ~1) * kM + (m.z & 1));
-                }
-                continue;
-            }
-            const float* v = row + li * J.slot_stride;
-            if (nc == kReduceC) {
-                // four columns in one load (m.y, m.z are multiples of 4); a warp's
-                // rows read 512 contiguous bytes
-                const float4 re = __ldg(reinterpret_cast<const float4*>(v + (size_t)m.y * kM));
-                const float4 im = __ldg(reinterpret_cast<const float4*>(v + (size_t)m.z * kM));
-                tr[0] += re.x; tr[1] += re.y; tr[2] += re.z; tr[3] += re.w;
-                ti[0] += im.x; ti[1] += im.y; ti[2] += im.z; ti[3] += im.w;
-            } else {
-                tr[0] += (double)__ldg(v + (size_t)(m.y & ~3) * kM + (m.y & 3));
-                ti[0] += (double)__ldg(v + (size_t)(m.z & ~3) * kM + (m.z & 3));
-            }
+            quad_load(J, li * J.slot_stride + rbase, rl, m, t);
         }
 #pragma unroll
         for (int i = 0; i < kReduceC; ++i) {
-            if (i < nc) {
-                const double w = J.coef ? (double)__ldg(J.coef + (size_t)n2[i] * J.coef_stride + q) * J.scale : J.scale;
-                sr[i] = fma(w, tr[i], sr[i]);
-                si[i] = fma(w * sign_im, ti[i], si[i]);
-            }
+            const double up = J.coef ? (double)wp[i] * J.scale : J.scale;
+            const double um = J.coef ? (double)wm[i] * J.scale : J.scale;
+            f.pr[i] = fma(up, t.cc[i] - t.ss[i], f.pr[i]);
+            f.pi[i] = fma(up, t.cs[i] + t.sc[i], f.pi[i]);
+            f.mr[i] = fma(um, t.cc[i] + t.ss[i], f.mr[i]);
+            f.mi[i] = fma(um, t.cs[i] - t.sc[i], f.mi[i]);
         }
     }
 }
 
-// The jobs of one output class (same spectrum, same per-frequency factor)
-// -> its float2 spectrum, added: planes c in [0, lz_tc) (tc_reduce_planes_kernel),
-// or the Nyquist plane c = lz_tc from the transposed jobs (tc_reduce_kernel):
-// for a >= 0 the a >= 0 jobs at row b_idx and column a; for a < 0 the
-// conjugate of the a < 0 jobs at row Ky - 1 - b_idx (frequency -b) and column
-// -a - 1 (frequency -a).  Times the factored Phi^(|k| h) in FP64 and the
-// scale.  The kernels gather the class's job descriptors in shared memory
-// first.
+// The jobs of one part (planes, Nyquist plane, b = -Ky/2 face) of one output
+// class (same spectrum, same per-frequency factor, same row layout) -> its
+// float2 spectrum, added, times the factored Phi^(|k| h) in FP64 and the
+// scale.  A thread takes one row representative, one b offset and kReduceC
+// columns, and writes both elements its accumulators hold.
+//
+// With the job list split over warps (parts of at least 8 jobs): a block
+// takes 32 representatives (lanes), warp w sums jobs w, w + 8, ..., and the
+// eight partial sums are added in warp order (a fixed order: the result does
+// not depend on timing), so eight independent load chains per element hide
+// the slots' latency.  With fewer jobs (f.warp_rows; one group per class, as
+// in a batch of particle sets) a block takes 8 x 32 representatives and each
+// warp sums every job of its own 32 in job order, so no warp idles.
 struct TcReduceArgs {
     const TcJob* jobs;
-    const int* list;      // planes: the class's jobs; nyquist: its a >= 0 jobs
+    const int* list;
     int n_list;
-    const int* list_neg;  // nyquist: its a < 0 jobs
-    int n_neg;
-    int kx, ky, lz_tc, lz_out;
+    TcPart part;
+    int kx, ky, lz_out;
     double step;
     int basis;
     double h;  // radius of the factored Phi^(|k| h); 1 without radii
     bool factored;
     double scale;
     float2* out;
-    int warp_rows;  // planes: every warp sums all jobs of its own 32 rows (classes of fewer jobs than warps)
+    int warp_rows;  // every warp sums all jobs of its own 32 representatives (parts of fewer jobs than warps)
 };
 
-// Warps per block of the reduction kernels (each sums every eighth job).
+// Warps per block of the reduction kernel.
 constexpr int kReduceWarps = 8;
 
-// The Nyquist plane of one output class, with the job list split over warps
-// as in tc_reduce_planes_kernel: a block takes 32 elements (lanes), warp w
-// sums the jobs w, w + 8, ... of the element's sign of a, and the eight
-// partial sums are added in warp order (a fixed order).
-__global__ void __launch_bounds__(32 * kReduceWarps) tc_reduce_kernel(TcReduceArgs f) {
-    extern __shared__ __align__(16) unsigned char s_raw[];  // descriptors, then the partial sums
-    ReduceJob* s_jobs = reinterpret_cast<ReduceJob*>(s_raw);
-    const int n_all = f.n_list + f.n_neg;
-    for (int i = threadIdx.x; i < n_all; i += blockDim.x)
-        s_jobs[i] = reduce_job(f.jobs[i < f.n_list ? f.list[i] : f.list_neg[i - f.n_list]]);
-    double2* s_part = reinterpret_cast<double2*>(s_raw + (((size_t)n_all * sizeof(ReduceJob) + 15) & ~(size_t)15));
-    __syncthreads();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const long long rows = (long long)f.kx * f.ky;
-    const long long e = (long long)blockIdx.x * 32 + lane;
-    const bool active = e < rows;
-    const int rho = active ? (int)e : 0;
-    const int a_idx = rho / f.ky, b_idx = rho % f.ky;
-    const int a = a_idx - f.kx / 2, b = b_idx - f.ky / 2;
-    const int c = f.lz_tc;
-    int n2[kReduceC];
-#pragma unroll
-    for (int i = 0; i < kReduceC; ++i) n2[i] = a * a + b * b + (c + i) * (c + i);
-    double sr[kReduceC] = {}, si[kReduceC] = {};
-    if (active) {
-        // for a >= 0 the a >= 0 jobs at row b_idx and column a; for a < 0 the
-        // conjugate of the a < 0 jobs at row Ky - 1 - b_idx (frequency -b) and
-        // column -a - 1 (frequency -a)
-        if (a >= 0) {
-            for (int j = warp; j < f.n_list; j += kReduceWarps) reduce_add(s_jobs[j], b_idx, a, n2, 1, sr, si, 1.0);
-        } else {
-            for (int j = warp; j < f.n_neg; j += kReduceWarps)
-                reduce_add(s_jobs[f.n_list + j], f.ky - 1 - b_idx, -a - 1, n2, 1, sr, si, -1.0);
-        }
-    }
-    s_part[warp * 32 + lane] = make_double2(sr[0], si[0]);
-    __syncthreads();
-    if (warp != 0 || !active) return;
-    double tr = 0.0, ti = 0.0;
-    for (int w = 0; w < kReduceWarps; ++w) {
-        const double2 v = s_part[w * 32 + lane];
-        tr += v.x;
-        ti += v.y;
-    }
-    double factor = f.scale;
-    if (f.factored) factor *= phi_fp64(f.basis, f.step * sqrt((double)n2[0]) * f.h);
-    const size_t idx = (size_t)rho * f.lz_out + c;
-    const float2 o = f.out[idx];
-    f.out[idx] = make_float2(o.x + (float)(tr * factor), o.y + (float)(ti * factor));
-}
-
-// The planes c < lz_tc of one output class.  With the job list split over
-// warps (classes of at least 8 jobs): a block takes 32 rows (lanes) x
-// kReduceC planes, warp w sums jobs w, w + 8, ..., and the eight partial sums
-// are added in warp order (a fixed order: the result does not depend on
-// timing), so eight independent load chains per element hide the slots'
-// latency.  With fewer jobs (f.warp_rows; one group per class, as in a batch
-// of particle sets) a block takes 8 x 32 rows and each warp sums every job of
-// its own 32 rows in job order, so no warp idles.
-__global__ void __launch_bounds__(32 * kReduceWarps, 2) tc_reduce_planes_kernel(TcReduceArgs f) {
+__global__ void __launch_bounds__(32 * kReduceWarps, 2) tc_reduce_kernel(TcReduceArgs f) {
     extern __shared__ __align__(16) unsigned char s_raw[];  // n_list descriptors, then the partial sums
     ReduceJob* s_jobs = reinterpret_cast<ReduceJob*>(s_raw);
     for (int i = threadIdx.x; i < f.n_list; i += blockDim.x) s_jobs[i] = reduce_job(f.jobs[f.list[i]]);
-    // [warp][lane][kReduceC], 16-byte aligned after the descriptors
+    // [warp][kReduceC * 2][lane], 16-byte aligned after the descriptors
     double2* s_part = reinterpret_cast<double2*>(s_raw + (((size_t)f.n_list * sizeof(ReduceJob) + 15) & ~(size_t)15));
     __syncthreads();
+    const TcPart& P = f.part;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const long long rows = (long long)f.kx * f.ky;
-    const int block_rows = f.warp_rows ? 32 * kReduceWarps : 32;
-    const long long row_blocks = (rows + block_rows - 1) / block_rows;
-    const int rho = (int)((blockIdx.x % row_blocks) * block_rows + (f.warp_rows ? warp * 32 : 0) + lane);
-    const int c0 = (int)(blockIdx.x / row_blocks) * kReduceC;
-    const bool active = rho < rows;
-    const int rr = active ? rho : 0;
-    const int a = rr / f.ky - f.kx / 2, b = rr % f.ky - f.ky / 2;
-    int n2[kReduceC];
-#pragma unroll
-    for (int i = 0; i < kReduceC; ++i) n2[i] = a * a + b * b + (c0 + i) * (c0 + i);
-    double sr[kReduceC] = {}, si[kReduceC] = {};
-    // spectrum element (rho, c0 + i) += its FP64 sum, with the factored Phi^
-    auto store = [&](int i, double tr, double ti) {
-        double factor = f.scale;
-        if (f.factored) factor *= phi_fp64(f.basis, f.step * sqrt((double)n2[i]) * f.h);
-        const size_t idx = (size_t)rho * f.lz_out + c0 + i;
-        const float2 o = f.out[idx];
-        f.out[idx] = make_float2(o.x + (float)(tr * factor), o.y + (float)(ti * factor));
+    const int block_reps = f.warp_rows ? 32 * kReduceWarps : 32;
+    const int rep_blocks = (P.n_reps + block_reps - 1) / block_reps;
+    const int rest = blockIdx.x / rep_blocks;
+    const int bl = rest % P.fold, c0 = rest / P.fold * kReduceC;
+    const int rep = (int)(blockIdx.x % rep_blocks) * block_reps + (f.warp_rows ? warp * 32 : 0) + lane;
+    const bool active = rep < P.n_reps;
+    const int fa = (active ? rep : 0) / P.rows + P.a_base;
+    const int rowb = (active ? rep : 0) % P.rows * P.fold + P.b_base;
+    // the frequencies of column c0 + i: plus (xp, yp, zp) and minus (xm, ym, zm)
+    int key = 0;
+    auto frequencies = [&](int i, int3& p, int3& m) {
+        const int c = c0 + i + P.c_base;
+        if (P.kind == kPartPlanes) {
+            p = make_int3(fa, rowb + bl, c);
+            m = make_int3(P.mirror_a - fa, P.mirror_b - rowb + bl, c);
+            key = fa;
+        } else if (P.kind == kPartExchanged) {
+            p = make_int3(fa, c, rowb);
+            m = make_int3(fa, -c, rowb);
+            key = c;
+        } else if (P.kind == kPartNyquist) {
+            p = make_int3(c, rowb, P.fixed);
+            m = make_int3(c, P.mirror_b - rowb, P.fixed);
+            key = rowb;
+        } else {  // kPartFace
+            p = make_int3(rowb, P.fixed, c);
+            m = make_int3(-rowb, P.fixed, c);
+            key = rowb;
+        }
     };
-    if (f.warp_rows) {  // uniform over the block: no barrier follows
-        if (!active) return;
-        for (int j = 0; j < f.n_list; ++j) reduce_add(s_jobs[j], rho, c0, n2, kReduceC, sr, si, 1.0);
-#pragma unroll
-        for (int i = 0; i < kReduceC; ++i) store(i, sr[i], si[i]);
-        return;
-    }
-    if (active)
-        for (int j = warp; j < f.n_list; j += kReduceWarps) reduce_add(s_jobs[j], rho, c0, n2, kReduceC, sr, si, 1.0);
-#pragma unroll
-    for (int i = 0; i < kReduceC; ++i) s_part[(warp * 32 + lane) * kReduceC + i] = make_double2(sr[i], si[i]);
-    __syncthreads();
-    if (warp != 0 || !active) return;
+    auto square = [](int3 k) { return k.x * k.x + k.y * k.y + k.z * k.z; };
+    int np[kReduceC], nm[kReduceC];
 #pragma unroll
     for (int i = 0; i < kReduceC; ++i) {
+        int3 p, m;
+        frequencies(i, p, m);
+        // elements off the lattice are not stored: keep their table reads inside it
+        auto inside = [&](int3 k) { return abs(2 * k.x) <= f.kx && abs(2 * k.y) <= f.ky; };
+        np[i] = inside(p) ? square(p) : 0;
+        nm[i] = inside(m) ? square(m) : 0;
+    }
+    PairSum s = {};
+    if (active)
+        for (int j = f.warp_rows ? 0 : warp; j < f.n_list; j += f.warp_rows ? 1 : kReduceWarps)
+            reduce_add(s_jobs[j], rep, P.fold, bl, c0, np, nm, s);
+    if (!f.warp_rows) {
+#pragma unroll
+        for (int i = 0; i < kReduceC; ++i) {
+            s_part[(warp * 2 * kReduceC + i) * 32 + lane] = make_double2(s.pr[i], s.pi[i]);
+            s_part[(warp * 2 * kReduceC + kReduceC + i) * 32 + lane] = make_double2(s.mr[i], s.mi[i]);
+        }
+        __syncthreads();
+        // warp w adds up the eight partial sums of slot w: plus column w, or minus column w - 4
         double tr = 0.0, ti = 0.0;
         for (int w = 0; w < kReduceWarps; ++w) {
-            const double2 v = s_part[(w * 32 + lane) * kReduceC + i];
+            const double2 v = s_part[(w * 2 * kReduceC + warp) * 32 + lane];
             tr += v.x;
             ti += v.y;
         }
-        store(i, tr, ti);
+#pragma unroll
+        for (int i = 0; i < kReduceC; ++i) {  // the other slots are not this warp's to store
+            s.pr[i] = s.mr[i] = tr;
+            s.pi[i] = s.mi[i] = ti;
+        }
+    }
+    if (!active) return;
+    // spectrum element k += its FP64 sum, with the factored Phi^
+    auto store = [&](int3 k, double tr, double ti) {
+        const int x = k.x + f.kx / 2, y = k.y + f.ky / 2;
+        if ((unsigned)x >= (unsigned)f.kx || (unsigned)y >= (unsigned)f.ky) return;
+        double factor = f.scale;
+        if (f.factored) factor *= phi_fp64(f.basis, f.step * sqrt((double)square(k)) * f.h);
+        const size_t idx = ((size_t)x * f.ky + y) * f.lz_out + k.z;
+        const float2 o = f.out[idx];
+        f.out[idx] = make_float2(o.x + (float)(tr * factor), o.y + (float)(ti * factor));
+    };
+#pragma unroll
+    for (int i = 0; i < kReduceC; ++i) {
+        int3 p, m;
+        frequencies(i, p, m);
+        if (P.write_plus && (f.warp_rows || warp == i)) store(p, s.pr[i], s.pi[i]);
+        // an exchanged part's mirror is along the columns: the conjugate B
+        if (key >= P.min_minus && (f.warp_rows || warp == kReduceC + i))
+            store(m, s.mr[i], P.kind == kPartExchanged ? -s.mi[i] : s.mi[i]);
     }
 }
 
@@ -1761,19 +1694,20 @@ bool tc_pairs_enabled() {
     return v && (active_tune().tc_shapes & kTileCtaPairs);
 }
 
-// Stages per TMEM accumulation chain before a flush into the FP32 total.
-// The single-accumulator tiles (kWide, kPair) stall the MMA for every flush
-// and take the tuned value (default 16: 4.1e-6 rel-L2 on C3 against 2.6e-6 at
-// 8, for 11% more speed); the double-buffered kNarrow tile hides its flushes
-// and keeps chains of at most 8.  MV_TC_FLUSH_STAGES (1..1024) overrides both.
-int tc_flush_stages(int mode) {
+// Stages per TMEM accumulation chain before a flush into the FP32 total.  The
+// chain's length sets the tensor form's error (kChainGain): pure-phase
+// and h-binned jobs take 8 stages of 64 particles, Gaussian jobs of the
+// single-accumulator tiles (kWide, kPair), which stall the MMA for every
+// flush, the tuned value (16: 84 ms on 2^20 particles and 256^3, 90 at 8),
+// and the narrow tiles at most 8.  MV_TC_FLUSH_STAGES (1..1024) overrides all.
+int tc_flush_stages(int mode, bool gauss) {
     static const int env = [] {
         const char* e = std::getenv("MV_TC_FLUSH_STAGES");
         const int x = e ? std::atoi(e) : 0;
         return (x >= 1 && x <= 1024) ? x : 0;
     }();
     if (env) return env;
-    return narrow_mode(mode) ? std::min(8, active_tune().tc_flush) : active_tune().tc_flush;
+    return narrow_mode(mode) || !gauss ? std::min(8, active_tune().tc_flush) : active_tune().tc_flush;
 }
 
 // B-operand images are made for jobs whose every image is copied by at
@@ -2016,12 +1950,13 @@ int tensor_sum_available(const SumRequest& r, int form) {
 namespace {
 
 // Groups whose slots one reduction sums into one output (an output class):
-// same output spectrum and the same per-frequency factor (none for Gaussian
-// and h-binned jobs, whose factors are applied per particle or per Chebyshev
-// block; Phi^(|k| h) with the same basis and h for factored ones).
+// same output spectrum, the same row layout and the same per-frequency factor
+// (none for Gaussian and h-binned jobs, whose factors are applied per particle
+// or per Chebyshev block; Phi^(|k| h) with the same basis and h for factored
+// ones).
 struct ClassKey {
     const float2* out;
-    int unfactored;
+    int unfactored;  // 0 factored, 1 Gaussian factors, 2 h-binned
     int basis;
     double h;
     bool operator==(const ClassKey& o) const {
@@ -2045,8 +1980,6 @@ int tensor_plan(const std::vector<SumRequest>& groups, TensorPlan& plan) {
         int cost_class = 0, m_block = 0;
     };
     std::vector<Item> items;
-    plan.flush_narrow = tc_flush_stages(kNarrow);
-    plan.flush = tc_flush_stages(kWide);
     // Tiles and particle splits of a job (rows kx * ky, columns lz_tc), its
     // items appended, B-operand images where the job allows them (image_ok)
     // and they fit the limit; returns the job's index.
@@ -2056,8 +1989,7 @@ int tensor_plan(const std::vector<SumRequest>& groups, TensorPlan& plan) {
     double launch_terms = 1.0;
     for (const SumRequest& r : groups)
         launch_terms += (double)std::max(0, r.n) * r.lat.nx * r.lat.ny * std::max(1, r.lat.nz - 1);
-    auto add_job = [&](TcJob j, int mode, bool image_ok, size_t tp_offset, int cls, int acc_part,
-                       size_t coef_offset) {
+    auto add_job = [&](TcJob j, int mode, bool image_ok, size_t tp_offset, int cls, int part, size_t coef_offset) {
         // equal n-tiles of at most kNc c values: 192 planes -> 96 + 96 (two
         // N = 192 MMAs) rather than 128 + 64 (an N = 128 one, bound by its
         // shared-memory operand reads); multiples of 16 for kPair
@@ -2067,22 +1999,23 @@ int tensor_plan(const std::vector<SumRequest>& groups, TensorPlan& plan) {
         j.nc_tile = ((j.lz_tc + j.n_ntiles - 1) / j.n_ntiles + nc_unit - 1) / nc_unit * nc_unit;
         j.n_ntiles = (j.lz_tc + j.nc_tile - 1) / j.nc_tile;
         const int ctas = pair_mode(mode) ? 2 : 1;
-        // the last m-tile may extend past the rows (Nyquist jobs): the flush
-        // skips rows >= kx * ky
-        j.n_mtiles = (int)(((long long)j.kx * j.ky + kM * ctas - 1) / (kM * ctas));
+        // the last m-tile may extend past the representatives: the reduction
+        // does not read them
+        j.n_mtiles = (int)(((long long)j.kx * j.ky + kReps * ctas - 1) / (kReps * ctas));
         // particle splits: items of at most the launch's terms / (units x
-        // tc_waves) (default 4 waves), at least 64 stages each; every split
+        // tc_waves) (default 4 waves), at least 32 stages each; every split
         // is one more slot to write and reduce
         const long long ftiles = (long long)j.n_mtiles * j.n_ntiles;
         const double item_budget = launch_terms / ((double)(device_sm_count() / ctas) * active_tune().tc_waves);
         long long splits = std::max<long long>(
             1, (long long)std::ceil((double)j.n * kM * ctas * std::min(j.nc_tile, j.lz_tc) / item_budget));
-        splits = std::min<long long>(splits, std::max<long long>(1, (j.n + 64 * kKp - 1) / (64 * kKp)));
+        splits = std::min<long long>(splits, std::max<long long>(1, (j.n + 32 * kKp - 1) / (32 * kKp)));
         // The 128-column tiles keep an item's whole sum in an FP32 total: at
         // most kMaxItemChains chains per item.  The 256-column tiles take items
         // of any length: their items add the FP32 total of every
         // kMaxItemChains chains into FP64 totals in the slot.
-        const int flush_stages = narrow_mode(mode) ? plan.flush_narrow : plan.flush;
+        const int flush_stages = tc_flush_stages(mode, j.gauss != 0);
+        j.flush = flush_stages;
         const long long max_chunk = (long long)kMaxItemChains * flush_stages * kKp;
         if (narrow_mode(mode)) splits = std::max<long long>(splits, (j.n + max_chunk - 1) / max_chunk);
         const long long chunk = ((j.n + splits - 1) / splits + kKp - 1) / kKp * kKp;
@@ -2108,8 +2041,6 @@ int tensor_plan(const std::vector<SumRequest>& groups, TensorPlan& plan) {
         plan.jobs.push_back(j);
         plan.bimg_offset.push_back(img_off);
         plan.job_tp.push_back(tp_offset);
-        plan.job_class.push_back(cls);
-        plan.job_acc.push_back(acc_part);
         plan.job_coef.push_back(coef_offset);
         plan.job_slot.push_back(plan.slot_bytes);
         plan.slot_bytes += (size_t)(splits * ftiles) * (size_t)j.slot_stride * (j.slot_fp64 ? 8 : 4);
@@ -2123,24 +2054,42 @@ int tensor_plan(const std::vector<SumRequest>& groups, TensorPlan& plan) {
             const int h = c_in / bnc, cc = c_in - h * bnc;
             plan.colmaps.push_back(make_int4(n_tile, h * 2 * bnc + cc, h * 2 * bnc + bnc + cc, 0));
         }
-        TensorPlan::Class& cl = plan.classes[cls];
-        (acc_part == 0 ? cl.jobs : acc_part == 1 ? cl.nyq_pos : cl.nyq_neg).push_back(job_index);
-        const int flush = narrow_mode(mode) ? plan.flush_narrow : plan.flush;
+        plan.classes[cls].parts[part].jobs.push_back(job_index);
         for (long long ks = 0; ks < splits; ++ks) {
             const long long k0 = ks * chunk, k1 = std::min<long long>(j.n, k0 + chunk);
             const long long stages = (k1 - k0 + kKp - 1) / kKp;
             for (long long t = 0; t < ftiles; ++t)
-                items.push_back({mode, stages + (stages + flush - 1) / flush, make_int2(job_index, (int)(ks * ftiles + t)),
+                items.push_back({mode, stages + (stages + flush_stages - 1) / flush_stages, make_int2(job_index, (int)(ks * ftiles + t)),
                                  (int)(t / j.n_ntiles), (int)ks});
         }
         return job_index;
     };
-    // tile mode of a job with `cols` columns over kx * ky rows: kNarrow up to
-    // 64 columns; beyond, kPair where every n-tile splits into two halves of
-    // 8-c chunks and the rows into 256-row m-tiles, else kWide
-    auto mode_of = [](int cols, long long rows) {
-        const bool pairs = tc_pairs_enabled() && cols % 16 == 0 && rows % 256 == 0;
+    // tile mode of a job with `cols` columns over `reps` row representatives:
+    // kNarrow up to 64 columns; beyond, kPair where every n-tile splits into
+    // two halves of 8-c chunks and the pairs' m-tiles of 128 representatives
+    // waste at most an eighth, else kWide
+    auto mode_of = [](int cols, long long reps) {
+        const long long tiles = (reps + 2 * kReps - 1) / (2 * kReps);
+        const bool pairs = tc_pairs_enabled() && cols % 16 == 0 && tiles * 2 * kReps * 8 <= reps * 9;
         return cols <= Shape<kNarrow>::kNc ? (pairs ? kPairNarrow : kNarrow) : (pairs ? kPair : kWide);
+    };
+    // where a part's elements lie in the spectrum
+    auto set_part = [&](int cls, int part, int kind, const TcJob& j, int mirror_a, int mirror_b, int min_minus,
+                        int write_plus, int fixed) {
+        TcPart& p = plan.classes[cls].parts[part].geometry;
+        p.kind = kind;
+        p.n_reps = j.kx * j.ky;
+        p.rows = j.ky;
+        p.fold = std::max(1, j.fold);
+        p.a_base = j.a_base;
+        p.b_base = j.b_base;
+        p.c_base = j.c_base;
+        p.columns = j.period > 0 ? j.period : j.lz_tc;
+        p.mirror_a = mirror_a;
+        p.mirror_b = mirror_b;
+        p.min_minus = min_minus;
+        p.write_plus = write_plus;
+        p.fixed = fixed;
     };
     for (size_t g = 0; g < groups.size(); ++g) {
         const SumRequest& r = groups[g];
@@ -2149,7 +2098,7 @@ int tensor_plan(const std::vector<SumRequest>& groups, TensorPlan& plan) {
         const bool uniform = r.radii && r.radius_min >= 0.f && r.radius_min == r.radius_max;
         const bool gauss = r.radii && !uniform && r.basis == kGaussianDecaying;
         const bool binned = !gauss && binned_group(r);
-        ClassKey key{r.out, (gauss || binned) ? 1 : 0, r.basis, uniform ? (double)r.radius_max : 1.0};
+        ClassKey key{r.out, gauss ? 1 : binned ? 2 : 0, r.basis, uniform ? (double)r.radius_max : 1.0};
         int cls = -1;
         for (size_t c = 0; c < keys.size(); ++c)
             if (keys[c] == key) cls = (int)c;
@@ -2160,28 +2109,25 @@ int tensor_plan(const std::vector<SumRequest>& groups, TensorPlan& plan) {
             c.out = r.out;
             c.kx = kx;
             c.ky = ky;
-            c.lz_tc = lz_tc;
             c.lz_out = lz_out;
             c.step = L.kx;
             c.basis = r.basis;
             c.h = key.h;
             c.factored = !key.unfactored;
             c.scale = r.scale;
-            c.nyquist = false;
             plan.classes.push_back(c);
         }
         plan.group_class.push_back(cls);
         plan.group_binned.push_back(-1);
         plan.nyq_job_of_group.push_back(-1);
+        plan.face_job_of_group.push_back(-1);
         plan.tp_nyq_offset.push_back(0);
         plan.tp_offset.push_back(plan.tp_bytes);
         if (r.n <= 0 || !(r.weight_max > 0.f)) {
             plan.job_of_group.push_back(-1);
             continue;
         }
-        const bool nyq_ok = ky % 16 == 0 && kx % 2 == 0 && (kx / 2) % 8 == 0;
-        // the class's Nyquist plane comes from transposed jobs
-        auto class_nyquist = [&]() { plan.classes[cls].nyquist = true; };
+        const bool nyq_ok = ky % 16 == 0 && kx % 16 == 0;
         if (binned) {
             // ------------------------------------------ h-binned group
             const std::shared_ptr<const HBinPlan> hp = hbin_plan(r);
@@ -2220,13 +2166,12 @@ int tensor_plan(const std::vector<SumRequest>& groups, TensorPlan& plan) {
             plan.coef_bytes += (bg.coef_count * sizeof(float) + 255) / 256 * 256;
             const size_t blocks_bytes = (size_t)blocks * kBlockBytes;
             plan.tp_bytes += blocks_bytes;
-            // the Nyquist plane as transposed jobs needs whole 8-c blocks of
-            // Kx/2 columns (and 16 for pairs, per job below)
+            // the Nyquist plane as a transposed job needs whole 8-column
+            // blocks of either sign of a
             const bool nyq = nyq_ok;
             if (nyq) {
                 plan.tp_nyq_offset.back() = plan.tp_bytes;
                 plan.tp_bytes += blocks_bytes;
-                class_nyquist();
             }
             size_t coef_at = 0;
             int first_job = -1, first_nyq = -1;
@@ -2237,10 +2182,10 @@ int tensor_plan(const std::vector<SumRequest>& groups, TensorPlan& plan) {
                 coef_at += (size_t)bin.order;
                 if (bin.count <= 0 || !(bin.wmax > 0.f)) continue;
                 TcJob j{};
-                j.kx = kx;
+                j.kx = kx / 2;
                 j.ky = ky / bfold;
                 j.lz_tc = bin.order * lz_tc * bfold;  // column blocks q bfold + bl of lz_tc planes
-                j.a_base = -kx / 2;
+                j.a_base = 0;
                 j.b_base = -ky / 2;
                 j.c_base = 0;
                 j.n = bin.count;
@@ -2250,26 +2195,27 @@ int tensor_plan(const std::vector<SumRequest>& groups, TensorPlan& plan) {
                 j.fold = bfold;
                 j.coef_stride = bg.total_q;
                 const size_t tp = plan.tp_offset.back() + (size_t)first_block[b] * kBlockBytes;
-                const int jm = add_job(j, mode_of(j.lz_tc, (long long)kx * j.ky), true, tp, cls, 0, coef_off);
-                if (first_job < 0) first_job = jm;
+                const int jm = add_job(j, mode_of(j.lz_tc, (long long)j.kx * j.ky), true, tp, cls, 0, coef_off);
+                if (first_job < 0) {
+                    first_job = jm;
+                    set_part(cls, 0, kPartPlanes, j, -1, -bfold, INT32_MIN, 1, 0);
+                }
                 if (nyq) {
                     TcJob t = j;
                     t.kx = 1;
-                    t.ky = ky;
-                    t.lz_tc = bin.order * (kx / 2);
-                    t.period = kx / 2;
+                    t.ky = ky / 2;
+                    t.lz_tc = bin.order * kx;
+                    t.period = kx;
                     t.fold = 0;
-                    t.a_base = lz_tc;
-                    t.b_base = -ky / 2;
-                    t.c_base = 0;
-                    const int nmode = mode_of(t.lz_tc, ky);
+                    t.a_base = 0;
+                    t.b_base = 0;
+                    t.c_base = -kx / 2;
                     const size_t tpn = plan.tp_nyq_offset.back() + (size_t)first_block[b] * kBlockBytes;
-                    const int jn = add_job(t, nmode, false, tpn, cls, 1, coef_off);
-                    if (first_nyq < 0) first_nyq = jn;
-                    t.a_base = -lz_tc;
-                    t.b_base = 1 - ky / 2;
-                    t.c_base = 1;
-                    add_job(t, nmode, false, tpn, cls, 2, coef_off);
+                    const int jn = add_job(t, mode_of(t.lz_tc, t.ky), false, tpn, cls, 1, coef_off);
+                    if (first_nyq < 0) {
+                        first_nyq = jn;
+                        set_part(cls, 1, kPartNyquist, t, 0, -1, INT32_MIN, 1, lz_tc);
+                    }
                 }
             }
             plan.job_of_group.push_back(first_job);
@@ -2282,73 +2228,74 @@ int tensor_plan(const std::vector<SumRequest>& groups, TensorPlan& plan) {
         const size_t blocks_bytes =
             (size_t)((std::max(0, r.n) + kBlockParticles - 1) / kBlockParticles) * kBlockBytes;
         plan.tp_bytes += blocks_bytes;
-        const int mode = mode_of(lz_tc, (long long)kx * ky);
         // Row fold of a group whose terms are pure phases: the F of {1, 2, 4}
         // whose columns F lz_tc fill the MMAs best.  A CTA-pair (or narrow)
         // MMA costs about the same whatever its N up to 256 (128 c values),
         // so the cost per column is n-tiles / columns.
+        auto cost = [](int cols) {
+            const int nc_max = cols <= Shape<kNarrow>::kNc ? Shape<kNarrow>::kNc : Shape<kWide>::kNc;
+            return (double)((cols + nc_max - 1) / nc_max) / cols;
+        };
         int fold = 1;
-        if (!gauss && tc_fold_enabled()) {
-            auto cost = [&](int f) {
-                const int cols = f * lz_tc;
-                const int nc_max = cols <= Shape<kNarrow>::kNc ? Shape<kNarrow>::kNc : Shape<kWide>::kNc;
-                return (double)((cols + nc_max - 1) / nc_max) / cols;
-            };
+        if (!gauss && tc_fold_enabled())
             for (int f : {2, 4})
-                if (ky % (16 * f) == 0 && cost(f) < cost(fold) * 0.99) fold = f;
-        }
-        // Axis exchange of a group that cannot fold (per-particle Gaussian
-        // factors): rows (a, c), columns b, where Ky columns fill the MMAs
-        // better than the planes (384^3: 3 n-tiles of 128 b values instead of
-        // 96 + 96 planes)
-        bool exch = false;
-        if (fold == 1 && tc_exchange_enabled()) {
-            auto cost = [&](int cols) {
-                const int nc_max = cols <= Shape<kNarrow>::kNc ? Shape<kNarrow>::kNc : Shape<kWide>::kNc;
-                return (double)((cols + nc_max - 1) / nc_max) / cols;
-            };
-            exch = ky % 16 == 0 && ((long long)kx * lz_tc) % 256 == 0 && cost(ky) < cost(lz_tc) * 0.99;
-        }
+                if (ky % (16 * f) == 0 && cost(f * lz_tc) < cost(fold * lz_tc) * 0.99) fold = f;
+        // Axis exchange of a Gaussian group: rows (a, c), columns b >= 0, where
+        // Ky / 2 columns fill the MMAs better than the planes
+        const bool exch = gauss && tc_exchange_enabled() && cost(ky / 2) < cost(lz_tc) * 0.99;
         TcJob j{};
-        j.kx = kx;
+        j.kx = exch ? kx : gauss ? kx / 2 + 1 : kx / 2;
         j.ky = exch ? lz_tc : ky / fold;
-        j.lz_tc = exch ? ky : fold * lz_tc;
-        j.a_base = -kx / 2;
+        j.lz_tc = exch ? ky / 2 : fold * lz_tc;
+        j.a_base = exch ? -kx / 2 : 0;
         j.b_base = exch ? 0 : -ky / 2;
-        j.c_base = exch ? -ky / 2 : 0;
+        j.c_base = 0;
         j.n = r.n;
         j.gauss = gauss ? 1 : 0;
         j.wmax = r.weight_max;
         j.fold = fold;
         j.period = fold > 1 ? lz_tc : 0;
         j.exch = exch ? 1 : 0;
-        plan.job_of_group.push_back(add_job(j, mode_of(j.lz_tc, (long long)kx * j.ky), true, plan.tp_offset.back(),
+        j.unit_col = gauss ? 1 : 0;
+        plan.job_of_group.push_back(add_job(j, mode_of(j.lz_tc, (long long)j.kx * j.ky), true, plan.tp_offset.back(),
                                             cls, 0, SIZE_MAX));
-        // The Nyquist plane as two transposed jobs (rows b, columns a >= 0 and
-        // -a > 0; see TcJob) in the same launch, where the Kx / 2 columns of
-        // each split into whole n-tile units (16 c for kPair, else 8);
-        // otherwise the plain form sums it.  Their Ky rows (8-row chunks of one
-        // sign of b) need not fill the last m-tile.
-        if (nyq_ok && (kx / 2) % (pair_mode(mode) ? 16 : 8) == 0) {
+        // mirrors: pure phases in (-1/2, -F/2), every one; Gaussians in 0,
+        // where a = 0 (exchanged: b = 0) is its own
+        if (exch) set_part(cls, 0, kPartExchanged, j, 0, 0, 1, 1, 0);
+        else if (gauss) set_part(cls, 0, kPartPlanes, j, 0, 0, 1, 1, 0);
+        else set_part(cls, 0, kPartPlanes, j, -1, -fold, INT32_MIN, 1, 0);
+        // The Nyquist plane as a transposed job (rows b >= 0 with their
+        // mirrors, columns a) in the same launch, where its 8-column blocks
+        // hold one sign of a; otherwise the plain form sums it.
+        TcJob t = j;
+        t.kx = 1;
+        t.a_base = 0;
+        t.b_base = 0;
+        t.fold = 0;
+        t.period = 0;
+        t.exch = 0;
+        t.unit_col = 0;
+        if (nyq_ok) {
             plan.tp_nyq_offset.back() = plan.tp_bytes;
             plan.tp_bytes += blocks_bytes;
-            TcJob t = j;
-            t.kx = 1;
-            t.ky = ky;
-            t.lz_tc = kx / 2;
-            t.a_base = lz_tc;
-            t.b_base = -ky / 2;
-            t.c_base = 0;
-            t.fold = 0;
-            t.period = 0;
-            t.exch = 0;
+            t.ky = gauss ? ky / 2 + 8 : ky / 2;  // Gaussians: up to b = Ky/2, whose mirror is -Ky/2
+            t.lz_tc = kx;
+            t.c_base = -kx / 2;
             const size_t tpn = plan.tp_nyq_offset.back();
-            plan.nyq_job_of_group.back() = add_job(t, mode, false, tpn, cls, 1, SIZE_MAX);  // one m-tile: no reuse
-            t.a_base = -lz_tc;
-            t.b_base = 1 - ky / 2;
-            t.c_base = 1;
-            add_job(t, mode, false, tpn, cls, 2, SIZE_MAX);
-            class_nyquist();
+            plan.nyq_job_of_group.back() = add_job(t, mode_of(kx, t.ky), false, tpn, cls, 1, SIZE_MAX);  // no reuse
+            if (gauss) set_part(cls, 1, kPartNyquist, t, 0, 0, 1, 1, lz_tc);
+            else set_part(cls, 1, kPartNyquist, t, 0, -1, INT32_MIN, 1, lz_tc);
+        }
+        // Gaussians: the elements at b = -Ky/2 that are no mirror of a
+        // representative: those of a < 0 (exchanged: of every a)
+        if (gauss) {
+            const size_t tpf = plan.tp_bytes;
+            plan.tp_bytes += blocks_bytes;
+            t.ky = (kx / 2 + 1 + 7) / 8 * 8;
+            t.lz_tc = lz_tc;
+            t.c_base = 0;
+            plan.face_job_of_group.back() = add_job(t, mode_of(lz_tc, t.ky), false, tpf, cls, 2, SIZE_MAX);
+            set_part(cls, 2, kPartFace, t, 0, 0, 1, exch ? 1 : 0, -ky / 2);
         }
     }
     if (items.size() > (size_t)INT32_MAX) return set_error(kInvalidValue, "tensor sum: too many work items");
@@ -2399,11 +2346,12 @@ int tensor_plan(const std::vector<SumRequest>& groups, TensorPlan& plan) {
     // the jobs' column maps
     plan.colmap_offset = plan.meta_bytes;
     plan.meta_bytes += (plan.colmaps.size() * sizeof(int4) + 255) / 256 * 256;
-    // each class's job lists (planes, Nyquist a >= 0, Nyquist a < 0)
-    for (TensorPlan::Class& c : plan.classes) {
-        c.list_offset = plan.meta_bytes;
-        plan.meta_bytes += ((c.jobs.size() + c.nyq_pos.size() + c.nyq_neg.size()) * sizeof(int) + 255) / 256 * 256;
-    }
+    // each class's job lists, part by part
+    for (TensorPlan::Class& c : plan.classes)
+        for (TensorPlan::Class::Part& p : c.parts) {
+            p.list_offset = plan.meta_bytes;
+            plan.meta_bytes += (p.jobs.size() * sizeof(int) + 255) / 256 * 256;
+        }
     // the binned groups' tables: edges, int4 bins, float4 spans, int first
     // particles (16-byte aligned)
     for (TensorPlan::Binned& bg : plan.binned) {
@@ -2444,12 +2392,10 @@ int tensor_reserve_upload(TensorPlan& plan, TensorWorkspace& ws, cudaStream_t st
         std::memcpy(meta.data() + plan.img_jobs_offset, plan.img_jobs.data(), plan.img_jobs.size() * sizeof(int));
         std::memcpy(meta.data() + plan.img_first_offset, plan.img_first.data(), plan.img_first.size() * sizeof(long long));
     }
-    for (const TensorPlan::Class& c : plan.classes) {
-        int* l = reinterpret_cast<int*>(meta.data() + c.list_offset);
-        for (int v : c.jobs) *l++ = v;
-        for (int v : c.nyq_pos) *l++ = v;
-        for (int v : c.nyq_neg) *l++ = v;
-    }
+    for (const TensorPlan::Class& c : plan.classes)
+        for (const TensorPlan::Class::Part& p : c.parts)
+            if (!p.jobs.empty())
+                std::memcpy(meta.data() + p.list_offset, p.jobs.data(), p.jobs.size() * sizeof(int));
     for (const TensorPlan::Binned& bg : plan.binned) {
         float* edges = reinterpret_cast<float*>(meta.data() + bg.meta_offset);
         const size_t edges_bytes = ((size_t)(bg.nbins + 1) * sizeof(float) + 15) / 16 * 16;
@@ -2625,6 +2571,7 @@ int tensor_enqueue(const std::vector<SumRequest>& groups, const TensorPlan& plan
             bp.spans = reinterpret_cast<const float4*>(bp.bins + bg.nbins);
             bp.out = reinterpret_cast<uint8_t*>(tp);
             bp.out_nyq = reinterpret_cast<uint8_t*>(tpn);
+            bp.half_z = r.lat.nz - 1;
             bp.first = reinterpret_cast<const int*>(bp.spans + bg.nbins);
             char* sorted = static_cast<char*>(ws.sorted.ptr) + bg.sorted_offset;
             bp.sorted = reinterpret_cast<float4*>(sorted);
@@ -2683,6 +2630,10 @@ int tensor_enqueue(const std::vector<SumRequest>& groups, const TensorPlan& plan
         pa.out = const_cast<unsigned char*>(plan.jobs[j].blocks);
         const int t = plan.nyq_job_of_group[g];
         pa.out_nyq = t < 0 ? nullptr : const_cast<unsigned char*>(plan.jobs[t].blocks);
+        const int face = plan.face_job_of_group[g];
+        pa.out_face = face < 0 ? nullptr : const_cast<unsigned char*>(plan.jobs[face].blocks);
+        pa.half_y = L.ny / 2;
+        pa.half_z = L.nz - 1;
         tc_prep_kernel<<<(r.n + 255) / 256, 256, 0, stream>>>(pa);
         count_launch();
     }
@@ -2717,7 +2668,6 @@ int tensor_enqueue(const std::vector<SumRequest>& groups, const TensorPlan& plan
             a.jobs = static_cast<const TcJob*>(plan.d_jobs);
             a.items = static_cast<const int2*>(plan.d_items) + first;
             a.n_items = counts[m];
-            a.flush_stages = narrow_mode(modes[m]) ? plan.flush_narrow : plan.flush;
             a.error_flag = error_flag;
             a.wait_limit_ns = kWaitLimitNs;
             a.withhold_first_arrival = 0;
@@ -2745,50 +2695,34 @@ int tensor_enqueue(const std::vector<SumRequest>& groups, const TensorPlan& plan
         if (st != kOk) return st;
     }
     // the items' tiles -> spectra, summed in FP64 (added to what is there)
-    for (const TensorPlan::Class& c : plan.classes) {
-        const int* lists = reinterpret_cast<const int*>(static_cast<const char*>(ws.meta.ptr) + c.list_offset);
-        TcReduceArgs f;
-        f.jobs = static_cast<const TcJob*>(plan.d_jobs);
-        f.list = lists;
-        f.n_list = (int)c.jobs.size();
-        f.list_neg = nullptr;
-        f.n_neg = 0;
-        f.kx = c.kx;
-        f.ky = c.ky;
-        f.lz_tc = c.lz_tc;
-        f.lz_out = c.lz_out;
-        f.step = c.step;
-        f.basis = c.basis;
-        f.h = c.h;
-        f.factored = c.factored;
-        f.scale = c.scale;
-        f.out = c.out;
-        f.warp_rows = f.n_list < kReduceWarps ? 1 : 0;
-        if (f.n_list > 0) {
-            const int block_rows = f.warp_rows ? 32 * kReduceWarps : 32;
-            const long long blocks =
-                ((long long)c.kx * c.ky + block_rows - 1) / block_rows * (c.lz_tc / kReduceC);
+    for (const TensorPlan::Class& c : plan.classes)
+        for (const TensorPlan::Class::Part& p : c.parts) {
+            if (p.jobs.empty()) continue;
+            TcReduceArgs f;
+            f.jobs = static_cast<const TcJob*>(plan.d_jobs);
+            f.list = reinterpret_cast<const int*>(static_cast<const char*>(ws.meta.ptr) + p.list_offset);
+            f.n_list = (int)p.jobs.size();
+            f.part = p.geometry;
+            f.kx = c.kx;
+            f.ky = c.ky;
+            f.lz_out = c.lz_out;
+            f.step = c.step;
+            f.basis = c.basis;
+            f.h = c.h;
+            f.factored = c.factored;
+            f.scale = c.scale;
+            f.out = c.out;
+            f.warp_rows = f.n_list < kReduceWarps ? 1 : 0;
+            const int block_reps = f.warp_rows ? 32 * kReduceWarps : 32;
+            const long long blocks = (long long)((f.part.n_reps + block_reps - 1) / block_reps) * f.part.fold *
+                                     (f.part.columns / kReduceC);
             const size_t smem = (((size_t)f.n_list * sizeof(ReduceJob) + 15) & ~(size_t)15) +
-                                (size_t)kReduceWarps * 32 * kReduceC * sizeof(double2);
-            st = reduce_smem(tc_reduce_planes_kernel, smem);
-            if (st != kOk) return st;
-            tc_reduce_planes_kernel<<<(unsigned)blocks, 32 * kReduceWarps, smem, stream>>>(f);
-            count_launch();
-        }
-        if (c.nyquist) {
-            f.list = lists + c.jobs.size();
-            f.n_list = (int)c.nyq_pos.size();
-            f.list_neg = lists + c.jobs.size() + c.nyq_pos.size();
-            f.n_neg = (int)c.nyq_neg.size();
-            const long long plane = (long long)c.kx * c.ky;
-            const size_t smem = (((size_t)(f.n_list + f.n_neg) * sizeof(ReduceJob) + 15) & ~(size_t)15) +
-                                (size_t)32 * kReduceWarps * sizeof(double2);
+                                (f.warp_rows ? 0 : (size_t)kReduceWarps * 32 * 2 * kReduceC * sizeof(double2));
             st = reduce_smem(tc_reduce_kernel, smem);
             if (st != kOk) return st;
-            tc_reduce_kernel<<<(unsigned)((plane + 31) / 32), 32 * kReduceWarps, smem, stream>>>(f);
+            tc_reduce_kernel<<<(unsigned)blocks, 32 * kReduceWarps, smem, stream>>>(f);
             count_launch();
         }
-    }
     st = check_cuda(cudaGetLastError(), "tc_reduce_kernel launch");
     if (st != kOk) return st;
     // the branch part of h-binned groups with the plain form, over their
