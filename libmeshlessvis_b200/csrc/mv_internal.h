@@ -275,6 +275,37 @@ struct TcPart {
     int fixed;       // Nyquist: z's frequency; face: y's
 };
 
+// One column block of a job (a Chebyshev order of an h-binned job, else the
+// job) as the reduction reads it; n_splits = 0: none.  Blocks come in fours;
+// an h-binned group's in lines of 32, whose first names the coefficients of
+// all (at [|k|^2][coef_stride], one 128-byte line).
+struct TcReduceBlock {
+    const void* slots;
+    const int4* colmap;  // of the block's first column
+    const float* coef;
+    double scale;        // W x 2^-24
+    int slot_fp64, slot_stride, n_splits, n_mtiles, n_ntiles;
+    int rank_stride;     // elements between the CTAs' parts of a slot: 128 * 2 nc_tile
+    int reps_log2;       // representatives per m-tile: 6 (one CTA) or 7 (CTA pair)
+    int coef_stride;
+};
+
+// One part of an output class: its fours, its blocks of the reduction's grid
+// and the spectrum they go to.
+struct TcReducePart {
+    TcPart part;
+    int first_four, n_fours, first_block;
+    int binned;     // h-binned: the blocks of whole 32-coefficient lines
+    int warp_rows;  // each warp sums every block of its own representatives
+    int simple;     // FP32 slots and one particle chunk in every block
+    int kx, ky, lz_out;
+    int basis;
+    int factored;
+    double step, h;  // h: radius of the factored Phi^(|k| h); 1 without radii
+    double scale;
+    float2* out;
+};
+
 // The h-bins of one binned group on one lattice (tensor_plan): consecutive
 // runs of fine bins, each with its Chebyshev order and weight scale.
 struct HBin {
@@ -302,7 +333,8 @@ struct TensorPlan {
         size_t coef_offset;     // into coef (floats)
         size_t coef_count;
         int nsq;                // |k|^2 / step^2 values: max a^2 + b^2 + c^2 + 1
-        int total_q;            // Chebyshev blocks over all bins: the table's stride per |k|^2
+        int total_q;            // Chebyshev blocks over all bins
+        int coef_stride;        // the table's stride per |k|^2: total_q padded to whole lines
         std::vector<HBin> bins;
         std::vector<float> edges;  // nbins + 1: the fine edges where the bins start (classification)
         size_t sorted_offset;      // into TensorWorkspace::sorted: n float4, n radii, then the radius sort's
@@ -323,15 +355,22 @@ struct TensorPlan {
         // the class's parts: planes, Nyquist plane, face (those with jobs)
         struct Part {
             TcPart geometry;
-            std::vector<int> jobs;   // indices into TensorPlan::jobs
-            size_t list_offset = 0;  // that list in meta (ints)
+            std::vector<int> jobs;  // indices into TensorPlan::jobs
         };
         Part parts[3];
     };
     std::vector<TcJob> jobs;
-    std::vector<int2> items;  // 128x128-tile items (n_narrow), narrow CTA-pair items (n_pair_narrow),
-                              // CTA-pair items (n_pair), then 128x256
-    int n_narrow = 0, n_pair_narrow = 0, n_pair = 0, n_pair_db = 0;
+    // work items (job, local item), tile mode by tile mode, and in each the
+    // units' lists one after the other (list_first: each list's first item and
+    // the last one's end, per launch)
+    std::vector<int2> items;
+    std::vector<int> list_first;
+    size_t list_offset = 0;  // list_first in meta
+    struct Launch {
+        int mode, n_lists, first;  // first: its lists in list_first
+        long long cost;            // of a list, in stages
+    };
+    std::vector<Launch> launches;
     std::vector<Class> classes;
     std::vector<int> group_class, job_of_group;
     std::vector<int> nyq_job_of_group;  // the Nyquist-plane job (h-binned: the first bin's), or -1
@@ -340,6 +379,20 @@ struct TensorPlan {
     // per job: its particle constants (offset into the particles workspace),
     // coefficient table (offset in floats into coef, SIZE_MAX for none)
     std::vector<size_t> job_tp, job_coef, job_slot;  // job_slot: byte offset into slots
+    std::vector<int> job_binned;                     // its binned group, or -1
+    // the reduction: its parts by launch, their column blocks (job, order; job
+    // -1: none) in fours, both in meta
+    std::vector<std::vector<TcReducePart>> reduce_levels;
+    std::vector<size_t> reduce_offset;
+    std::vector<int> reduce_grid;
+    std::vector<int2> reduce_blocks;
+    struct ReduceLine {
+        size_t block;  // a line's first block
+        int binned;    // its binned group and its first coefficient
+        int first_coef;
+    };
+    std::vector<ReduceLine> reduce_lines;
+    size_t reduce_blocks_offset = 0;
     std::vector<size_t> job_colmap;                 // the job's column map: index into colmaps
     std::vector<int4> colmaps;                      // all jobs' column maps
     size_t colmap_offset = 0;                       // colmaps in meta

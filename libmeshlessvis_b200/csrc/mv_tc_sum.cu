@@ -89,6 +89,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <functional>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -155,6 +156,10 @@ constexpr double kInvProductScale = 1.0 / (4096.0 * 4096.0);  // 2^-24
 // frequency 0 of a Gaussian job's columns, whose factors are exactly 1, so
 // that many low bits are 0) loses 0.8e-7: kChainGainUnit.
 constexpr float kChainGain = 2.1e-7f / 64, kChainAgree = 4.f, kChainGainMost = 2.f, kChainGainUnit = 0.4f;
+// What an item costs beside its stages (the pipeline's fill, the last flush
+// and its slot), and a flush of the single-accumulator tiles, in stages (about
+// 1 us each): 2 and 2, measured on the 256^3 set with chains of 4 to 16.
+constexpr int kItemCost = 2;
 // An FP32 total in TMEM sums at most this many accumulation chains (random-walk
 // rounding of about 2^-24 sqrt(64) of the total) before it goes to the item's
 // slot.
@@ -232,8 +237,9 @@ __host__ __device__ constexpr uint32_t mma_idesc(int m, int n) {
 
 struct TcArgs {
     const TcJob* jobs;
-    const int2* items;  // (job, local item), longest first
-    int n_items;
+    const int2* items;      // (job, local item), the units' lists one after the other
+    const int* list_first;  // n_lists + 1: list l is items [list_first[l], list_first[l + 1])
+    int n_lists;
     int* error_flag;
     unsigned long long wait_limit_ns;  // bound of every mbarrier wait (kWaitLimitNs unless a test shortens it)
     int withhold_first_arrival;        // test hook: CTA 0's loader skips its arrival on the first full barrier
@@ -295,6 +301,30 @@ __device__ __forceinline__ TcItem tc_item(const TcArgs& a, int it, int rank) {
              ((size_t)v.y * r.job->slot_stride + (size_t)rank * kM * 2 * r.job->nc_tile) * (r.slot_fp64 ? 8 : 4);
     return r;
 }
+
+// The items of one CTA or CTA pair, in order: every role of it walks them alike.
+struct ItemWalk {
+    const int* first;
+    int list, n_lists, n_units, it, end;
+    __device__ __forceinline__ ItemWalk(const TcArgs& a, int unit, int units)
+        : first(a.list_first), list(unit), n_lists(a.n_lists), n_units(units), it(0), end(0) {
+        open();
+    }
+    __device__ __forceinline__ void open() {
+        while (list < n_lists) {
+            it = __ldg(first + list);
+            end = __ldg(first + list + 1);
+            if (it < end) return;
+            list += n_units;
+        }
+    }
+    __device__ __forceinline__ bool more() const { return list < n_lists; }
+    __device__ __forceinline__ void next() {
+        if (++it < end) return;
+        list += n_units;
+        open();
+    }
+};
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -636,8 +666,8 @@ __device__ __forceinline__ void b_unit(uint8_t* bhi, int bnc, int chunk, int col
     else unit_chain<true, true>(re_base, im_base, lo_gap, c16, X, Y, RX, RY, NRY, Q, RHO);
 }
 
-// Persistent: CTA (or CTA pair) b walks items b, b + grid, ... of the
-// longest-first item list.  Every role walks the same items in the same
+// Persistent: CTA (or CTA pair) u walks the items of lists u, u + grid, ...
+// (tensor_plan makes one list a unit).  Every role walks the same items in the same
 // order, and the pipeline's stage and chain counters (hence mbarrier phases
 // and the TMEM accumulator parity) run on across items; TMEM and the barriers
 // are set up once per CTA.
@@ -725,14 +755,18 @@ __global__ void __launch_bounds__(kThreads, 1) tc_sum_kernel(TcArgs a) {
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
 
+    // the next tile kind's launch, if any, may take the SMs this one leaves
+    // (launch_tile)
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+
     if (warp == 0) {
         // ------------------------------------------------------------- MMA
         // (kPair: CTA 0 issues the pair's MMAs; warp 0 of CTA 1 only
         // allocates and releases TMEM)
         if (lane == 0 && rank == 0) {
             int S = 0, C = 0;  // stages and chains issued so far by this CTA
-            for (int it = unit; it < a.n_items && !*abort_flag; it += n_units) {
-                const TcItem I = tc_item<MODE>(a, it, 0);
+            for (ItemWalk w(a, unit, n_units); w.more() && !*abort_flag; w.next()) {
+                const TcItem I = tc_item<MODE>(a, w.it, 0);
                 const uint32_t idesc = mma_idesc(kM * kCtas, 2 * I.nc);
                 for (int s = 0; s < I.n_stages; ++s, ++S) {
                     const int fb = S % kFull, ab = S % kAStages, bb = S % kBStages;
@@ -771,8 +805,8 @@ __global__ void __launch_bounds__(kThreads, 1) tc_sum_kernel(TcArgs a) {
             // stage instead of one per producer warp)
             if (lane == 0 && rank == 1) {
                 int S = 0;
-                for (int it = unit; it < a.n_items && !*abort_flag; it += n_units) {
-                    const TcItem I = tc_item<MODE>(a, it, 1);
+                for (ItemWalk w(a, unit, n_units); w.more() && !*abort_flag; w.next()) {
+                    const TcItem I = tc_item<MODE>(a, w.it, 1);
                     int s = 0;
                     for (; s < I.n_stages; ++s, ++S) {
                         const int fb = S % kFull;
@@ -790,8 +824,8 @@ __global__ void __launch_bounds__(kThreads, 1) tc_sum_kernel(TcArgs a) {
         const uint32_t lane_base = tmem + ((uint32_t)(quarter * 32) << 16);
         const int row = quarter * 32 + lane;  // M row owned by this thread
         int C = 0;
-        for (int it = unit; it < a.n_items && !__any_sync(0xffffffffu, *abort_flag != 0); it += n_units) {
-            const TcItem I = tc_item<MODE>(a, it, rank);
+        for (ItemWalk w(a, unit, n_units); w.more() && !__any_sync(0xffffffffu, *abort_flag != 0); w.next()) {
+            const TcItem I = tc_item<MODE>(a, w.it, rank);
             const int ncols = 2 * I.nc;
             // FP32 slot: columns n..n+3 (n % 4 == 0) at [(n / 4) * 512 + row * 4];
             // FP64 slot: columns n, n + 1 (n even) at [(n / 2) * 256 + row * 2]
@@ -936,8 +970,8 @@ __global__ void __launch_bounds__(kThreads, 1) tc_sum_kernel(TcArgs a) {
         // ---------------------------------------------------------- loader
         if (lane == 0) {
             int S = 0;
-            for (int it = unit; it < a.n_items && !*abort_flag; it += n_units) {
-                const TcItem I = tc_item<MODE>(a, it, rank);
+            for (ItemWalk w(a, unit, n_units); w.more() && !*abort_flag; w.next()) {
+                const TcItem I = tc_item<MODE>(a, w.it, rank);
                 for (int s = 0; s < I.n_stages; ++s, ++S) {
                     const int buf = S % kSlots;
                     // this CTA's producers have read the slot's constants of stage S - kSlots
@@ -956,8 +990,8 @@ __global__ void __launch_bounds__(kThreads, 1) tc_sum_kernel(TcArgs a) {
             // buffer's previous contents: the copy may then overwrite them, and
             // the arrival cannot count toward the barrier's previous phase.
             int S = 0;
-            for (int it = unit; it < a.n_items && !*abort_flag; it += n_units) {
-                const TcItem I = tc_item<MODE>(a, it, rank);
+            for (ItemWalk w(a, unit, n_units); w.more() && !*abort_flag; w.next()) {
+                const TcItem I = tc_item<MODE>(a, w.it, rank);
                 int s = 0;
                 for (; s < I.n_stages; ++s, ++S) {
                     const int bb = S % kBStages;
@@ -986,8 +1020,8 @@ __global__ void __launch_bounds__(kThreads, 1) tc_sum_kernel(TcArgs a) {
         const bool has_a = pw < 8;   // A unit: chunk pw of 8 representatives; else B unit: c chunks cb, cb + 4, ...
         const int cb = pw - 8;
         int S = 0;
-        for (int it = unit; it < a.n_items && !__any_sync(0xffffffffu, *abort_flag != 0); it += n_units) {
-            const TcItem I = tc_item<MODE>(a, it, rank);
+        for (ItemWalk w(a, unit, n_units); w.more() && !__any_sync(0xffffffffu, *abort_flag != 0); w.next()) {
+            const TcItem I = tc_item<MODE>(a, w.it, rank);
             const int ky = I.job->ky;
             const bool gauss = I.job->gauss != 0;
             const int rho0 = I.row0 + pw * 8;
@@ -1100,6 +1134,9 @@ __global__ void __launch_bounds__(kThreads, 1) tc_sum_kernel(TcArgs a) {
             }
         }
     }
+
+    // a launch that overlaps the one before it does not complete before it
+    asm volatile("griddepcontrol.wait;" ::: "memory");
 
     // ------------------------------------------------------------- teardown
     // a CTA that gave up a wait may still have bulk copies in flight into its
@@ -1307,7 +1344,7 @@ struct TcCoefArgs {
     double step;
     int nbins;
     int nsq;               // |k|^2 / step^2 = 0 .. nsq - 1
-    int total_q;           // the group's Chebyshev blocks over all bins
+    int coef_stride;       // floats per |k|^2: the group's Chebyshev blocks over all bins, padded to fours
     const int4* bins;      // (first block, capacity, first Chebyshev block, order)
     const float4* spans;   // (lo, hi, ...)
     const float* edges;    // the bins' classification edges
@@ -1317,7 +1354,7 @@ struct TcCoefArgs {
 
 // Chebyshev coefficients c_q(|k|) of h -> Phi^(|k| h) on each bin, for every
 // integer |k|^2 / step^2 of the lattice, in FP64, stored as floats:
-// coef[n2 * total_q + q_offset(bin) + q] (one |k|^2's coefficients together,
+// coef[n2 * coef_stride + q_offset(bin) + q] (one |k|^2's coefficients together,
 // as the reduction reads them).  Phi^ is smooth on a bin unless the bin holds
 // r0 / |k| (the reference's branch point, where its slope jumps): for that one
 // bin the smooth closed form is interpolated instead (phi_smooth_fp64), and
@@ -1346,7 +1383,7 @@ __global__ void tc_coef_kernel(TcCoefArgs c) {
         for (int p = 0; p < order; ++p) acc += f[p] * cospi(q * (2.0 * p + 1.0) / (2.0 * order));
         acc *= 2.0 / order;
         if (q == 0) acc *= 0.5;
-        c.coef[(size_t)n2 * c.total_q + bin.z + q] = (float)acc;
+        c.coef[(size_t)n2 * c.coef_stride + bin.z + q] = (float)acc;
     }
 }
 
@@ -1400,39 +1437,6 @@ __global__ void __launch_bounds__(256) tc_bimg_kernel(TcImageArgs g) {
                J.coef != nullptr, pqz, pqy, pob, pgam, gauss, RX, RY, NRY, RHO);
 }
 
-// What the reduction needs of a job, gathered into shared memory once per
-// block (the job table's other fields are not read).
-struct ReduceJob {
-    const void* slots;
-    const int4* colmap;
-    const float* coef;  // null unless h-binned
-    double scale;       // W x 2^-24
-    int slot_fp64;
-    int slot_stride, n_splits, n_mtiles, n_ntiles;
-    int rank_stride;    // elements between the CTAs' parts of a slot: 128 * 2 nc_tile
-    int reps_log2;      // representatives per m-tile: 6 (one CTA) or 7 (CTA pair)
-    int period, blocks, coef_stride;
-};
-
-__device__ __forceinline__ ReduceJob reduce_job(const TcJob& J) {
-    ReduceJob r;
-    r.slots = J.slots;
-    r.slot_fp64 = J.slot_fp64;
-    r.colmap = J.colmap;
-    r.coef = J.period > 0 ? J.coef : nullptr;
-    r.scale = J.wmax * kInvProductScale;
-    r.slot_stride = J.slot_stride;
-    r.n_splits = J.n_splits;
-    r.n_mtiles = J.n_mtiles;
-    r.n_ntiles = J.n_ntiles;
-    r.rank_stride = kM * 2 * J.nc_tile;
-    r.reps_log2 = J.ctas == 2 ? 7 : 6;
-    r.period = J.period;
-    r.blocks = J.period > 0 ? J.lz_tc / J.period / (J.fold > 1 ? J.fold : 1) : 1;
-    r.coef_stride = J.coef_stride;
-    return r;
-}
-
 constexpr int kReduceC = 4;
 
 // The four accumulators (Re A, Im A) x (Re B, Im B) of one representative and
@@ -1441,7 +1445,7 @@ struct Quad {
     double cc[kReduceC], cs[kReduceC], sc[kReduceC], ss[kReduceC];
 };
 
-__device__ __forceinline__ void quad_load(const ReduceJob& J, size_t base, int rl, int4 m, Quad& t) {
+__device__ __forceinline__ void quad_load(const TcReduceBlock& J, size_t base, int rl, int4 m, Quad& t) {
     // FP32 slots: column n (a multiple of 4) of row r at (n / 4) * 512 + 4 r,
     // four columns in one load, a warp's rows 512 contiguous bytes; FP64:
     // column n (even) at (n / 2) * 256 + 2 r
@@ -1480,89 +1484,120 @@ struct PairSum {
     double pr[kReduceC], pi[kReduceC], mr[kReduceC], mi[kReduceC];
 };
 
-// Adds one job's contribution at row representative rep and the kReduceC
-// columns from c0 of every Chebyshev block's b offset bl (they share one
-// n-tile and one CTA half, as n-tiles and halves hold multiples of 8
-// columns): the totals of all its particle chunks (FP32 or FP64 slots) summed
-// in FP64, each h-binned block weighted by its coefficients at the two
-// elements' |k|^2 = np[i] step^2 and nm[i] step^2, times W 2^-24.
-__device__ __forceinline__ void reduce_add(const ReduceJob& J, int rep, int fold, int bl, int c0, const int* np,
-                                           const int* nm, PairSum& f) {
+// Adds one column block of one job at row representative rep and the kReduceC
+// columns from column col of the block (they share one n-tile and one CTA
+// half, as n-tiles and halves hold multiples of 8 columns): the totals of all
+// its particle chunks (FP32 or FP64 slots) summed in FP64, times W 2^-24 and
+// (h-binned) its Chebyshev coefficients wp[i] and wm[i] at the two elements.
+__device__ __forceinline__ void reduce_add(const TcReduceBlock& J, int rep, int col, bool weighted, const float* wp,
+                                           const float* wm, PairSum& f) {
     const int m_tile = rep >> J.reps_log2, within = rep - (m_tile << J.reps_log2);
     const int rl = within & (kReps - 1);
     const size_t rbase = (size_t)(within / kReps) * J.rank_stride;
-    for (int q = 0; q < J.blocks; ++q) {
-        const int4 m = __ldg(J.colmap + (q * fold + bl) * J.period + c0);  // the same for a warp's rows
-        float wp[kReduceC], wm[kReduceC];
-        if (J.coef) {
+    const int4 m = __ldg(J.colmap + col);  // the same for a warp's rows
+    Quad t = {};
+    for (int ks = 0; ks < J.n_splits; ++ks) {
+        const size_t li = ((size_t)ks * J.n_mtiles + m_tile) * J.n_ntiles + m.x;
+        quad_load(J, li * J.slot_stride + rbase, rl, m, t);
+    }
 #pragma unroll
-            for (int i = 0; i < kReduceC; ++i) {
-                wp[i] = __ldg(J.coef + (size_t)np[i] * J.coef_stride + q);
-                wm[i] = __ldg(J.coef + (size_t)nm[i] * J.coef_stride + q);
-            }
-        }
-        Quad t = {};
-        for (int ks = 0; ks < J.n_splits; ++ks) {
-            const size_t li = ((size_t)ks * J.n_mtiles + m_tile) * J.n_ntiles + m.x;
-            quad_load(J, li * J.slot_stride + rbase, rl, m, t);
-        }
-#pragma unroll
-        for (int i = 0; i < kReduceC; ++i) {
-            const double up = J.coef ? (double)wp[i] * J.scale : J.scale;
-            const double um = J.coef ? (double)wm[i] * J.scale : J.scale;
-            f.pr[i] = fma(up, t.cc[i] - t.ss[i], f.pr[i]);
-            f.pi[i] = fma(up, t.cs[i] + t.sc[i], f.pi[i]);
-            f.mr[i] = fma(um, t.cc[i] + t.ss[i], f.mr[i]);
-            f.mi[i] = fma(um, t.cs[i] - t.sc[i], f.mi[i]);
-        }
+    for (int i = 0; i < kReduceC; ++i) {
+        const double up = weighted ? (double)wp[i] * J.scale : J.scale;
+        const double um = weighted ? (double)wm[i] * J.scale : J.scale;
+        f.pr[i] = fma(up, t.cc[i] - t.ss[i], f.pr[i]);
+        f.pi[i] = fma(up, t.cs[i] + t.sc[i], f.pi[i]);
+        f.mr[i] = fma(um, t.cc[i] + t.ss[i], f.mr[i]);
+        f.mi[i] = fma(um, t.cs[i] - t.sc[i], f.mi[i]);
     }
 }
 
-// The jobs of one part (planes, Nyquist plane, b = -Ky/2 face) of one output
-// class (same spectrum, same per-frequency factor, same row layout) -> its
-// float2 spectrum, added, times the factored Phi^(|k| h) in FP64 and the
-// scale.  A thread takes one row representative, one b offset and kReduceC
-// columns, and writes both elements its accumulators hold.
-//
-// With the job list split over warps (parts of at least 8 jobs): a block
-// takes 32 representatives (lanes), warp w sums jobs w, w + 8, ..., and the
-// eight partial sums are added in warp order (a fixed order: the result does
-// not depend on timing), so eight independent load chains per element hide
-// the slots' latency.  With fewer jobs (f.warp_rows; one group per class, as
-// in a batch of particle sets) a block takes 8 x 32 representatives and each
-// warp sums every job of its own 32 in job order, so no warp idles.
-struct TcReduceArgs {
-    const TcJob* jobs;
-    const int* list;
-    int n_list;
-    TcPart part;
-    int kx, ky, lz_out;
-    double step;
-    int basis;
-    double h;  // radius of the factored Phi^(|k| h); 1 without radii
-    bool factored;
+// Where a representative's accumulators of an FP32 block of one particle chunk
+// lie (null: no job), so that the loads of the next blocks can be issued
+// before the sums of these.
+__device__ __forceinline__ float component(const float4& v, int i) {
+    return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w;
+}
+struct BlockAt {
+    const float *re, *im;
     double scale;
-    float2* out;
-    int warp_rows;  // every warp sums all jobs of its own 32 representatives (parts of fewer jobs than warps)
+};
+__device__ __forceinline__ BlockAt block_at(const TcReduceBlock& J, int rep, int col) {
+    BlockAt b;
+    b.re = b.im = nullptr;
+    b.scale = 0.0;
+    if (J.n_splits == 0) return b;
+    const int4 m = __ldg(J.colmap + col);
+    const int m_tile = rep >> J.reps_log2, within = rep - (m_tile << J.reps_log2);
+    const float* v = static_cast<const float*>(J.slots) + ((size_t)m_tile * J.n_ntiles + m.x) * J.slot_stride +
+                     (size_t)(within / kReps) * J.rank_stride + (within & (kReps - 1)) * 4;
+    b.re = v + (size_t)m.y * kM;
+    b.im = v + (size_t)m.z * kM;
+    b.scale = J.scale;
+    return b;
+}
+
+// The jobs of every part (planes, Nyquist plane, b = -Ky/2 face) of the output
+// classes -> their float2 spectra, added, times the factored Phi^(|k| h) in
+// FP64 and the scale: one launch for all parts that no two classes share a
+// spectrum in (tensor_plan's levels), block by block found in the parts'
+// block ranges.  (A launch a part took 20 us each for the Nyquist planes of a
+// batch of 16 sets, latency only: 1.2 ms of its 18.4 ms.)  A thread takes one
+// row representative, one b offset and kReduceC columns, and writes both
+// elements its accumulators hold.
+//
+// A part's column blocks (job, Chebyshev order) come in fours.  With the fours
+// split over warps (h-binned parts, and others of at least kReduceWarps fours):
+// a block takes 32 representatives (lanes), warp w sums fours w, w + 8, ...,
+// and the eight partial sums are added in warp order (a fixed order: the
+// result does not depend on timing), so eight independent load chains per
+// element hide the slots' latency.  With fewer (warp_rows; one group per
+// class, as in a batch of particle sets) a block takes 8 x 32 representatives
+// and each warp sums every block of its own 32 in order, so no warp idles.
+//
+// h-binned parts: the block's 32 x 8 elements each need the coefficients of
+// their own |k|^2.  Those of the next eight fours (one 128-byte line per
+// element) are copied to shared memory while the current eight are summed;
+// read by every lane from its own rows of the table, 4 or 16 bytes at a time,
+// they bound the kernel by L1 tag lookups (76%; 2.98 ms on the 156-bin
+// SPH-like set).
+struct TcReduceArgs {
+    const TcReducePart* parts;
+    int n_parts;
+    const TcReduceBlock* blocks;
 };
 
-// Warps per block of the reduction kernel.
+// Warps per block of the reduction kernel; an h-binned part's coefficients come
+// kCoefLine floats (one 128-byte line, eight fours) an element at a time, in
+// rows of kCoefRow floats in shared memory (their padding keeps a warp's
+// 16-byte reads of 32 rows free of bank conflicts).
 constexpr int kReduceWarps = 8;
+constexpr int kCoefLine = 4 * kReduceWarps, kCoefRow = kCoefLine + 4;
+constexpr int kCoefBuffer = 2 * kReduceC * 32 * kCoefRow;  // floats of one buffer
+constexpr size_t kReduceSmemBinned = 2 * kCoefBuffer * sizeof(float);
+constexpr size_t kReduceSmem = kReduceWarps * 2 * kReduceC * 32 * sizeof(double2);  // the partial sums
+static_assert(kReduceSmem <= kReduceSmemBinned && kReduceWarps == 2 * kReduceC, "reduction");
 
-__global__ void __launch_bounds__(32 * kReduceWarps, 2) tc_reduce_kernel(TcReduceArgs f) {
-    extern __shared__ __align__(16) unsigned char s_raw[];  // n_list descriptors, then the partial sums
-    ReduceJob* s_jobs = reinterpret_cast<ReduceJob*>(s_raw);
-    for (int i = threadIdx.x; i < f.n_list; i += blockDim.x) s_jobs[i] = reduce_job(f.jobs[f.list[i]]);
-    // [warp][kReduceC * 2][lane], 16-byte aligned after the descriptors
-    double2* s_part = reinterpret_cast<double2*>(s_raw + (((size_t)f.n_list * sizeof(ReduceJob) + 15) & ~(size_t)15));
-    __syncthreads();
+__global__ void __launch_bounds__(32 * kReduceWarps, 2) tc_reduce_kernel(TcReduceArgs g) {
+    // h-binned parts: two buffers of coefficients; then the partial sums,
+    // [warp][plus, minus columns][lane]
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    double2* s_part = reinterpret_cast<double2*>(s_raw);
+    int lo = 0, hi = g.n_parts;
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (__ldg(&g.parts[mid].first_block) <= (int)blockIdx.x) lo = mid;
+        else hi = mid;
+    }
+    const TcReducePart& f = g.parts[lo];
     const TcPart& P = f.part;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int block_reps = f.warp_rows ? 32 * kReduceWarps : 32;
+    const bool warp_rows = f.warp_rows != 0;
+    const int block = (int)blockIdx.x - f.first_block;
+    const int block_reps = warp_rows ? 32 * kReduceWarps : 32;
     const int rep_blocks = (P.n_reps + block_reps - 1) / block_reps;
-    const int rest = blockIdx.x / rep_blocks;
+    const int rest = block / rep_blocks;
     const int bl = rest % P.fold, c0 = rest / P.fold * kReduceC;
-    const int rep = (int)(blockIdx.x % rep_blocks) * block_reps + (f.warp_rows ? warp * 32 : 0) + lane;
+    const int rep = block % rep_blocks * block_reps + (warp_rows ? warp * 32 : 0) + lane;
     const bool active = rep < P.n_reps;
     const int fa = (active ? rep : 0) / P.rows + P.a_base;
     const int rowb = (active ? rep : 0) % P.rows * P.fold + P.b_base;
@@ -1600,10 +1635,107 @@ __global__ void __launch_bounds__(32 * kReduceWarps, 2) tc_reduce_kernel(TcReduc
         nm[i] = inside(m) ? square(m) : 0;
     }
     PairSum s = {};
-    if (active)
-        for (int j = f.warp_rows ? 0 : warp; j < f.n_list; j += f.warp_rows ? 1 : kReduceWarps)
-            reduce_add(s_jobs[j], rep, P.fold, bl, c0, np, nm, s);
-    if (!f.warp_rows) {
+    const int col = bl * P.columns + c0;
+    const TcReduceBlock* first = g.blocks + (size_t)f.first_four * 4;
+    if (f.binned) {
+        // warp w copies the lines of element set w (plus column w, or minus
+        // column w - 4) of the block's 32 representatives
+        float* s_coef = reinterpret_cast<float*>(s_raw);
+        int n2 = np[0];
+#pragma unroll
+        for (int i = 0; i < kReduceC; ++i) {
+            if (warp == i) n2 = np[i];
+            if (warp == kReduceC + i) n2 = nm[i];
+        }
+        const int chunks = f.n_fours / kReduceWarps;  // tensor_plan pads a group's blocks to whole lines
+        auto copy = [&](int chunk) {
+            const TcReduceBlock& head = first[(size_t)chunk * kCoefLine];
+            float* dst = s_coef + (chunk & 1) * kCoefBuffer + warp * 32 * kCoefRow;
+#pragma unroll
+            for (int r = 0; r < 32; r += 4) {
+                const int row = r + (lane >> 3);
+                const int k2 = __shfl_sync(0xffffffffu, n2, row);
+                const float* src = head.coef + (size_t)k2 * head.coef_stride + (lane & 7) * 4;
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                                 smem_u32(dst + row * kCoefRow + (lane & 7) * 4)),
+                             "l"(src)
+                             : "memory");
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        copy(0);
+        for (int chunk = 0; chunk < chunks; ++chunk) {
+            if (chunk + 1 < chunks) {
+                copy(chunk + 1);
+                asm volatile("cp.async.wait_group 1;" ::: "memory");
+            } else {
+                asm volatile("cp.async.wait_group 0;" ::: "memory");
+            }
+            __syncthreads();
+            const TcReduceBlock* four = first + (size_t)chunk * kCoefLine + warp * 4;
+            const float* w = s_coef + (chunk & 1) * kCoefBuffer + lane * kCoefRow + warp * 4;
+            if (active) {
+                if (f.simple) {
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {  // two blocks' loads in flight
+                        BlockAt at[2];
+                        float4 v[2][4];
+#pragma unroll
+                        for (int e = 0; e < 2; ++e) {
+                            at[e] = block_at(four[2 * h + e], rep, col);
+                            const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+                            const bool any = at[e].re != nullptr;
+                            v[e][0] = any ? __ldcs(reinterpret_cast<const float4*>(at[e].re)) : z;
+                            v[e][1] = any ? __ldcs(reinterpret_cast<const float4*>(at[e].im)) : z;
+                            v[e][2] = any ? __ldcs(reinterpret_cast<const float4*>(at[e].re + 4 * kReps)) : z;
+                            v[e][3] = any ? __ldcs(reinterpret_cast<const float4*>(at[e].im + 4 * kReps)) : z;
+                        }
+#pragma unroll
+                        for (int i = 0; i < kReduceC; ++i) {
+                            const float2 wp = *reinterpret_cast<const float2*>(w + i * 32 * kCoefRow + 2 * h);
+                            const float2 wm = *reinterpret_cast<const float2*>(w + (kReduceC + i) * 32 * kCoefRow + 2 * h);
+#pragma unroll
+                            for (int e = 0; e < 2; ++e) {
+                                const double cc = component(v[e][0], i), cs = component(v[e][1], i);
+                                const double sc = component(v[e][2], i), ss = component(v[e][3], i);
+                                // no job: the line's padding is not a number to multiply with
+                                const bool any = at[e].re != nullptr;
+                                const double up = any ? (double)(e ? wp.y : wp.x) * at[e].scale : 0.0;
+                                const double um = any ? (double)(e ? wm.y : wm.x) * at[e].scale : 0.0;
+                                s.pr[i] = fma(up, cc - ss, s.pr[i]);
+                                s.pi[i] = fma(up, cs + sc, s.pi[i]);
+                                s.mr[i] = fma(um, cc + ss, s.mr[i]);
+                                s.mi[i] = fma(um, cs - sc, s.mi[i]);
+                            }
+                        }
+                    }
+                } else {
+#pragma unroll 1
+                    for (int e = 0; e < 4; ++e) {
+                        if (four[e].n_splits == 0) continue;  // no job here
+                        float up[kReduceC], um[kReduceC];
+#pragma unroll
+                        for (int i = 0; i < kReduceC; ++i) {
+                            up[i] = w[i * 32 * kCoefRow + e];
+                            um[i] = w[(kReduceC + i) * 32 * kCoefRow + e];
+                        }
+                        reduce_add(four[e], rep, col, true, up, um, s);
+                    }
+                }
+            }
+            __syncthreads();  // before the buffer is filled again (or holds the partial sums)
+        }
+    } else if (active) {
+        const int dq = warp_rows ? 1 : kReduceWarps;
+        const float none[kReduceC] = {};
+        for (int q = warp_rows ? 0 : warp; q < f.n_fours; q += dq)
+#pragma unroll 1
+            for (int e = 0; e < 4; ++e) {
+                const TcReduceBlock& b = first[4 * q + e];
+                if (b.n_splits > 0) reduce_add(b, rep, col, false, none, none, s);
+            }
+    }
+    if (!warp_rows) {
 #pragma unroll
         for (int i = 0; i < kReduceC; ++i) {
             s_part[(warp * 2 * kReduceC + i) * 32 + lane] = make_double2(s.pr[i], s.pi[i]);
@@ -1638,9 +1770,9 @@ __global__ void __launch_bounds__(32 * kReduceWarps, 2) tc_reduce_kernel(TcReduc
     for (int i = 0; i < kReduceC; ++i) {
         int3 p, m;
         frequencies(i, p, m);
-        if (P.write_plus && (f.warp_rows || warp == i)) store(p, s.pr[i], s.pi[i]);
+        if (P.write_plus && (warp_rows || warp == i)) store(p, s.pr[i], s.pi[i]);
         // an exchanged part's mirror is along the columns: the conjugate B
-        if (key >= P.min_minus && (f.warp_rows || warp == kReduceC + i))
+        if (key >= P.min_minus && (warp_rows || warp == kReduceC + i))
             store(m, s.mr[i], P.kind == kPartExchanged ? -s.mi[i] : s.mi[i]);
     }
 }
@@ -2002,14 +2134,20 @@ int tensor_plan(const std::vector<SumRequest>& groups, TensorPlan& plan) {
         // the last m-tile may extend past the representatives: the reduction
         // does not read them
         j.n_mtiles = (int)(((long long)j.kx * j.ky + kReps * ctas - 1) / (kReps * ctas));
-        // particle splits: items of at most the launch's terms / (units x
-        // tc_waves) (default 4 waves), at least 32 stages each; every split
-        // is one more slot to write and reduce
+        // particle splits: items of at most 1 / (units x tc_waves) of the
+        // launch's stages (default 4 waves), as full tiles would take them, and
+        // at least 8 stages each; every split is one more slot to write and
+        // reduce.  The limit is in stages, not terms, and an eighth of it for
+        // the jobs of a few tiles (Nyquist planes, faces), whose items fill
+        // the SMs that the others leave at the end: uncut, those of 16
+        // particle sets kept 20 SMs for 6.9 ms after the 15 ms launch of the
+        // planes.
         const long long ftiles = (long long)j.n_mtiles * j.n_ntiles;
-        const double item_budget = launch_terms / ((double)(device_sm_count() / ctas) * active_tune().tc_waves);
-        long long splits = std::max<long long>(
-            1, (long long)std::ceil((double)j.n * kM * ctas * std::min(j.nc_tile, j.lz_tc) / item_budget));
-        splits = std::min<long long>(splits, std::max<long long>(1, (j.n + 32 * kKp - 1) / (32 * kKp)));
+        const double tile_stages = launch_terms / ((double)kKp * kM * ctas * Shape<kWide>::kNc);
+        const double item_stages = tile_stages / ((double)(device_sm_count() / ctas) * active_tune().tc_waves) /
+                                   (ftiles * ctas < 16 ? 8.0 : 1.0);
+        const long long job_stages = (j.n + kKp - 1) / kKp;
+        long long splits = std::max<long long>(1, (long long)std::ceil((double)job_stages / std::max(8.0, item_stages)));
         // The 128-column tiles keep an item's whole sum in an FP32 total: at
         // most kMaxItemChains chains per item.  The 256-column tiles take items
         // of any length: their items add the FP32 total of every
@@ -2042,6 +2180,7 @@ int tensor_plan(const std::vector<SumRequest>& groups, TensorPlan& plan) {
         plan.bimg_offset.push_back(img_off);
         plan.job_tp.push_back(tp_offset);
         plan.job_coef.push_back(coef_offset);
+        plan.job_binned.push_back(coef_offset == SIZE_MAX ? -1 : (int)plan.binned.size());
         plan.job_slot.push_back(plan.slot_bytes);
         plan.slot_bytes += (size_t)(splits * ftiles) * (size_t)j.slot_stride * (j.slot_fp64 ? 8 : 4);
         // column c of the job -> its n-tile and the slot columns of its Re and
@@ -2059,7 +2198,7 @@ int tensor_plan(const std::vector<SumRequest>& groups, TensorPlan& plan) {
             const long long k0 = ks * chunk, k1 = std::min<long long>(j.n, k0 + chunk);
             const long long stages = (k1 - k0 + kKp - 1) / kKp;
             for (long long t = 0; t < ftiles; ++t)
-                items.push_back({mode, stages + (stages + flush_stages - 1) / flush_stages, make_int2(job_index, (int)(ks * ftiles + t)),
+                items.push_back({mode, stages + kItemCost + (mode == kPair || mode == kWide ? 2 : 0) * ((stages + flush_stages - 1) / flush_stages), make_int2(job_index, (int)(ks * ftiles + t)),
                                  (int)(t / j.n_ntiles), (int)ks});
         }
         return job_index;
@@ -2162,7 +2301,8 @@ int tensor_plan(const std::vector<SumRequest>& groups, TensorPlan& plan) {
                 blocks += (bg.bins[b].count + kBlockParticles - 1) / kBlockParticles;
                 bg.total_q += bg.bins[b].order;
             }
-            bg.coef_count = (size_t)bg.total_q * bg.nsq;  // [n2][bin's blocks]
+            bg.coef_stride = (bg.total_q + kCoefLine - 1) / kCoefLine * kCoefLine;  // the reduction reads whole lines
+            bg.coef_count = (size_t)bg.coef_stride * bg.nsq;  // [n2][bin's blocks]
             plan.coef_bytes += (bg.coef_count * sizeof(float) + 255) / 256 * 256;
             const size_t blocks_bytes = (size_t)blocks * kBlockBytes;
             plan.tp_bytes += blocks_bytes;
@@ -2193,7 +2333,7 @@ int tensor_plan(const std::vector<SumRequest>& groups, TensorPlan& plan) {
                 j.wmax = bin.wmax;
                 j.period = lz_tc;
                 j.fold = bfold;
-                j.coef_stride = bg.total_q;
+                j.coef_stride = bg.coef_stride;
                 const size_t tp = plan.tp_offset.back() + (size_t)first_block[b] * kBlockBytes;
                 const int jm = add_job(j, mode_of(j.lz_tc, (long long)j.kx * j.ky), true, tp, cls, 0, coef_off);
                 if (first_job < 0) {
@@ -2320,16 +2460,46 @@ int tensor_plan(const std::vector<SumRequest>& groups, TensorPlan& plan) {
         return x.item.y < y.item.y;
     });
     plan.items.reserve(items.size());
-    plan.n_narrow = plan.n_pair_narrow = plan.n_pair = plan.n_pair_db = 0;
-    for (auto& it : items) {
-        plan.items.push_back(it.item);
-        plan.n_narrow += it.mode == kNarrow ? 1 : 0;
-        plan.n_pair_narrow += it.mode == kPairNarrow ? 1 : 0;
-        plan.n_pair += it.mode == kPair ? 1 : 0;
-        plan.n_pair_db += it.mode == kPairDB ? 1 : 0;
+    // One launch per tile mode.  Its items go, in this order, each to the unit
+    // (CTA or CTA pair) that has the least to do so far: a unit's items are one
+    // list.  (Dealt out round-robin, the sixteen uneven sets of a batch left
+    // units idle for a fifth of the launch.)
+    for (size_t b = 0; b < items.size();) {
+        size_t e = b;
+        long long total = 0;
+        const int mode = items[b].mode;
+        for (; e < items.size() && items[e].mode == mode; ++e) total += items[e].cost;
+        const int units = (int)std::min<size_t>(e - b, (size_t)(pair_mode(mode) ? sms / 2 : sms));
+        std::vector<std::vector<int2>> lists(units);
+        std::vector<std::pair<long long, int>> heap(units);  // (load, unit), least first
+        for (int u = 0; u < units; ++u) heap[u] = {0, u};
+        const auto later = std::greater<std::pair<long long, int>>();
+        for (size_t i = b; i < e; ++i) {
+            std::pop_heap(heap.begin(), heap.end(), later);
+            lists[heap.back().second].push_back(items[i].item);
+            heap.back().first += items[i].cost;
+            std::push_heap(heap.begin(), heap.end(), later);
+        }
+        TensorPlan::Launch l;
+        l.mode = mode;
+        l.n_lists = units;
+        l.first = (int)plan.list_first.size();
+        l.cost = total / units;
+        for (const std::vector<int2>& v : lists) {
+            plan.list_first.push_back((int)plan.items.size());
+            plan.items.insert(plan.items.end(), v.begin(), v.end());
+        }
+        plan.list_first.push_back((int)plan.items.size());
+        plan.launches.push_back(l);
+        b = e;
     }
+    // longest first: the others fill the SMs it leaves at its end
+    std::stable_sort(plan.launches.begin(), plan.launches.end(),
+                     [](const TensorPlan::Launch& x, const TensorPlan::Launch& y) { return x.cost > y.cost; });
     const size_t jobs_bytes = ((plan.jobs.size() * sizeof(TcJob) + 255) / 256) * 256;
     plan.meta_bytes = jobs_bytes + ((plan.items.size() * sizeof(int2) + 255) / 256) * 256;
+    plan.list_offset = plan.meta_bytes;
+    plan.meta_bytes += (plan.list_first.size() * sizeof(int) + 255) / 256 * 256;
     // the jobs with B-operand images and their first images
     plan.img_jobs.clear();
     plan.img_first.assign(1, 0);
@@ -2346,12 +2516,74 @@ int tensor_plan(const std::vector<SumRequest>& groups, TensorPlan& plan) {
     // the jobs' column maps
     plan.colmap_offset = plan.meta_bytes;
     plan.meta_bytes += (plan.colmaps.size() * sizeof(int4) + 255) / 256 * 256;
-    // each class's job lists, part by part
-    for (TensorPlan::Class& c : plan.classes)
-        for (TensorPlan::Class::Part& p : c.parts) {
-            p.list_offset = plan.meta_bytes;
-            plan.meta_bytes += (p.jobs.size() * sizeof(int) + 255) / 256 * 256;
+    // the reduction's parts and column blocks: fours of a part's jobs, or for
+    // binned groups whole lines of one group's blocks, each at its
+    // coefficient's place; a class that shares its spectrum with earlier ones
+    // goes to a later launch
+    for (size_t c = 0; c < plan.classes.size(); ++c) {
+        const TensorPlan::Class& cl = plan.classes[c];
+        int level = 0;
+        for (size_t b = 0; b < c; ++b)
+            if (plan.classes[b].out == cl.out) ++level;
+        for (const TensorPlan::Class::Part& p : cl.parts) {
+            if (p.jobs.empty()) continue;
+            TcReducePart rp{};
+            rp.part = p.geometry;
+            rp.first_four = (int)(plan.reduce_blocks.size() / 4);
+            rp.kx = cl.kx;
+            rp.ky = cl.ky;
+            rp.lz_out = cl.lz_out;
+            rp.step = cl.step;
+            rp.basis = cl.basis;
+            rp.h = cl.h;
+            rp.factored = cl.factored;
+            rp.scale = cl.scale;
+            rp.out = cl.out;
+            std::map<size_t, size_t> group_at;  // coefficient base of a binned group -> its first block
+            for (int ji : p.jobs) {
+                const TcJob& J = plan.jobs[ji];
+                const int blocks = J.period > 0 ? J.lz_tc / J.period / std::max(1, J.fold) : 1;
+                if (plan.job_coef[ji] == SIZE_MAX) {
+                    plan.reduce_blocks.push_back({ji, 0});
+                    continue;
+                }
+                const TensorPlan::Binned& bg = plan.binned[plan.job_binned[ji]];
+                auto at = group_at.find(bg.coef_offset);
+                if (at == group_at.end()) {
+                    at = group_at.emplace(bg.coef_offset, plan.reduce_blocks.size()).first;
+                    for (int q = 0; q < bg.coef_stride; q += kCoefLine)
+                        plan.reduce_lines.push_back({plan.reduce_blocks.size() + q, plan.job_binned[ji], q});
+                    plan.reduce_blocks.resize(plan.reduce_blocks.size() + bg.coef_stride, {-1, 0});
+                }
+                for (int q = 0; q < blocks; ++q)
+                    plan.reduce_blocks[at->second + (plan.job_coef[ji] - bg.coef_offset) + q] = {ji, q};
+            }
+            while (plan.reduce_blocks.size() % 4) plan.reduce_blocks.push_back({-1, 0});
+            rp.n_fours = (int)(plan.reduce_blocks.size() / 4) - rp.first_four;
+            rp.binned = group_at.empty() ? 0 : 1;
+            rp.warp_rows = !rp.binned && rp.n_fours < kReduceWarps ? 1 : 0;
+            rp.simple = 1;
+            for (int ji : p.jobs)
+                if (plan.jobs[ji].slot_fp64 || plan.jobs[ji].n_splits != 1) rp.simple = 0;
+            if ((int)plan.reduce_levels.size() <= level) plan.reduce_levels.resize(level + 1);
+            plan.reduce_levels[level].push_back(rp);
         }
+    }
+    for (std::vector<TcReducePart>& parts : plan.reduce_levels) {
+        long long blocks = 0;
+        for (TcReducePart& rp : parts) {
+            rp.first_block = (int)blocks;
+            const int block_reps = rp.warp_rows ? 32 * kReduceWarps : 32;
+            blocks += (long long)((rp.part.n_reps + block_reps - 1) / block_reps) * rp.part.fold *
+                      (rp.part.columns / kReduceC);
+            if (blocks > INT32_MAX) return set_error(kInvalidValue, "tensor sum: too many reduction blocks");
+        }
+        plan.reduce_offset.push_back(plan.meta_bytes);
+        plan.reduce_grid.push_back((int)blocks);
+        plan.meta_bytes += (parts.size() * sizeof(TcReducePart) + 255) / 256 * 256;
+    }
+    plan.reduce_blocks_offset = plan.meta_bytes;
+    plan.meta_bytes += (plan.reduce_blocks.size() * sizeof(TcReduceBlock) + 255) / 256 * 256;
     // the binned groups' tables: edges, int4 bins, float4 spans, int first
     // particles (16-byte aligned)
     for (TensorPlan::Binned& bg : plan.binned) {
@@ -2386,16 +2618,42 @@ int tensor_reserve_upload(TensorPlan& plan, TensorWorkspace& ws, cudaStream_t st
     const size_t jobs_bytes = ((plan.jobs.size() * sizeof(TcJob) + 255) / 256) * 256;
     if (!plan.jobs.empty()) std::memcpy(meta.data(), plan.jobs.data(), plan.jobs.size() * sizeof(TcJob));
     if (!plan.items.empty()) std::memcpy(meta.data() + jobs_bytes, plan.items.data(), plan.items.size() * sizeof(int2));
+    if (!plan.list_first.empty())
+        std::memcpy(meta.data() + plan.list_offset, plan.list_first.data(), plan.list_first.size() * sizeof(int));
     if (!plan.colmaps.empty())
         std::memcpy(meta.data() + plan.colmap_offset, plan.colmaps.data(), plan.colmaps.size() * sizeof(int4));
     if (!plan.img_jobs.empty()) {
         std::memcpy(meta.data() + plan.img_jobs_offset, plan.img_jobs.data(), plan.img_jobs.size() * sizeof(int));
         std::memcpy(meta.data() + plan.img_first_offset, plan.img_first.data(), plan.img_first.size() * sizeof(long long));
     }
-    for (const TensorPlan::Class& c : plan.classes)
-        for (const TensorPlan::Class::Part& p : c.parts)
-            if (!p.jobs.empty())
-                std::memcpy(meta.data() + p.list_offset, p.jobs.data(), p.jobs.size() * sizeof(int));
+    for (size_t l = 0; l < plan.reduce_levels.size(); ++l)
+        std::memcpy(meta.data() + plan.reduce_offset[l], plan.reduce_levels[l].data(),
+                    plan.reduce_levels[l].size() * sizeof(TcReducePart));
+    TcReduceBlock* rb = reinterpret_cast<TcReduceBlock*>(meta.data() + plan.reduce_blocks_offset);
+    for (size_t k = 0; k < plan.reduce_blocks.size(); ++k) {
+        TcReduceBlock b{};
+        const int2 jq = plan.reduce_blocks[k];
+        if (jq.x >= 0) {
+            const TcJob& J = plan.jobs[jq.x];
+            b.slots = J.slots;
+            b.colmap = J.colmap + (size_t)jq.y * std::max(1, J.fold) * J.period;
+            b.scale = J.wmax * kInvProductScale;
+            b.slot_fp64 = J.slot_fp64;
+            b.slot_stride = J.slot_stride;
+            b.n_splits = J.n_splits;
+            b.n_mtiles = J.n_mtiles;
+            b.n_ntiles = J.n_ntiles;
+            b.rank_stride = kM * 2 * J.nc_tile;
+            b.reps_log2 = J.ctas == 2 ? 7 : 6;
+        }
+        rb[k] = b;
+    }
+    // the first block of a binned group's line names its coefficients
+    for (const TensorPlan::ReduceLine& l : plan.reduce_lines) {
+        const TensorPlan::Binned& bg = plan.binned[l.binned];
+        rb[l.block].coef = static_cast<const float*>(ws.coef.ptr) + bg.coef_offset + l.first_coef;
+        rb[l.block].coef_stride = bg.coef_stride;
+    }
     for (const TensorPlan::Binned& bg : plan.binned) {
         float* edges = reinterpret_cast<float*>(meta.data() + bg.meta_offset);
         const size_t edges_bytes = ((size_t)(bg.nbins + 1) * sizeof(float) + 15) / 16 * 16;
@@ -2488,30 +2746,29 @@ int tensor_prepare(const std::vector<SumRequest>& groups, TensorWorkspace& ws, c
 
 namespace {
 
-// One persistent launch of a tile mode: min(items, SMs) CTAs, or for the CTA
-// pair modes clusters of 2, as many as can be resident at once.
+// One persistent launch of a tile mode: a CTA a list, at most one an SM, or
+// for the CTA pair modes clusters of 2, as many as can be resident at once.
+// overlap: a launch after another tile mode's (on which it does not depend)
+// takes the SMs that one leaves at its end; its CTAs end after that launch
+// has (griddepcontrol.wait), so what follows waits for both.
 template <int MODE>
-int launch_tile(const TcArgs& a, cudaStream_t stream) {
+int launch_tile(const TcArgs& a, bool overlap, cudaStream_t stream) {
     using SH = Shape<MODE>;
     int st = check_cuda(
         cudaFuncSetAttribute(tc_sum_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SH::kSmemBytes),
         "cudaFuncSetAttribute");
     if (st != kOk) return st;
-    if constexpr (SH::kCtas == 1) {
-        const int grid = std::min<int>(a.n_items, device_sm_count());
-        tc_sum_kernel<MODE><<<grid, kThreads, SH::kSmemBytes, stream>>>(a);
-        return kOk;
-    } else {
-        cudaLaunchConfig_t lc = {};
-        cudaLaunchAttribute attr[1];
+    cudaLaunchConfig_t lc = {};
+    cudaLaunchAttribute attr[2];
+    lc.blockDim = dim3(kThreads);
+    lc.dynamicSmemBytes = SH::kSmemBytes;
+    lc.stream = stream;
+    lc.attrs = attr;
+    if constexpr (SH::kCtas == 2) {
         attr[0].id = cudaLaunchAttributeClusterDimension;
         attr[0].val.clusterDim.x = 2;
         attr[0].val.clusterDim.y = 1;
         attr[0].val.clusterDim.z = 1;
-        lc.blockDim = dim3(kThreads);
-        lc.dynamicSmemBytes = SH::kSmemBytes;
-        lc.stream = stream;
-        lc.attrs = attr;
         lc.numAttrs = 1;
         lc.gridDim = dim3(2 * std::max(1, device_sm_count() / 2));
         int clusters = 0;
@@ -2519,22 +2776,18 @@ int launch_tile(const TcArgs& a, cudaStream_t stream) {
                         "cudaOccupancyMaxActiveClusters");
         if (st != kOk) return st;
         if (clusters < 1) return set_error(kCudaError, "tensor sum: no CTA pair fits on this device");
-        lc.gridDim = dim3(2 * std::min(a.n_items, clusters));
-        return check_cuda(cudaLaunchKernelEx(&lc, tc_sum_kernel<MODE>, a), "tc_sum_kernel (pairs) launch");
+        lc.gridDim = dim3(2 * std::min(a.n_lists, clusters));
+    } else {
+        lc.gridDim = dim3(std::min(a.n_lists, device_sm_count()));
     }
+    if (overlap) {
+        attr[lc.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[lc.numAttrs].val.programmaticStreamSerializationAllowed = 1;
+        ++lc.numAttrs;
+    }
+    return check_cuda(cudaLaunchKernelEx(&lc, tc_sum_kernel<MODE>, a), "tc_sum_kernel launch");
 }
 
-}  // namespace
-
-namespace {
-// Dynamic shared memory of the reduction kernels: the class's job
-// descriptors (and the planes kernel's partial sums).
-int reduce_smem(void (*kernel)(TcReduceArgs), size_t bytes) {
-    if (bytes > 200 * 1024) return set_error(kInvalidValue, "tensor sum: too many jobs in one output class");
-    if (bytes <= 48 * 1024) return kOk;
-    return check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes),
-                      "cudaFuncSetAttribute(reduction)");
-}
 }  // namespace
 
 int tensor_enqueue(const std::vector<SumRequest>& groups, const TensorPlan& plan, TensorWorkspace& ws,
@@ -2605,7 +2858,7 @@ int tensor_enqueue(const std::vector<SumRequest>& groups, const TensorPlan& plan
             ca.step = r.lat.kx;
             ca.nbins = bg.nbins;
             ca.nsq = bg.nsq;
-            ca.total_q = bg.total_q;
+            ca.coef_stride = bg.coef_stride;
             ca.bins = bp.bins;
             ca.spans = bp.spans;
             ca.edges = bp.edges;
@@ -2657,72 +2910,57 @@ int tensor_enqueue(const std::vector<SumRequest>& groups, const TensorPlan& plan
     // one persistent launch per tile mode for all groups
     if (!plan.items.empty()) {
         timer_begin(timer, 3, stream);
-        const int counts[5] = {plan.n_narrow, plan.n_pair_narrow, plan.n_pair, plan.n_pair_db,
-                               (int)plan.items.size() - plan.n_narrow - plan.n_pair_narrow - plan.n_pair -
-                                   plan.n_pair_db};
-        const int modes[5] = {kNarrow, kPairNarrow, kPair, kPairDB, kWide};
-        int first = 0;
-        bool hooked = false;
-        for (int m = 0; m < 5 && st == kOk; first += counts[m], ++m) {
+        bool first = true;
+        for (const TensorPlan::Launch& l : plan.launches) {
             TcArgs a;
             a.jobs = static_cast<const TcJob*>(plan.d_jobs);
-            a.items = static_cast<const int2*>(plan.d_items) + first;
-            a.n_items = counts[m];
+            a.items = static_cast<const int2*>(plan.d_items);
+            a.list_first = reinterpret_cast<const int*>(static_cast<const char*>(ws.meta.ptr) + plan.list_offset) + l.first;
+            a.n_lists = l.n_lists;
             a.error_flag = error_flag;
             a.wait_limit_ns = kWaitLimitNs;
             a.withhold_first_arrival = 0;
-            if (a.n_items == 0) continue;
-            if (!hooked) {
-                hooked = true;
+            if (first) {
                 const long long t = g_test_wait_limit_ns.exchange(0);
                 if (t > 0) {
                     a.wait_limit_ns = (unsigned long long)t;
                     a.withhold_first_arrival = 1;
                 }
             }
-            switch (modes[m]) {
-            case kNarrow: st = launch_tile<kNarrow>(a, stream); break;
-            case kPairNarrow: st = launch_tile<kPairNarrow>(a, stream); break;
-            case kPair: st = launch_tile<kPair>(a, stream); break;
-            case kPairDB: st = launch_tile<kPairDB>(a, stream); break;
-            default: st = launch_tile<kWide>(a, stream); break;
+            switch (l.mode) {
+            case kNarrow: st = launch_tile<kNarrow>(a, !first, stream); break;
+            case kPairNarrow: st = launch_tile<kPairNarrow>(a, !first, stream); break;
+            case kPair: st = launch_tile<kPair>(a, !first, stream); break;
+            case kPairDB: st = launch_tile<kPairDB>(a, !first, stream); break;
+            default: st = launch_tile<kWide>(a, !first, stream); break;
             }
+            first = false;
             if (st != kOk) break;
             count_launch();
             st = check_cuda(cudaGetLastError(), "tc_sum_kernel launch");
+            if (st != kOk) break;
         }
         timer_end(timer, 3, stream);
         if (st != kOk) return st;
     }
     // the items' tiles -> spectra, summed in FP64 (added to what is there)
-    for (const TensorPlan::Class& c : plan.classes)
-        for (const TensorPlan::Class::Part& p : c.parts) {
-            if (p.jobs.empty()) continue;
-            TcReduceArgs f;
-            f.jobs = static_cast<const TcJob*>(plan.d_jobs);
-            f.list = reinterpret_cast<const int*>(static_cast<const char*>(ws.meta.ptr) + p.list_offset);
-            f.n_list = (int)p.jobs.size();
-            f.part = p.geometry;
-            f.kx = c.kx;
-            f.ky = c.ky;
-            f.lz_out = c.lz_out;
-            f.step = c.step;
-            f.basis = c.basis;
-            f.h = c.h;
-            f.factored = c.factored;
-            f.scale = c.scale;
-            f.out = c.out;
-            f.warp_rows = f.n_list < kReduceWarps ? 1 : 0;
-            const int block_reps = f.warp_rows ? 32 * kReduceWarps : 32;
-            const long long blocks = (long long)((f.part.n_reps + block_reps - 1) / block_reps) * f.part.fold *
-                                     (f.part.columns / kReduceC);
-            const size_t smem = (((size_t)f.n_list * sizeof(ReduceJob) + 15) & ~(size_t)15) +
-                                (f.warp_rows ? 0 : (size_t)kReduceWarps * 32 * 2 * kReduceC * sizeof(double2));
-            st = reduce_smem(tc_reduce_kernel, smem);
-            if (st != kOk) return st;
-            tc_reduce_kernel<<<(unsigned)blocks, 32 * kReduceWarps, smem, stream>>>(f);
-            count_launch();
-        }
+    for (size_t l = 0; l < plan.reduce_levels.size(); ++l) {
+        const char* meta = static_cast<const char*>(ws.meta.ptr);
+        TcReduceArgs f;
+        f.parts = reinterpret_cast<const TcReducePart*>(meta + plan.reduce_offset[l]);
+        f.n_parts = (int)plan.reduce_levels[l].size();
+        f.blocks = reinterpret_cast<const TcReduceBlock*>(meta + plan.reduce_blocks_offset);
+        bool binned = false;
+        for (const TcReducePart& p : plan.reduce_levels[l]) binned = binned || p.binned;
+        const size_t smem = binned ? kReduceSmemBinned : kReduceSmem;
+        if (binned)
+            st = check_cuda(cudaFuncSetAttribute(tc_reduce_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 (int)kReduceSmemBinned),
+                            "cudaFuncSetAttribute(reduction)");
+        if (st != kOk) return st;
+        tc_reduce_kernel<<<plan.reduce_grid[l], 32 * kReduceWarps, smem, stream>>>(f);
+        count_launch();
+    }
     st = check_cuda(cudaGetLastError(), "tc_reduce_kernel launch");
     if (st != kOk) return st;
     // the branch part of h-binned groups with the plain form, over their
