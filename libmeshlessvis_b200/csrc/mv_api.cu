@@ -839,7 +839,8 @@ void vis_fourier_volume_rendering(MeshlessDataset* ds, VisConfig* c) {
     vis_config_compute_scale(c);
     const int cx = c->_cutoff_frequency.x, cy = c->_cutoff_frequency.y;
     const int nx = c->_number_of_samples.x, ny = c->_number_of_samples.y;
-    if (check_cuda(cudaMemsetAsync(c->_d_freq_image_arranged, 0, sizeof(float2) * arranged_count(c), s->stream),
+    if (ds->number_of_groups == 0 &&
+        check_cuda(cudaMemsetAsync(c->_d_freq_image_arranged, 0, sizeof(float2) * arranged_count(c), s->stream),
                    "cudaMemsetAsync") != kOk)
         return;
     for (int g = 0; g < ds->number_of_groups; ++g) {
@@ -888,7 +889,7 @@ void vis_fourier_volume_rendering(MeshlessDataset* ds, VisConfig* c) {
             if (cull_aliased_terms(r, c->u_axis, c->v_axis, c->step_size, s->cull, s->stream, &kept) != kOk) return;
             r = kept;
         }
-        if (launch_plain_sum(r, s->partials, &s->timer) != kOk) return;
+        if (launch_slice_sum(r, nx, ny, s->partials, &s->timer) != kOk) return;
     }
     if (check_cufft(cufftSetStream(c->_plan, s->stream), "cufftSetStream") != kOk) return;
     timer_begin(&s->timer, 2, s->stream);

@@ -108,6 +108,17 @@ struct KernelTimer;  // per-stage event pairs, see mv_api.cu
 // Plain FP32 form.  Uses `ws` for split-K partial sums.
 int launch_plain_sum(const SumRequest& req, Workspace& ws, KernelTimer* timer);
 
+// The table of Phi^ the plain kernels read: its cell width and size (up to
+// |k| h = smax), and the launch that fills cells 0 .. n (the last all zero).
+double phi_table_cell(int basis);
+int phi_table_cells(int basis, double smax);
+void launch_phi_table(int basis, double ds, int n, float4* out, cudaStream_t stream);
+
+// One group's direct slice (mv_slice_sum.cu) into the C2R layout
+// float2[nx][ny/2+1]: every element written, or (req.accumulate) the samples
+// added.  Uses `ws` for split-K partial sums.
+int launch_slice_sum(const SumRequest& req, int nx, int ny, Workspace& ws, KernelTimer* timer);
+
 // Aliasing cull of the direct path (mv_cull.cu): `out` is `in` restricted to
 // the particles whose footprint in the view (u, v) lies in [0, 1/(2 step.x)] x
 // [0, 1/(2 step.y)], compacted in order into `ws`; waits for the kept count.

@@ -681,6 +681,19 @@ int shell_representatives(const Lattice& lat, int xp_count, int yrows, const uin
 
 }  // namespace
 
+double phi_table_cell(int basis) { return table_cell(basis); }
+
+// Beyond kMaxTable cells (s > 63 for Wendland, > 60 for SPH) |Phi^| < 1e-11
+// and the zero cell stands in for it.
+int phi_table_cells(int basis, double smax) {
+    return std::max(1, (int)std::min<double>(kMaxTable, std::ceil(smax / table_cell(basis)) + 2.0));
+}
+
+void launch_phi_table(int basis, double ds, int n, float4* out, cudaStream_t stream) {
+    phi_table_kernel<<<(n + 128) / 128, 128, 0, stream>>>(basis, ds, n, out, 0);
+    count_launch();
+}
+
 int launch_plain_sum(const SumRequest& req, Workspace& ws, KernelTimer* timer) {
     const Lattice& lat = req.lat;
     if (lat.nx <= 0 || lat.ny <= 0 || lat.nz <= 0) return kOk;
@@ -779,10 +792,7 @@ int launch_plain_sum(const SumRequest& req, Workspace& ws, KernelTimer* timer) {
         const double kz = std::fabs(lat.kz) * std::max(std::abs(lat.z0), std::abs(lat.z0 + lat.nz - 1));
         const double rmax = std::sqrt(kx * kx + ky * ky + kz * kz);
         const double smax = req.radius_max >= 0.f ? rmax * req.radius_max : 1e30;
-        // Beyond kMaxTable cells (s > 63 for Wendland, > 60 for SPH) |Phi^| < 1e-11
-        // and the zero cell stands in for it.
-        table_n = (int)std::min<double>(kMaxTable, std::ceil(smax / ds) + 2.0);
-        table_n = std::max(table_n, 1);
+        table_n = phi_table_cells(req.basis, smax);
         // the branch part ends at the branch point, (K + 1/2) ds: cells 0 .. K
         if (req.kink) table_n = std::min(table_n, (int)std::llround(phi_branch_point(req.basis) / ds - 0.5) + 1);
     }
