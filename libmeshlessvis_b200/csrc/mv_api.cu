@@ -21,7 +21,6 @@
 #include <map>
 #include <mutex>
 #include <string>
-#include <thread>
 #include <tuple>
 #include <unordered_map>
 #include <vector>
@@ -112,37 +111,6 @@ int hbin_fine_index(const std::vector<float>& edges, float h) {
 
 namespace {
 
-// Runs fn(part, begin, end) over [0, n) in contiguous ranges, one per host
-// thread (up to 16; the calling thread takes part 0), and returns the number
-// of parts.  Below 2^16 items, or when no thread can be started, one part
-// runs inline.  The registration's statistics are order-independent maxima,
-// minima and counts, so the parts' results combine to the serial ones.
-template <typename F>
-int parallel_parts(long long n, int max_parts, F fn) {
-    int parts = 1;
-    if (n >= (1LL << 16)) {
-        const unsigned hw = std::thread::hardware_concurrency();
-        parts = (int)std::min<long long>(std::min<unsigned>(hw ? hw : 1, 16u), n >> 15);
-        parts = std::max(1, std::min(parts, max_parts));
-    }
-    std::vector<std::thread> threads;
-    int started = 1;
-    auto range = [&](int p) { return std::make_pair(n * p / parts, n * (p + 1) / parts); };
-    for (int p = 1; p < parts; ++p) {
-        try {
-            threads.emplace_back([&fn, p, range] { fn(p, range(p).first, range(p).second); });
-            ++started;
-        } catch (...) {
-            break;
-        }
-    }
-    // parts no thread took run here, after part 0
-    fn(0, range(0).first, range(0).second);
-    for (int p = started; p < parts; ++p) fn(p, range(p).first, range(p).second);
-    for (std::thread& t : threads) t.join();
-    return parts;
-}
-
 // hbin_fine_index for many radii against the same edges: a guess from the
 // logarithm, then float comparisons against the edges up and down to the
 // largest i with edges[i] <= h, so the result is the binary search's exactly
@@ -166,49 +134,126 @@ struct FineIndex {
     }
 };
 
-// The smoothing-length histogram of a group whose Phi^ does not separate per
-// axis (SPH, WENDLAND_D3_C2) with varying radii; null otherwise.
-std::shared_ptr<const HBinStats> hbin_histogram(const Group& grp, const GroupStats& gs) {
+// Whether a group has a smoothing-length histogram: Phi^ does not separate per
+// axis (SPH, WENDLAND_D3_C2) and the radii vary.
+bool wants_histogram(const Group& grp, const GroupStats& gs) {
     const int b = (int)grp.basis_function_id;
-    if (!grp.h_radii || grp.number_of_terms <= 0 || (b != (int)SPH && b != (int)WENDLAND_D3_C2)) return nullptr;
-    if (!(gs.radius_min > 0.f) || !(gs.radius_max > gs.radius_min) || !std::isfinite(gs.radius_max)) return nullptr;
+    if (!grp.h_radii || grp.number_of_terms <= 0 || (b != (int)SPH && b != (int)WENDLAND_D3_C2)) return false;
+    return gs.radius_min > 0.f && gs.radius_max > gs.radius_min && std::isfinite(gs.radius_max);
+}
+
+std::shared_ptr<HBinStats> empty_histogram(const GroupStats& gs) {
     auto hs = std::make_shared<HBinStats>();
     hs->h_min = gs.radius_min;
     hs->h_max = gs.radius_max;
     hs->edges = hbin_fine_edges(gs.radius_min, gs.radius_max);
     hs->count.assign(kHBinFine, 0);
     hs->wmax.assign(kHBinFine, 0.f);
-    const FineIndex fine(hs->edges);
-    constexpr int kMaxParts = 16;
-    std::vector<std::vector<int>> count(kMaxParts);
-    std::vector<std::vector<float>> wmax(kMaxParts);
-    const int parts = parallel_parts(grp.number_of_terms, kMaxParts, [&](int p, long long b, long long e) {
-        count[p].assign(kHBinFine, 0);
-        wmax[p].assign(kHBinFine, 0.f);
-        for (long long k = b; k < e; ++k) {
-            const int f = fine(grp.h_radii[k]);
-            count[p][f] += 1;
-            wmax[p][f] = std::max(wmax[p][f], std::fabs(grp.h_constraints[k].weight));
-        }
-    });
-    for (int p = 0; p < parts; ++p)
-        for (int f = 0; f < kHBinFine; ++f) {
-            hs->count[f] += count[p][f];
-            hs->wmax[f] = std::max(hs->wmax[f], wmax[p][f]);
-        }
-    // the id names the content (plans are cached by it): FNV-1a of the range,
-    // the counts and the weight maxima, never 0
+    return hs;
+}
+
+// The histogram's id names its content (plans are cached by it): FNV-1a of the
+// range, the counts and the weight maxima, never 0.
+void name_histogram(HBinStats& hs) {
     uint64_t h = 1469598103934665603ull;
     auto mix = [&h](const void* p, size_t n) {
         const unsigned char* c = static_cast<const unsigned char*>(p);
         for (size_t i = 0; i < n; ++i) h = (h ^ c[i]) * 1099511628211ull;
     };
-    mix(&hs->h_min, sizeof(float));
-    mix(&hs->h_max, sizeof(float));
-    mix(hs->count.data(), hs->count.size() * sizeof(int));
-    mix(hs->wmax.data(), hs->wmax.size() * sizeof(float));
-    hs->id = h ? h : 1;
-    return hs;
+    mix(&hs.h_min, sizeof(float));
+    mix(&hs.h_max, sizeof(float));
+    mix(hs.count.data(), hs.count.size() * sizeof(int));
+    mix(hs.wmax.data(), hs.wmax.size() * sizeof(float));
+    hs.id = h ? h : 1;
+}
+
+// The statistics of a registered group from the host arrays: the largest
+// |weight|, the radius extremes (a NaN is passed over, or kept from the first
+// radius) and the histogram.
+GroupStats host_statistics(const Group& grp) {
+    GroupStats gs;
+    gs.weight_max = 0.f;
+    for (int k = 0; k < grp.number_of_terms; ++k)
+        gs.weight_max = std::max(gs.weight_max, std::fabs(grp.h_constraints[k].weight));
+    if (grp.h_radii && grp.number_of_terms > 0) {
+        gs.radius_min = gs.radius_max = grp.h_radii[0];
+        for (int k = 0; k < grp.number_of_terms; ++k) {
+            gs.radius_min = std::min(gs.radius_min, grp.h_radii[k]);
+            gs.radius_max = std::max(gs.radius_max, grp.h_radii[k]);
+        }
+    }
+    if (wants_histogram(grp, gs)) {
+        auto hs = empty_histogram(gs);
+        const FineIndex fine(hs->edges);
+        for (int k = 0; k < grp.number_of_terms; ++k) {
+            const int f = fine(grp.h_radii[k]);
+            hs->count[f] += 1;
+            hs->wmax[f] = std::max(hs->wmax[f], std::fabs(grp.h_constraints[k].weight));
+        }
+        name_histogram(*hs);
+        gs.hbins = hs;
+    }
+    return gs;
+}
+
+// The same from the device copies, for groups of at least kDeviceStats terms:
+// registering 30,011 particles with radii took 340 us, most of it one host
+// thread's passes over them.  `scratch` holds a RegisterStats and a histogram.
+constexpr int kDeviceStats = 8192;
+
+int device_statistics(const std::vector<Group*>& groups, Workspace& scratch, cudaStream_t stream,
+                      std::vector<GroupStats>& out) {
+    const size_t n = groups.size();
+    out.assign(n, GroupStats{});
+    if (n == 0) return kOk;
+    const size_t extremes_bytes = (n * sizeof(RegisterStats) + 255) / 256 * 256;
+    int st = scratch.reserve(extremes_bytes + n * register_histogram_bytes());
+    if (st != kOk) return st;
+    RegisterStats* d_ext = static_cast<RegisterStats*>(scratch.ptr);
+    char* d_hist = static_cast<char*>(scratch.ptr) + extremes_bytes;
+    std::vector<RegisterStats> ext(n);
+    st = launch_register_extremes_clear(d_ext, (int)n, stream);
+    for (size_t i = 0; i < n && st == kOk; ++i)
+        st = launch_register_extremes(reinterpret_cast<const float4*>(groups[i]->d_constraints), groups[i]->d_radii,
+                                      groups[i]->number_of_terms, d_ext + i, stream);
+    if (st == kOk)
+        st = check_cuda(cudaMemcpyAsync(ext.data(), d_ext, n * sizeof(RegisterStats), cudaMemcpyDeviceToHost, stream),
+                        "registration statistics D2H");
+    if (st == kOk) st = check_cuda(cudaStreamSynchronize(stream), "registration statistics");
+    if (st != kOk) return st;
+    std::vector<std::shared_ptr<HBinStats>> hist(n);
+    std::vector<char> host(register_histogram_bytes());
+    bool any = false;
+    for (size_t i = 0; i < n; ++i) {
+        GroupStats& gs = out[i];
+        gs.weight_max = register_value(ext[i].weight_max, 0.f);
+        if (groups[i]->h_radii) {
+            // a NaN first radius stays (no other compares below or above it)
+            const float r0 = groups[i]->h_radii[0];
+            gs.radius_min = std::isnan(r0) ? r0 : register_value(ext[i].radius_min ? ~ext[i].radius_min : 0u, r0);
+            gs.radius_max = std::isnan(r0) ? r0 : register_value(ext[i].radius_max, r0);
+        }
+        if (!wants_histogram(*groups[i], gs)) continue;
+        hist[i] = empty_histogram(gs);
+        st = launch_register_histogram(reinterpret_cast<const float4*>(groups[i]->d_constraints), groups[i]->d_radii,
+                                       groups[i]->number_of_terms, hist[i]->edges.data(),
+                                       d_hist + i * register_histogram_bytes(), stream);
+        if (st != kOk) return st;
+        any = true;
+    }
+    if (!any) return kOk;
+    for (size_t i = 0; i < n; ++i) {
+        if (!hist[i]) continue;
+        st = check_cuda(cudaMemcpyAsync(host.data(), d_hist + i * register_histogram_bytes(), host.size(),
+                                        cudaMemcpyDeviceToHost, stream),
+                        "registration histogram D2H");
+        if (st == kOk) st = check_cuda(cudaStreamSynchronize(stream), "registration histogram");
+        if (st != kOk) return st;
+        read_register_histogram(host.data(), hist[i]->count.data(), hist[i]->wmax.data());
+        name_histogram(*hist[i]);
+        out[i].hbins = hist[i];
+    }
+    return kOk;
 }
 }  // namespace
 
@@ -723,6 +768,7 @@ void vis_register_meshless_dataset(VisConfig* c, MeshlessDataset* ds) {
         return;
     }
     const long long multiple = std::max(1LL, (long long)std::max(1, c->_number_of_partial_sums) * std::max(1, c->block_length));
+    std::vector<Group*> large;
     for (int g = 0; g < ds->number_of_groups; ++g) {
         Group& grp = ds->groups[g];
         grp.d_constraints = nullptr;
@@ -740,51 +786,27 @@ void vis_register_meshless_dataset(VisConfig* c, MeshlessDataset* ds) {
         grp.d_number_of_terms = (int)padded;
         if (padded == 0) continue;
         if (registration_alloc(&grp.d_constraints, (size_t)padded, s->registrations, s->stream) != kOk) return;
-        cudaMemsetAsync(grp.d_constraints, 0, sizeof(Constraint) * padded, s->stream);
-        cudaMemcpyAsync(grp.d_constraints, grp.h_constraints, sizeof(Constraint) * grp.number_of_terms,
-                        cudaMemcpyHostToDevice, s->stream);
-        GroupStats gs;
-        // the largest |weight| and the radius extremes: each part folds from
-        // the same start as the serial loop (0, and the first radius), so a
-        // NaN is ignored, or kept from the first radius, alike
-        {
-            constexpr int kMaxParts = 16;
-            const bool radii = grp.h_radii && grp.number_of_terms > 0;
-            const float r0 = radii ? grp.h_radii[0] : 0.f;
-            float wm[kMaxParts], rmin[kMaxParts], rmax[kMaxParts];
-            const int parts = parallel_parts(grp.number_of_terms, kMaxParts, [&](int p, long long b, long long e) {
-                float w = 0.f, lo = r0, hi = r0;
-                for (long long k = b; k < e; ++k) w = std::max(w, std::fabs(grp.h_constraints[k].weight));
-                if (radii)
-                    for (long long k = b; k < e; ++k) {
-                        lo = std::min(lo, grp.h_radii[k]);
-                        hi = std::max(hi, grp.h_radii[k]);
-                    }
-                wm[p] = w;
-                rmin[p] = lo;
-                rmax[p] = hi;
-            });
-            gs.weight_max = 0.f;
-            for (int p = 0; p < parts; ++p) gs.weight_max = std::max(gs.weight_max, wm[p]);
-            if (radii) {
-                gs.radius_min = gs.radius_max = r0;
-                for (int p = 0; p < parts; ++p) {
-                    gs.radius_min = std::min(gs.radius_min, rmin[p]);
-                    gs.radius_max = std::max(gs.radius_max, rmax[p]);
-                }
-                gs.hbins = hbin_histogram(grp, gs);
-            }
-        }
-        {
-            std::lock_guard<std::mutex> lock(g_stats_mu);
-            g_stats[grp.d_constraints] = gs;
-        }
+        const size_t n = (size_t)grp.number_of_terms, pad = (size_t)padded - n;
+        cudaMemcpyAsync(grp.d_constraints, grp.h_constraints, sizeof(Constraint) * n, cudaMemcpyHostToDevice, s->stream);
+        if (pad) cudaMemsetAsync(grp.d_constraints + n, 0, sizeof(Constraint) * pad, s->stream);
         if (grp.h_radii) {
             if (registration_alloc(&grp.d_radii, (size_t)padded, s->registrations, s->stream) != kOk) return;
-            cudaMemsetAsync(grp.d_radii, 0, sizeof(float) * padded, s->stream);
-            cudaMemcpyAsync(grp.d_radii, grp.h_radii, sizeof(float) * grp.number_of_terms, cudaMemcpyHostToDevice,
-                            s->stream);
+            cudaMemcpyAsync(grp.d_radii, grp.h_radii, sizeof(float) * n, cudaMemcpyHostToDevice, s->stream);
+            if (pad) cudaMemsetAsync(grp.d_radii + n, 0, sizeof(float) * pad, s->stream);
         }
+        if (grp.number_of_terms >= kDeviceStats) {
+            large.push_back(&grp);
+            continue;
+        }
+        const GroupStats gs = host_statistics(grp);
+        std::lock_guard<std::mutex> lock(g_stats_mu);
+        g_stats[grp.d_constraints] = gs;
+    }
+    std::vector<GroupStats> stats;
+    if (device_statistics(large, s->post, s->stream, stats) != kOk) return;
+    {
+        std::lock_guard<std::mutex> lock(g_stats_mu);
+        for (size_t i = 0; i < large.size(); ++i) g_stats[large[i]->d_constraints] = stats[i];
     }
     check_cuda(cudaStreamSynchronize(s->stream), "vis_register_meshless_dataset");
 }
@@ -1196,7 +1218,7 @@ struct VisBatch {
     TensorWorkspace tensor;
     Workspace partials, views_table;
     int n_views = 0;
-    long long total_elements = 0;
+    long long total_tiles = 0;
     std::vector<uint64_t> registered;  // batch_signature of the captured launches
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -1261,7 +1283,7 @@ int batch_enqueue(VisBatch* b, ConfigState* s) {
         rc = launch_plain_sum(r, b->partials, nullptr);
         if (rc != kOk) return rc;
     }
-    rc = launch_slice_extract_batch(static_cast<const SliceView*>(b->views_table.ptr), b->n_views, b->total_elements,
+    rc = launch_slice_extract_batch(static_cast<const SliceView*>(b->views_table.ptr), b->n_views, b->total_tiles,
                                     s->stream, nullptr);
     if (rc != kOk) return rc;
     for (VisBatch::SizeClass& c : b->classes) {
@@ -1312,7 +1334,7 @@ int batch_build(VisBatch* b, ConfigState* s, int form) {
     }
     std::vector<SliceView> views;
     std::vector<int> class_done(b->classes.size(), 0);
-    long long elements = 0;
+    long long tiles = 0;
     for (VisBatch::SizeClass& c : b->classes) {
         const size_t per_arr = (size_t)c.nx * (c.ny / 2 + 1), per_img = (size_t)c.nx * c.ny;
         rc = c.arranged.reserve(per_arr * c.views * sizeof(float2));
@@ -1331,7 +1353,7 @@ int batch_build(VisBatch* b, ConfigState* s, int form) {
             SliceView v{};
             v.spectrum = j.sp->data;
             v.arranged = static_cast<float2*>(c.arranged.ptr) + per_arr * class_done[j.size_class]++;
-            v.element_offset = elements;
+            v.first_tile = tiles;
             v.gx = j.sp->grid.x;
             v.gy = j.sp->grid.y;
             v.gz = j.sp->grid.z;
@@ -1345,11 +1367,11 @@ int batch_build(VisBatch* b, ConfigState* s, int form) {
             v.nx = j.samples.x;
             v.ny = j.samples.y;
             views.push_back(v);
-            elements += (long long)per_arr;
+            tiles += slice_tiles(j.samples.x, j.samples.y);
         }
     }
     b->n_views = (int)views.size();
-    b->total_elements = elements;
+    b->total_tiles = tiles;
     if (!views.empty()) {
         rc = b->views_table.reserve(views.size() * sizeof(SliceView));
         if (rc == kOk)

@@ -146,7 +146,7 @@ int launch_slice_extract(const SliceRequest& req, KernelTimer* timer);
 struct SliceView {
     const float2* spectrum;
     float2* arranged;          // float2[nx][ny/2+1]
-    long long element_offset;  // prefix sum of nx*(ny/2+1) over the batch's views
+    long long first_tile;      // prefix sum of slice_tiles(nx, ny) over the batch's views
     int gx, gy, gz;            // the spectrum's lattice extents
     float inv_step;            // 1 / spectral step
     float u[3], v[3];
@@ -154,9 +154,11 @@ struct SliceView {
     int cx, cy, nx, ny;
     int pad;
 };
+// Blocks a view of an nx x ny image takes.
+long long slice_tiles(int nx, int ny);
 // Slices of `number_of_views` views (descriptors in device memory) in one
-// launch; total_elements = sum over views of nx*(ny/2+1).
-int launch_slice_extract_batch(const SliceView* d_views, int number_of_views, long long total_elements,
+// launch; total_tiles = sum over views of slice_tiles(nx, ny).
+int launch_slice_extract_batch(const SliceView* d_views, int number_of_views, long long total_tiles,
                                cudaStream_t stream, KernelTimer* timer);
 
 // Tensor-core form (mv_tc_sum.cu).  A set of groups -- of one or several
@@ -505,6 +507,21 @@ struct GroupStats {
     std::shared_ptr<const HBinStats> hbins;  // SPH / Wendland groups with varying radii
 };
 GroupStats registered_group_stats(const void* d_constraints);
+
+// Registration statistics on the device (mv_register.cu): extremes as ordered
+// integers, the minimum's complement (0: none seen), and a histogram of kHBinFine counts and largest
+// |weight|s.
+struct RegisterStats {
+    uint32_t weight_max, radius_min, radius_max;
+};
+float register_value(uint32_t ordered, float none);
+int launch_register_extremes_clear(RegisterStats* d, int n, cudaStream_t stream);
+int launch_register_extremes(const float4* particles, const float* radii, int n, RegisterStats* out, cudaStream_t stream);
+size_t register_histogram_bytes();
+// edges: kHBinFine + 1 host floats; out: register_histogram_bytes() device bytes.
+int launch_register_histogram(const float4* particles, const float* radii, int n, const float* edges, void* out,
+                              cudaStream_t stream);
+void read_register_histogram(const void* host, int* count, float* wmax);
 
 // Counts a launch of one of this library's kernels (vis_kernel_launch_count).
 void count_launch();
