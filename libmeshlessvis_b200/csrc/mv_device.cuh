@@ -79,14 +79,16 @@ __device__ __forceinline__ double phi_fp64(int basis, double r) {
     switch (basis) {
     case kSph:
         if (r >= (double)0.06f) {
-            double m = kPi * r, c = cos(2.0 * m), s = sin(2.0 * m);
+            double m = kPi * r, c, s;
+            sincos(2.0 * m, &s, &c);
             return (2.3561944901923448 / (m * m * m * m * m * m)) * (c - 1.0) * (c + m * s - 1.0);
         }
         return kPi + r * (-0.007968913156311 + r * (-18.293608272337678));
     case kGaussian: return exp(kPi * r * r);
     case kWendland:
         if (r >= (double)0.24f) {
-            double m = kPi * r, c = cos(2.0 * m), s = sin(2.0 * m);
+            double m = kPi * r, c, s;
+            sincos(2.0 * m, &s, &c);
             double m2 = m * m, m4 = m2 * m2;
             return ((kPi * 7.5) / (m4 * m4)) * (4.0 * m2 - 6.0 + (6.0 - m2) * c + 4.5 * m * s);
         }

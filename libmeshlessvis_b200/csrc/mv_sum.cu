@@ -519,18 +519,24 @@ __global__ void __launch_bounds__(kThreads, 2) fold_sum_kernel(FoldKernelArgs fa
 // fr = s/ds - k interpolating Phi^ (FP64, reference branch points) at the four
 // Chebyshev points of the cell.  Cells never straddle a branch point because
 // ds is chosen so that each branch point is a half-integer multiple of ds.
-__global__ void phi_table_kernel(int basis, double ds, int n, float4* out, int kink) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k > n) return;
+// Four lanes a cell, one Chebyshev point each (the FP64 sine and cosine of one
+// point are the kernel's time: 8 us with a thread a cell, which a small slice
+// waits for).
+constexpr int kTableCells = 32;  // cells a block
+__global__ void __launch_bounds__(4 * kTableCells) phi_table_kernel(int basis, double ds, int n, float4* out, int kink) {
+    const int k = blockIdx.x * kTableCells + threadIdx.x / 4, point = threadIdx.x % 4;
+    const int cell = min(k, n - 1);  // whole warps: the exchanges below take every lane
+    double x[4], f[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) x[i] = 0.5 * cospi((2 * i + 1) / 8.0);
+    const double at = (cell + (point == 0 ? x[0] : point == 1 ? x[1] : point == 2 ? x[2] : x[3])) * ds;
+    const double mine = kink ? phi_kink_fp64(basis, at) : phi_fp64(basis, at);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) f[i] = __shfl_sync(0xffffffffu, mine, i, 4);
+    if (point != 0 || k > n) return;
     if (k == n) {
         out[k] = make_float4(0.f, 0.f, 0.f, 0.f);
         return;
-    }
-    double x[4], f[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        x[i] = 0.5 * cospi((2 * i + 1) / 8.0);
-        f[i] = kink ? phi_kink_fp64(basis, (k + x[i]) * ds) : phi_fp64(basis, (k + x[i]) * ds);
     }
     // Newton divided differences, then expansion to monomials in fr.
     double d[4] = {f[0], f[1], f[2], f[3]};
@@ -632,6 +638,12 @@ SumKernel pick(int basis, int amp) {
     }
 }
 
+// Cells 0 .. n of the table.
+void launch_table(int basis, double ds, int n, float4* out, int kink, cudaStream_t stream) {
+    phi_table_kernel<<<(n + kTableCells) / kTableCells, 4 * kTableCells, 0, stream>>>(basis, ds, n, out, kink);
+    count_launch();
+}
+
 // Table cell width: a branch point of the reference's piecewise Phi^ (0.06f
 // for SPH, 0.24f for Wendland) sits at (K + 1/2) ds.
 double table_cell(int basis) { return basis == kSph ? (double)0.06f / 3.5 : (double)0.24f / 15.5; }
@@ -690,8 +702,7 @@ int phi_table_cells(int basis, double smax) {
 }
 
 void launch_phi_table(int basis, double ds, int n, float4* out, cudaStream_t stream) {
-    phi_table_kernel<<<(n + 128) / 128, 128, 0, stream>>>(basis, ds, n, out, 0);
-    count_launch();
+    launch_table(basis, ds, n, out, 0, stream);
 }
 
 int launch_plain_sum(const SumRequest& req, Workspace& ws, KernelTimer* timer) {
@@ -822,9 +833,7 @@ int launch_plain_sum(const SumRequest& req, Workspace& ws, KernelTimer* timer) {
     a.amp_scale = req.basis == kGaussian ? kPiLog2e : -kPiLog2e;
 
     if (amp == kAmpTable || amp == kAmpShell) {
-        phi_table_kernel<<<(table_n + 128) / 128, 128, 0, req.stream>>>(req.basis, ds, table_n,
-                                                                         const_cast<float4*>(a.table), req.kink);
-        count_launch();
+        launch_table(req.basis, ds, table_n, const_cast<float4*>(a.table), req.kink, req.stream);
     }
 
     const size_t dyn_smem = table_cells * sizeof(float4);
@@ -1021,8 +1030,7 @@ extern "C" int vis_fourier_slice_sum_noalloc(const Constraint* d_constraints, co
     a.amp_scale = basis == kGaussian ? kPiLog2e : -kPiLog2e;
 
     if (amp == kAmpTable) {
-        phi_table_kernel<<<(table_n + 128) / 128, 128, 0, stream>>>(basis, ds, table_n, const_cast<float4*>(a.table), 0);
-        count_launch();
+        launch_table(basis, ds, table_n, const_cast<float4*>(a.table), 0, stream);
     }
     SumKernel k = (L == 8) ? pick<8>(basis, amp) : pick<1>(basis, amp);
     const size_t dyn_smem = amp == kAmpTable ? (size_t)(table_n + 1) * sizeof(float4) : 0;

@@ -1360,31 +1360,43 @@ struct TcCoefArgs {
 // bin the smooth closed form is interpolated instead (phi_smooth_fp64), and
 // the plain form adds the rest for the bin's particles at that k
 // (kAmpShell, mv_sum.cu).  Both sides find the bin from the same float |k|.
-__global__ void tc_coef_kernel(TcCoefArgs c) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (long long)c.nbins * c.nsq) return;
-    const int b = (int)(i / c.nsq), n2 = (int)(i % c.nsq);
+//
+// One bin a blockIdx.y: its nodes and the Chebyshev polynomials at them are
+// computed once a block (a cosine for every (q, p) and |k|^2 made the kernel
+// 0.27 ms on the 156-bin SPH-like set).
+constexpr int kCoefMaxOrder = 16;
+__global__ void __launch_bounds__(128) tc_coef_kernel(TcCoefArgs c) {
+    __shared__ double s_x[kCoefMaxOrder], s_t[kCoefMaxOrder][kCoefMaxOrder];  // nodes x_p; (2 / P) T_q(x_p), q = 0 halved
+    const int b = blockIdx.y;
     const int4 bin = c.bins[b];
     const float4 sp = c.spans[b];
-    const int order = bin.w;
+    const int order = min(bin.w, kCoefMaxOrder);
+    for (int i = threadIdx.x; i < order * order; i += blockDim.x) {
+        const int q = i / order, p = i % order;
+        s_t[q][p] = cospi(q * (2.0 * p + 1.0) / (2.0 * order)) * (q == 0 ? 1.0 : 2.0) / order;
+        if (q == 0) s_x[p] = cospi((2.0 * p + 1.0) / (2.0 * order));
+    }
+    __syncthreads();
+    const int n2 = blockIdx.x * blockDim.x + threadIdx.x;
+    if (n2 >= c.nsq) return;
     const double k = c.step * sqrt((double)n2);
     const float kf = (float)sqrt(c.step * c.step * (double)n2);
     const bool shell = hbin_of(c.edges, c.nbins, kf > 0.f ? c.r0 / kf : INFINITY) == b;
     const double mid = 0.5 * ((double)sp.x + (double)sp.y), half = 0.5 * ((double)sp.y - (double)sp.x);
-    constexpr int kMaxOrder = 16;
-    double f[kMaxOrder], x[kMaxOrder];
-    for (int p = 0; p < order && p < kMaxOrder; ++p) {
-        x[p] = cospi((2.0 * p + 1.0) / (2.0 * order));
-        const double r = k * (mid + half * x[p]);
-        f[p] = shell ? phi_smooth_fp64(c.basis, r) : phi_fp64(c.basis, r);
+    double acc[kCoefMaxOrder];
+#pragma unroll
+    for (int q = 0; q < kCoefMaxOrder; ++q) acc[q] = 0.0;
+    for (int p = 0; p < order; ++p) {
+        const double r = k * (mid + half * s_x[p]);
+        const double f = shell ? phi_smooth_fp64(c.basis, r) : phi_fp64(c.basis, r);
+#pragma unroll
+        for (int q = 0; q < kCoefMaxOrder; ++q)
+            if (q < order) acc[q] = fma(f, s_t[q][p], acc[q]);
     }
-    for (int q = 0; q < order && q < kMaxOrder; ++q) {
-        double acc = 0.0;
-        for (int p = 0; p < order; ++p) acc += f[p] * cospi(q * (2.0 * p + 1.0) / (2.0 * order));
-        acc *= 2.0 / order;
-        if (q == 0) acc *= 0.5;
-        c.coef[(size_t)n2 * c.coef_stride + bin.z + q] = (float)acc;
-    }
+    float* out = c.coef + (size_t)n2 * c.coef_stride + bin.z;
+#pragma unroll
+    for (int q = 0; q < kCoefMaxOrder; ++q)
+        if (q < order) out[q] = (float)acc[q];
 }
 
 // B-operand images of one job (layout in TcJob): one CTA per image (n-tile,
@@ -1496,6 +1508,7 @@ __device__ __forceinline__ void reduce_add(const TcReduceBlock& J, int rep, int 
     const size_t rbase = (size_t)(within / kReps) * J.rank_stride;
     const int4 m = __ldg(J.colmap + col);  // the same for a warp's rows
     Quad t = {};
+#pragma unroll 2
     for (int ks = 0; ks < J.n_splits; ++ks) {
         const size_t li = ((size_t)ks * J.n_mtiles + m_tile) * J.n_ntiles + m.x;
         quad_load(J, li * J.slot_stride + rbase, rl, m, t);
@@ -2864,8 +2877,7 @@ int tensor_enqueue(const std::vector<SumRequest>& groups, const TensorPlan& plan
             ca.edges = bp.edges;
             ca.r0 = (float)phi_branch_point(r.basis);
             ca.coef = static_cast<float*>(ws.coef.ptr) + bg.coef_offset;
-            const long long entries = (long long)bg.nbins * bg.nsq;
-            tc_coef_kernel<<<(unsigned)((entries + 127) / 128), 128, 0, stream>>>(ca);
+            tc_coef_kernel<<<dim3((unsigned)((bg.nsq + 127) / 128), (unsigned)bg.nbins), 128, 0, stream>>>(ca);
             count_launch();
             continue;
         }
