@@ -70,7 +70,7 @@ struct SumKernelArgs {
     const float4* particles;
     const float* radii;
     int n;
-    int chunk;  // particles per split (multiple of kThreads)
+    int chunk;  // particles per split
     Lattice lat;
     int nxc;     // number of x chunks of L
     int n_rest;  // ny * nz
@@ -258,6 +258,7 @@ struct FoldKernelArgs {
     int yrows;     // FY == 2: YP representatives yp; FY == 1: lat.ny
     size_t plane;  // partial sums per split: lat.nx * n_rest
     double2* sums;  // [split][L * 2 FY][gridDim.x * kThreads] running FP64 sums
+    const int* rows;  // (yp, z) rows in the order the threads take them (null: as they lie)
     // kAmpShell: particles sorted into shell_nbins h-bins (classification
     // edges, first particle of each bin) and the branch point r0
     int shell_nbins;
@@ -301,7 +302,8 @@ __global__ void __launch_bounds__(kThreads, 2) fold_sum_kernel(FoldKernelArgs fa
     } else {
         active = t < (long long)fa.xpc * n_rest_f;
         xc = active ? (int)(t / n_rest_f) : 0;
-        const int rf = active ? (int)(t % n_rest_f) : 0;
+        int rf = active ? (int)(t % n_rest_f) : 0;
+        if (fa.rows) rf = fa.rows[rf];
         yr = rf / nz;
         zr = rf % nz;
     }
@@ -523,7 +525,52 @@ __global__ void __launch_bounds__(kThreads, 2) fold_sum_kernel(FoldKernelArgs fa
 // point are the kernel's time: 8 us with a thread a cell, which a small slice
 // waits for).
 constexpr int kTableCells = 32;  // cells a block
-__global__ void __launch_bounds__(4 * kTableCells) phi_table_kernel(int basis, double ds, int n, float4* out, int kink) {
+
+// The rows (yp, z) of a folded lattice sorted by their distance from the x
+// axis (ties by yp, then z): a row's place is the number of rows before it,
+// found for each yp by bisection over z >= 0, along which the distance grows.
+// Every comparison evaluates the same expression, so the places are a
+// permutation.  Four lanes a row, by the blocks of the table's launch behind the
+// cells' own.
+struct RowOrder {
+    int* rows;       // [yrows * nz], null: none wanted
+    int yrows, nz, z0;
+    double ky, kz;
+    int first_block;
+};
+
+__device__ __forceinline__ double row_key(const RowOrder& o, int y, int z) {
+    const double ry = o.ky * y, rz = o.kz * (o.z0 + z);
+    return ry * ry + rz * rz;
+}
+
+__device__ void order_rows(const RowOrder& o) {
+    const int row = ((int)blockIdx.x - o.first_block) * kTableCells + threadIdx.x / 4, count = o.yrows * o.nz;
+    const int y = min(row, count - 1) / o.nz, z = min(row, count - 1) % o.nz;
+    const double key = row_key(o, y, z);
+    int place = 0;
+    for (int yy = threadIdx.x % 4; yy < o.yrows; yy += 4) {
+        int lo = 0, hi = o.nz;  // z' < lo: before the row, z' >= hi: not
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            const double k = row_key(o, yy, mid);
+            const bool before = k < key || (k == key && (yy < y || (yy == y && mid < z)));
+            if (before) lo = mid + 1;
+            else hi = mid;
+        }
+        place += lo;
+    }
+    place += __shfl_xor_sync(0xffffffffu, place, 1);
+    place += __shfl_xor_sync(0xffffffffu, place, 2);
+    if (row < count && threadIdx.x % 4 == 0) o.rows[place] = row;
+}
+
+__global__ void __launch_bounds__(4 * kTableCells) phi_table_kernel(int basis, double ds, int n, float4* out, int kink,
+                                                                    RowOrder order) {
+    if (order.rows && (int)blockIdx.x >= order.first_block) {
+        order_rows(order);
+        return;
+    }
     const int k = blockIdx.x * kTableCells + threadIdx.x / 4, point = threadIdx.x % 4;
     const int cell = min(k, n - 1);  // whole warps: the exchanges below take every lane
     double x[4], f[4];
@@ -638,9 +685,11 @@ SumKernel pick(int basis, int amp) {
     }
 }
 
-// Cells 0 .. n of the table.
-void launch_table(int basis, double ds, int n, float4* out, int kink, cudaStream_t stream) {
-    phi_table_kernel<<<(n + kTableCells) / kTableCells, 4 * kTableCells, 0, stream>>>(basis, ds, n, out, kink);
+// Cells 0 .. n of the table, and the rows' order where one is wanted.
+void launch_table(int basis, double ds, int n, float4* out, int kink, RowOrder order, cudaStream_t stream) {
+    order.first_block = (n + kTableCells) / kTableCells;
+    const int more = order.rows ? (order.yrows * order.nz + kTableCells - 1) / kTableCells : 0;
+    phi_table_kernel<<<order.first_block + more, 4 * kTableCells, 0, stream>>>(basis, ds, n, out, kink, order);
     count_launch();
 }
 
@@ -702,7 +751,7 @@ int phi_table_cells(int basis, double smax) {
 }
 
 void launch_phi_table(int basis, double ds, int n, float4* out, cudaStream_t stream) {
-    launch_table(basis, ds, n, out, 0, stream);
+    launch_table(basis, ds, n, out, 0, RowOrder{}, stream);
 }
 
 int launch_plain_sum(const SumRequest& req, Workspace& ws, KernelTimer* timer) {
@@ -790,7 +839,10 @@ int launch_plain_sum(const SumRequest& req, Workspace& ws, KernelTimer* timer) {
     // cut in 8, the longest runs no longer hold the launch (2.2 ms at 5% issue
     // on 262,144 particles and 128^3 uncut).
     if (amp == kAmpShell) splits = std::min<long long>(8, max_splits);
-    long long chunk = req.n > 0 ? ((req.n + splits - 1) / splits + kThreads - 1) / kThreads * kThreads : kThreads;
+    // Equal runs: a run's last tile may be short.  Rounded up to whole tiles, the
+    // last of 5 splits of 4,373 particles had a quarter of the others' work (450
+    // us and 384 on 100 x 90 x 70).
+    long long chunk = req.n > 0 ? (req.n + splits - 1) / splits : kThreads;
     splits = req.n > 0 ? (req.n + chunk - 1) / chunk : 1;
 
     // Table size: cells up to the largest s = |k|max * hmax (when known).
@@ -815,8 +867,27 @@ int launch_plain_sum(const SumRequest& req, Workspace& ws, KernelTimer* timer) {
     // folded form: the running FP64 sums, 2 FY pairs per representative
     const size_t sums_bytes =
         fold ? (size_t)splits * fold_l * (fold_y ? 4 : 2) * (size_t)blocks_f * kThreads * sizeof(double2) : 0;
-    int st = ws.reserve(part_bytes + table_bytes + sums_bytes);
+    // Rows sorted by their distance from the x axis: a warp's 32 representatives
+    // then have nearly the same |k| and read the same cell or two of the table,
+    // where 32 rows along z read cells far apart, whose bank conflicts bound the
+    // kernel wherever h dk spans several cells: 20,011 SPH particles on 100 x 90
+    // x 70, 2182 us and 1666 with radii of 0.1 to 0.4 (a cell is h k = 0.017),
+    // 1663 and 1654 with 0.01 to 0.1.  The order costs 5 us, beside the table.
+    const long long rows = (long long)yrows * lat.nz;
+    const bool sorted = fold_y && amp == kAmpTable && lat.nz > 1 && lat.z0 >= 0 && std::isfinite(lat.ky * lat.ky) &&
+                        std::isfinite(lat.kz * lat.kz);
+    const size_t rows_bytes = sorted ? (size_t)rows * sizeof(int) : 0;
+    int st = ws.reserve(part_bytes + table_bytes + sums_bytes + rows_bytes);
     if (st != kOk) return st;
+    RowOrder order{};
+    if (sorted) {
+        order.rows = reinterpret_cast<int*>(static_cast<char*>(ws.ptr) + part_bytes + table_bytes + sums_bytes);
+        order.yrows = yrows;
+        order.nz = lat.nz;
+        order.z0 = lat.z0;
+        order.ky = lat.ky;
+        order.kz = lat.kz;
+    }
 
     SumKernelArgs a;
     a.particles = req.particles;
@@ -833,7 +904,7 @@ int launch_plain_sum(const SumRequest& req, Workspace& ws, KernelTimer* timer) {
     a.amp_scale = req.basis == kGaussian ? kPiLog2e : -kPiLog2e;
 
     if (amp == kAmpTable || amp == kAmpShell) {
-        launch_table(req.basis, ds, table_n, const_cast<float4*>(a.table), req.kink, req.stream);
+        launch_table(req.basis, ds, table_n, const_cast<float4*>(a.table), req.kink, order, req.stream);
     }
 
     const size_t dyn_smem = table_cells * sizeof(float4);
@@ -844,6 +915,7 @@ int launch_plain_sum(const SumRequest& req, Workspace& ws, KernelTimer* timer) {
         fa.yrows = yrows;
         fa.plane = plane;
         fa.sums = reinterpret_cast<double2*>(static_cast<char*>(ws.ptr) + part_bytes + table_bytes);
+        fa.rows = order.rows;
         fa.shell_nbins = req.kink ? req.shell_nbins : 0;
         fa.shell_edges = req.shell_edges;
         fa.shell_first = req.shell_first;
@@ -1030,7 +1102,7 @@ extern "C" int vis_fourier_slice_sum_noalloc(const Constraint* d_constraints, co
     a.amp_scale = basis == kGaussian ? kPiLog2e : -kPiLog2e;
 
     if (amp == kAmpTable) {
-        launch_table(basis, ds, table_n, const_cast<float4*>(a.table), 0, stream);
+        launch_table(basis, ds, table_n, const_cast<float4*>(a.table), 0, RowOrder{}, stream);
     }
     SumKernel k = (L == 8) ? pick<8>(basis, amp) : pick<1>(basis, amp);
     const size_t dyn_smem = amp == kAmpTable ? (size_t)(table_n + 1) * sizeof(float4) : 0;

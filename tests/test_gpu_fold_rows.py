@@ -1,0 +1,34 @@
+"""The folded plain form of SPH and Wendland groups with radii on 3D lattices:
+its threads take the (y, z) rows in the order of their distance from the x axis,
+and a split's run of particles ends anywhere.  Every element against the FP64
+oracle, on lattices whose rows tie in distance (cubes), lie in few planes, or
+fill no block, at particle counts around a tile and a split, with radii up to
+where Phi^'s table has its last cell."""
+import numpy as np
+import pytest
+
+import oracle as O
+from libmeshlessvis_b200 import meshless as M
+from libmeshlessvis_b200.workloads import constraints
+
+from util import spectrum_and_views
+
+pytestmark = pytest.mark.gpu
+
+# the suite's tolerance on spectra (rel-L2)
+SPEC_TOL = 1e-5
+
+
+@pytest.mark.parametrize("basis", [M.SPH, M.WENDLAND_D3_C2])
+@pytest.mark.parametrize("grid", [(16, 16, 16), (20, 18, 14), (6, 34, 2), (14, 4, 50), (22, 70, 30)])
+@pytest.mark.parametrize("n,h", [(1, 0.3), (255, 0.02), (1025, 0.1), (3000, 0.9)])
+def test_rows_match_fp64(basis, grid, n, h):
+    rng = np.random.default_rng(n)
+    groups = [(constraints(rng.random((n, 3), dtype=np.float32), rng.standard_normal(n).astype(np.float32)),
+               rng.uniform(0.1 * h, h, n).astype(np.float32), basis)]
+    spec, _ = spectrum_and_views(groups, grid, 1.0, (1.0, 1.0), (8, 4), (16, 16), None, M.FORM_PLAIN)
+    ref = O.spectrum_grid(groups, 1.0, grid)
+    assert O.rel_l2(spec, ref) < SPEC_TOL
+    # the axis planes by themselves: a row out of its place shows there
+    for a, b in ((spec[:, grid[1] // 2], ref[:, grid[1] // 2]), (spec[:, :, 0], ref[:, :, 0])):
+        assert O.rel_l2(a, b) < SPEC_TOL
