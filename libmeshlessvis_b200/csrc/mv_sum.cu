@@ -53,6 +53,9 @@ namespace {
 
 constexpr int kThreads = 256;  // threads per block == particles per tile
 constexpr int kMaxTable = 4096;  // cubic cells held in shared memory (64 KB)
+// Shared memory a block gets without asking for more, static and dynamic
+// together, and the most that a kernel of this file holds statically.
+constexpr size_t kSmemDefault = 48 << 10, kSmemStatic = 8 << 10;
 
 // kAmpGaussRec: decaying Gaussian exp(-pi h^2 |k|^2) factored as
 // exp(-pi h^2 (y^2+z^2)) (one exp2 per particle and thread) times the x factor
@@ -928,7 +931,7 @@ int launch_plain_sum(const SumRequest& req, Workspace& ws, KernelTimer* timer) {
                        : fold_l == 4  ? pick_fold<4, 2>(amp)
                        : fold_l == 5  ? pick_fold<5, 2>(amp)
                                       : pick_fold<6, 2>(amp);
-        if (dyn_smem > 48 * 1024) {
+        if (dyn_smem > kSmemDefault - kSmemStatic) {
             st = check_cuda(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn_smem),
                             "cudaFuncSetAttribute");
             if (st != kOk) return st;
@@ -940,7 +943,7 @@ int launch_plain_sum(const SumRequest& req, Workspace& ws, KernelTimer* timer) {
         st = check_cuda(cudaGetLastError(), "fold_sum_kernel launch");
     } else {
         SumKernel k = (L == 8) ? pick<8>(req.basis, amp) : pick<1>(req.basis, amp);
-        if (dyn_smem > 48 * 1024) {
+        if (dyn_smem > kSmemDefault - kSmemStatic) {
             st = check_cuda(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn_smem),
                             "cudaFuncSetAttribute");
             if (st != kOk) return st;
@@ -1106,7 +1109,7 @@ extern "C" int vis_fourier_slice_sum_noalloc(const Constraint* d_constraints, co
     }
     SumKernel k = (L == 8) ? pick<8>(basis, amp) : pick<1>(basis, amp);
     const size_t dyn_smem = amp == kAmpTable ? (size_t)(table_n + 1) * sizeof(float4) : 0;
-    if (dyn_smem > 48 * 1024) {
+    if (dyn_smem > kSmemDefault - kSmemStatic) {
         st = check_cuda(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn_smem),
                         "cudaFuncSetAttribute");
         if (st != kOk) return st;

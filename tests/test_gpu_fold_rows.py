@@ -32,3 +32,17 @@ def test_rows_match_fp64(basis, grid, n, h):
     # the axis planes by themselves: a row out of its place shows there
     for a, b in ((spec[:, grid[1] // 2], ref[:, grid[1] // 2]), (spec[:, :, 0], ref[:, :, 0])):
         assert O.rel_l2(a, b) < SPEC_TOL
+
+
+@pytest.mark.parametrize("cells", [2500, 2700, 2900, 3070, 3100])
+def test_tables_around_48_kb(cells):
+    """A table between 40 KB and 48 KB leaves the kernel's static shared memory
+    no room below the size a block gets without asking for more."""
+    rng = np.random.default_rng(cells)
+    n, kmax, ds = 300, np.sqrt(3.0) * 8, 0.24 / 15.5
+    radii = rng.uniform(0.002, 0.2, n).astype(np.float32)
+    radii[0] = (cells - 2.5) * ds / kmax
+    groups = [(constraints(rng.random((n, 3), dtype=np.float32), rng.standard_normal(n).astype(np.float32)),
+               radii, M.WENDLAND_D3_C2)]
+    spec, _ = spectrum_and_views(groups, (16, 16, 16), 1.0, (1.0, 1.0), (8, 4), (16, 16), None, M.FORM_PLAIN)
+    assert O.rel_l2(spec, O.spectrum_grid(groups, 1.0, (16, 16, 16))) < SPEC_TOL
