@@ -54,15 +54,13 @@ METRIC_BATCH = "GTerms/s (particle x frequency terms per second; batch of 64 une
 def sum_terms_split(w):
     """Terms per step done by the tensor-core kernel if every group takes it,
     and by the plain form.  The planes l < Kz/2 go to the tensor cores, and so
-    does the Nyquist plane l = Kz/2 (two transposed jobs in the same launch)
-    when Kx/2 fills whole n-tile units (16 c for CTA pairs, else 8); otherwise
-    the plain form sums it.  The rule is the library's tensor_plan."""
+    does the Nyquist plane l = Kz/2 (a transposed job) when Kx and Ky are
+    multiples of 16; otherwise the plain form sums it.  The rule is the
+    library's tensor_plan."""
     kx, ky, kz = w["grid"]
     n = sum(len(c) for c, _, _ in w["groups"])
     lz_tc = kz // 2
-    pairs = os.environ.get("MV_TC_PAIRS", "1")[:1] != "0"
-    pair = pairs and lz_tc > 64 and lz_tc % 16 == 0 and (kx * ky) % 256 == 0
-    nyq_tc = ky % 16 == 0 and (kx // 2) % (16 if pair else 8) == 0 and kx % 2 == 0
+    nyq_tc = ky % 16 == 0 and kx % 16 == 0
     plane = n * kx * ky
     return plane * (lz_tc + (1 if nyq_tc else 0)), (0 if nyq_tc else plane)
 
@@ -71,7 +69,7 @@ def sum_terms_split(w):
 # captures of dram__bytes_read.sum + dram__bytes_write.sum of the full-size
 # launch (profiles/tc_sum_kernel_c3_dram.md names the capture and its
 # command); None where no capture exists.
-DRAM_TRAFFIC_PER_LAUNCH = {("C3", "tc_sum_kernel"): 21.89e9 + 4.44e9}
+DRAM_TRAFFIC_PER_LAUNCH = {("C3", "tc_sum_kernel"): 14.08e9 + 1.43e9}
 
 
 def sum_roofline(stage_t, w, steps, peaks, peak_src, clk, sm_count):
@@ -87,14 +85,15 @@ def sum_roofline(stage_t, w, steps, peaks, peak_src, clk, sm_count):
         per_launch_terms = tc_terms * steps / t_n
         launch_s = t_ms / t_n / 1000.0
         alg = 8.0 * per_launch_terms / launch_s / 1e12
-        issued = 24.0 * per_launch_terms / launch_s / 1e12
+        issued = 12.0 * per_launch_terms / launch_s / 1e12
         peak = peaks.get("bf16_tflops_sustained", 1400.0)
         burst = peaks.get("bf16_tflops", 1590.0)
         return {"bound": "tensor", "achieved": alg, "peak": peak, "unit": "TFLOP/s", "frac": alg / peak,
                 "traffic": DRAM_TRAFFIC_PER_LAUNCH.get((w["name"], "tc_sum_kernel")), "kernel": "tc_sum_kernel",
                 "flops_per_term": 8,
                 "issued_tflops": issued, "issued_frac": issued / peak, "issued_frac_of_burst": issued / burst,
-                "issued_note": "3 FP16 products per term (hi*hi, hi*lo, lo*hi): 24 issued flops per term",
+                "issued_note": "3 FP16 products (hi*hi, hi*lo, lo*hi) of the four real products of a term, which also give "
+                               "the mirrored row's term: 12 issued flops per term",
                 "terms_per_launch": per_launch_terms, "launch_ms": t_ms / t_n, "launches": t_n,
                 "peak_source": f"{peak_src} dense bf16 cuBLAS, sustained (the kernel runs back to back inside a "
                                f"long step; burst {burst})"}
@@ -790,7 +789,7 @@ def run_batch(args):
         peak = peaks.get("bf16_tflops_sustained", 1400.0)
         roofline = {"bound": "tensor", "achieved": alg, "peak": peak, "unit": "TFLOP/s", "frac": alg / peak,
                     "traffic": None, "kernel": "tc_sum_kernel", "flops_per_term": 8,
-                    "issued_tflops": 3 * alg, "issued_frac": 3 * alg / peak,
+                    "issued_tflops": 1.5 * alg, "issued_frac": 1.5 * alg / peak,
                     "timing": "whole-step CUDA-event time (graph replay: every kernel of the step included), so "
                               "achieved is a lower bound for the tensor kernel",
                     "peak_source": f"{peak_src} dense bf16 cuBLAS, sustained"}

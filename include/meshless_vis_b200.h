@@ -101,9 +101,8 @@ int vis_spectrum_render_views(VisSpectrum* spectrum, VisConfig* vis_config, int 
  * shape (lattice, total particles of the dataset, number of groups, form) by
  * timing candidates on the caller's data: the plain form's split-K (2, 4, 6, 8
  * blocks per SM), the tensor form's particle splits (2, 4, 8 waves), the
- * accumulation chain of its single-accumulator tiles (8 or 16 stages; longer
- * chains lose accuracy; the double-buffered tile keeps at most 8), its tile
- * shapes (each VIS_TILE_* shape turned off in turn, for the tensor and auto
+ * accumulation chain of Gaussian groups (8 or 16 stages of 64 particles;
+ * longer chains lose accuracy; other groups keep at most 8), its tile shapes (each VIS_TILE_* shape turned off in turn, for the tensor and auto
  * forms) and, for datasets with h-binned groups, the price of one more h-bin
  * (256, 1024, 4096: the h-bin count).  Each candidate runs
  * vis_spectrum_compute twice (the spectrum holds the last result); the best

@@ -1875,7 +1875,7 @@ size_t operand_cache_limit() {
         return mb >= 0 ? std::min(mb, 1LL << 40) << 20 : -1LL;
     }();
     if (env >= 0) return (size_t)env;
-    // three eighths of the device's memory (the 51 GB of images of 2^24
+    // three eighths of the device's memory (the 26 GB of images of 2^24
     // particles on 384^3 fit a 180 GB device; they are 2.5% faster there than
     // B computed per tile), queried once per device (threads that race here
     // store the same value)

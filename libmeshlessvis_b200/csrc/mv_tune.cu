@@ -2,9 +2,10 @@
 // kernels otherwise derive from fixed rules (TuneParams in mv_internal.h):
 //   plain_waves  split-K of the plain form, in blocks per SM: 2, 4, 6, 8
 //   tc_waves     particle splits of the tensor form, in waves: 2, 4, 8
-//   tc_flush     tensor-core accumulation chain of the single-accumulator
-//                tiles, in stages: 8, 16 (longer chains lose accuracy, so
-//                they are not candidates)
+//   tc_flush     tensor-core accumulation chain of Gaussian jobs in the tiles
+//                wider than 64 columns, in stages of 64 particles: 8, 16
+//                (longer chains lose accuracy, so they are not candidates;
+//                other jobs and tiles keep at most 8)
 //   hbin_job_cost  h-binned groups (SPH / Wendland with per-particle radii):
 //                the price of one more h-bin in the bin-count optimisation,
 //                256, 1024 (default), 4096: lower gives more, narrower bins

@@ -28,8 +28,8 @@ def lib():
 
 def set_operand_cache_limit(nbytes):
     """Device memory the tensor form may keep as precomputed B operands
-    (vis_set_operand_cache_limit): None restores the default (an eighth of
-    device memory, or MV_TC_OPERAND_CACHE_MB), 0 turns them off.  Applies to
+    (vis_set_operand_cache_limit): None restores the default (three eighths
+    of device memory, or MV_TC_OPERAND_CACHE_MB), 0 turns them off.  Applies to
     later computes in this process."""
     lib().vis_set_operand_cache_limit(-1 if nbytes is None else max(0, int(nbytes)))
 
