@@ -1,0 +1,47 @@
+"""Image post-processing at sizes and addresses that fill no vector, warp or
+block: batches of odd images behind a float's and an RGB byte's offset, more
+images than a group, a single pixel, constant and non-positive images."""
+import numpy as np
+import pytest
+
+import oracle as O
+from libmeshlessvis_b200 import _lib as L
+from libmeshlessvis_b200 import meshless as M
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("count,nx,ny", [(1, 1, 1), (3, 5, 7), (2, 33, 127), (5, 64, 64), (70, 31, 9), (1, 257, 513)])
+@pytest.mark.parametrize("offset", [0, 1, 3])
+def test_post_at_odd_sizes(count, nx, ny, offset):
+    import torch
+
+    rng = np.random.default_rng(nx * ny + offset)
+    imgs = rng.uniform(-1.0, 9.0, (count, nx, ny)).astype(np.float32)
+    imgs[0, 0, 0] = 12.0
+    if count > 2:
+        imgs[1] = 2.5
+    n = imgs.size
+    d_img = torch.zeros(n + offset, dtype=torch.float32, device="cuda")[offset:]
+    d_img.copy_(torch.from_numpy(imgs.ravel()))
+    whole = torch.full((3 * n + 2 * offset + 1,), -7.0, dtype=torch.float32, device="cuda")
+    d_rgb = whole[offset:offset + 3 * n]
+    cfg = M.Config(step=(1.0, 1.0), cutoff=(8, 4), samples=(16, 16), block_length=64)
+    lib = M.lib()
+
+    def rgb():
+        cfg.synchronize()
+        got = d_rgb.cpu().numpy().reshape(count, nx, ny, 3)
+        rest = torch.cat((whole[:offset], whole[offset + 3 * n:])).cpu().numpy()
+        assert np.all(rest == -7.0)  # nothing written past the images
+        return got
+
+    torch.cuda.synchronize()
+    assert lib.vis_images_normalize_to_rgb(cfg.ptr, d_img.data_ptr(), count, L.int2(nx, ny), d_rgb.data_ptr()) == 0
+    np.testing.assert_allclose(rgb(), O.normalize_to_rgb(imgs), rtol=1e-6, atol=1e-7)
+    # 3e-7 of the value going in, 1e-6 of the logarithm quotient, through slopes of at most 10
+    for log_scale, color_map in ((0, 1), (1, 2), (1, 3)):
+        assert lib.vis_images_colormap(cfg.ptr, d_img.data_ptr(), count, L.int2(nx, ny), -1.0, 9.0, log_scale, color_map,
+                                       d_rgb.data_ptr()) == 0
+        np.testing.assert_allclose(rgb(), O.colormap(imgs, -1.0, 9.0, log_scale, color_map), rtol=2e-5, atol=2e-5)
+    cfg.close()
