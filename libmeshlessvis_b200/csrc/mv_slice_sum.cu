@@ -235,8 +235,8 @@ __global__ void __launch_bounds__(kThreads, 2) slice_gemm_kernel(SliceSumArgs a)
 // radii and of NaNs read its last, all-zero cell; a tile whose radii all lie in
 // the table's range (a group's usually do: the table reaches its largest radius)
 // uses the index as it is.
-constexpr int kL = 4, kTableWarps = 4, kTableThreads = 32 * kTableWarps;
-constexpr int kTableBlocks = 6;  // an SM: 24 warps of 80 registers
+constexpr int kL = 4;
+constexpr int kTableResident = 24;  // warps an SM, of 80 registers
 constexpr int kXRow = kL / 2;      // float4 of a particle's x factors
 constexpr int kSpan = 4;           // chunks a warp's 32 rows lie in at most (4 + 8 + 12 rows, then more)
 
@@ -246,7 +246,13 @@ __host__ __device__ inline int triangle_threads(int c) {
     return kL * g * (g + 1) / 2;
 }
 
-__global__ void __launch_bounds__(kTableThreads, kTableBlocks) slice_table_kernel(SliceSumArgs a) {
+// Shared memory of a block of `warps` warps beside the table, with the 1 KB the
+// system keeps.
+constexpr int table_block_smem(int warps) { return 8192 + warps * kSpan * 32 * kXRow * 16 + 1024; }
+
+template <int kTableWarps>
+__global__ void __launch_bounds__(32 * kTableWarps, kTableResident / kTableWarps) slice_table_kernel(SliceSumArgs a) {
+    constexpr int kTableThreads = 32 * kTableWarps;
     extern __shared__ float4 s_tab[];  // table cells
     __shared__ uint4 s_q[kThreads];    // Qx, Qy, w, h / ds
     __shared__ float4 s_rot[kThreads];  // the unit rotations of Qx and Qy: their re, their im
@@ -567,20 +573,37 @@ int launch_slice_sum(const SumRequest& req, int nx, int ny, Workspace& ws, Kerne
     int splits = 0;
     if (req.n > 0) {
         const bool by_table = !factored && table;
-        const int threads = by_table ? kTableThreads : kThreads;
-        const long long blocks = by_table ? (triangle_threads(a.cx) + kTableThreads - 1) / kTableThreads
-                                          : (long long)((a.cx + kTile - 1) / kTile) * ((a.cy + kTile - 1) / kTile);
-        if (blocks > INT32_MAX) return set_error(kInvalidValue, "slice too large");
         double ds = 0.0;
         int resident = 2;  // blocks an SM
+        int threads = kThreads;
+        long long blocks = (long long)((a.cx + kTile - 1) / kTile) * ((a.cy + kTile - 1) / kTile);
         if (by_table) {
             ds = phi_table_cell(req.basis);
             const double rmax = lat.kx * std::sqrt(2.0) * (lat.ny - 1);
             a.table_n = phi_table_cells(req.basis, req.radius_max >= 0.f ? rmax * req.radius_max : 1e30);
             a.inv_ds = (float)(1.0 / ds);
-            // shared memory: the table beside 24.3 KB a block
-            resident = std::max(1, std::min<int>(kTableBlocks, (int)(227 * 1024 / (26 * 1024 + 16 * (size_t)a.table_n))));
+            // Warps a block: 4, or 3 where that leaves clearly fewer warps past
+            // the triangle's end (17 warps of rows at a cutoff of 64 take 20 or
+            // 18: 825 us and 758 with 245,066 particles) and the smaller
+            // blocks, each with a table of its own, still fill an SM.  6 are
+            // as fast there, and slower at some sizes of few splits (282 us
+            // against 252 with 60,000 particles).
+            const int warps = (triangle_threads(a.cx) + 31) / 32;
+            double most = 0.0;
+            for (int w : {4, 3}) {
+                const int fit = std::max(1, std::min<int>(kTableResident / w,
+                                                          (int)(227 * 1024 / (table_block_smem(w) + 16 * (size_t)(a.table_n + 1)))));
+                const int count = (warps + w - 1) / w;
+                const double on_an_sm = (double)fit * warps / count;
+                if (on_an_sm > 1.05 * most) {
+                    most = on_an_sm;
+                    threads = 32 * w;
+                    blocks = count;
+                    resident = fit;
+                }
+            }
         }
+        if (blocks > INT32_MAX) return set_error(kInvalidValue, "slice too large");
         a.chunk = split_chunk(req.n, blocks, a.plane, resident);
         splits = (int)(((long long)req.n + a.chunk - 1) / a.chunk);
         if (splits > 65535) return set_error(kInvalidValue, "slice sum: too many splits");
@@ -599,7 +622,7 @@ int launch_slice_sum(const SumRequest& req, int nx, int ny, Workspace& ws, Kerne
         if (by_table) {
             a.table = reinterpret_cast<const float4*>(base + part_bytes);
             launch_phi_table(req.basis, ds, a.table_n, reinterpret_cast<float4*>(base + part_bytes), req.stream);
-            kernel = slice_table_kernel;
+            kernel = threads == 32 * 4 ? slice_table_kernel<4> : slice_table_kernel<3>;
             smem = (size_t)(a.table_n + 1) * sizeof(float4);
         }
         // beside the static shared memory (25 KB at most), over the 48 KB a launch may take by itself
