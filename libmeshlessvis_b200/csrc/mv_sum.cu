@@ -812,7 +812,7 @@ int launch_plain_sum(const SumRequest& req, Workspace& ws, KernelTimer* timer) {
 
     // Split the particle range until the grid holds ~plain_waves blocks per SM
     // (default 6: three waves of the 2 resident blocks; the autotuner may pick
-    // another), keeping at least 4 tiles per split.
+    // another), keeping at least 4 tiles per split where that fills two waves.
     const long long target = (long long)device_sm_count() * active_tune().plain_waves;
     long long max_splits = std::max<long long>(1, (req.n + 4 * kThreads - 1) / (4 * kThreads));
     long long splits = std::min<long long>(std::max<long long>(1, (target + blocks_f - 1) / blocks_f), max_splits);
@@ -836,6 +836,29 @@ int launch_plain_sum(const SumRequest& req, Workspace& ws, KernelTimer* timer) {
             }
         }
         splits = best;
+        // Grids that 4 tiles a split leave below two waves: the splits of least
+        // cost instead, down to one tile.  In particles of one resident block an
+        // SM: two take 1.47 times as long as one; a tile's flush 16, a block's
+        // start 40, its partial sums 0.07.  37 blocks a split, 4,178 particles:
+        // 5 splits (37 SMs hold two blocks) took 354 us, 4 splits 296, 8 (two
+        // blocks on every SM) 232; 8 groups of 1,000 there, a split each of 37
+        // blocks, 1,933 us and 647 so.
+        if (fold && (double)(blocks_f * splits) < 2.0 * resident) {
+            const long long tiles = ((long long)req.n + kThreads - 1) / kThreads;
+            const long long most = std::min<long long>(std::max<long long>(splits, (target + blocks_f - 1) / blocks_f), tiles);
+            double best_cost = 1e300;
+            for (long long sp = 1; sp <= most; ++sp) {
+                const long long per = ((long long)req.n + sp - 1) / sp, grid = blocks_f * ((req.n + per - 1) / per);
+                const long long full = grid / (long long)resident, rest = grid % (long long)resident;
+                const double rounds = 1.47 * (double)full + (rest == 0 ? 0.0 : rest <= device_sm_count() ? 1.0 : 1.47);
+                const double flushes = 16.0 * (double)((per + kThreads - 1) / kThreads);
+                const double cost = ((double)per + flushes + 40.0) * rounds + 0.07 * (double)grid;
+                if (cost < best_cost) {
+                    best_cost = cost;
+                    splits = sp;
+                }
+            }
+        }
     }
     // Each block of the branch part reads the run of a few h-bins, known on
     // the device only and of very uneven length over the blocks (sorted by |k|):

@@ -46,3 +46,16 @@ def test_tables_around_48_kb(cells):
                radii, M.WENDLAND_D3_C2)]
     spec, _ = spectrum_and_views(groups, (16, 16, 16), 1.0, (1.0, 1.0), (8, 4), (16, 16), None, M.FORM_PLAIN)
     assert O.rel_l2(spec, O.spectrum_grid(groups, 1.0, (16, 16, 16))) < SPEC_TOL
+
+
+@pytest.mark.parametrize("radii", ["none", "varying"])
+@pytest.mark.parametrize("grid", [(16, 16, 16), (92, 76, 58)])
+@pytest.mark.parametrize("n", [257, 513, 2049, 4178])
+def test_splits_down_to_one_tile(grid, n, radii):
+    """Grids of few blocks split the particles further, into runs around a tile."""
+    rng = np.random.default_rng(n)
+    h = rng.uniform(0.01, 0.1, n).astype(np.float32) if radii == "varying" else None
+    groups = [(constraints(rng.random((n, 3), dtype=np.float32), rng.standard_normal(n).astype(np.float32)), h,
+               M.WENDLAND_D3_C2)]
+    spec, _ = spectrum_and_views(groups, grid, 1.0, (1.0, 1.0), (8, 4), (16, 16), None, M.FORM_PLAIN)
+    assert O.rel_l2(spec, O.spectrum_grid(groups, 1.0, grid)) < SPEC_TOL
