@@ -46,6 +46,7 @@
 #include "meshless.h"
 #include "mv_device.cuh"
 #include "mv_internal.h"
+#include "mv_row_order.h"
 
 namespace mv {
 
@@ -529,40 +530,12 @@ __global__ void __launch_bounds__(kThreads, 2) fold_sum_kernel(FoldKernelArgs fa
 // waits for).
 constexpr int kTableCells = 32;  // cells a block
 
-// The rows (yp, z) of a folded lattice sorted by their distance from the x
-// axis (ties by yp, then z): a row's place is the number of rows before it,
-// found for each yp by bisection over z >= 0, along which the distance grows.
-// Every comparison evaluates the same expression, so the places are a
-// permutation.  Four lanes a row, by the blocks of the table's launch behind the
-// cells' own.
-struct RowOrder {
-    int* rows;       // [yrows * nz], null: none wanted
-    int yrows, nz, z0;
-    double ky, kz;
-    int first_block;
-};
-
-__device__ __forceinline__ double row_key(const RowOrder& o, int y, int z) {
-    const double ry = o.ky * y, rz = o.kz * (o.z0 + z);
-    return ry * ry + rz * rz;
-}
-
+// Writes the rows' order (mv_row_order.h): four lanes a row, by the blocks of
+// the table's launch behind the cells' own.
 __device__ void order_rows(const RowOrder& o) {
     const int row = ((int)blockIdx.x - o.first_block) * kTableCells + threadIdx.x / 4, count = o.yrows * o.nz;
     const int y = min(row, count - 1) / o.nz, z = min(row, count - 1) % o.nz;
-    const double key = row_key(o, y, z);
-    int place = 0;
-    for (int yy = threadIdx.x % 4; yy < o.yrows; yy += 4) {
-        int lo = 0, hi = o.nz;  // z' < lo: before the row, z' >= hi: not
-        while (lo < hi) {
-            const int mid = (lo + hi) >> 1;
-            const double k = row_key(o, yy, mid);
-            const bool before = k < key || (k == key && (yy < y || (yy == y && mid < z)));
-            if (before) lo = mid + 1;
-            else hi = mid;
-        }
-        place += lo;
-    }
+    int place = rows_before(o, y, z, threadIdx.x % 4, 4);
     place += __shfl_xor_sync(0xffffffffu, place, 1);
     place += __shfl_xor_sync(0xffffffffu, place, 2);
     if (row < count && threadIdx.x % 4 == 0) o.rows[place] = row;

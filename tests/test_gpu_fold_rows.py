@@ -59,3 +59,19 @@ def test_splits_down_to_one_tile(grid, n, radii):
                M.WENDLAND_D3_C2)]
     spec, _ = spectrum_and_views(groups, grid, 1.0, (1.0, 1.0), (8, 4), (16, 16), None, M.FORM_PLAIN)
     assert O.rel_l2(spec, O.spectrum_grid(groups, 1.0, grid)) < SPEC_TOL
+
+
+@pytest.mark.parametrize("step", [0.1, 0.3, 1.0 / 3.0])
+@pytest.mark.parametrize("grid", [(16, 16, 16), (22, 70, 30), (100, 90, 70)])
+def test_rows_at_steps_that_are_no_binary_fractions(grid, step):
+    """The squared distances of the rows are not exact there: rows that tie, or
+    nearly do, still take each place once."""
+    rng = np.random.default_rng(7)
+    n = 1025
+    groups = [(constraints(rng.random((n, 3), dtype=np.float32), rng.standard_normal(n).astype(np.float32)),
+               (rng.uniform(0.01, 0.1, n) / step).astype(np.float32), M.WENDLAND_D3_C2)]
+    spec, _ = spectrum_and_views(groups, grid, step, (step, step), (8, 4), (16, 16), None, M.FORM_PLAIN)
+    ref = O.spectrum_grid(groups, float(np.float32(step)), grid)
+    assert O.rel_l2(spec, ref) < SPEC_TOL
+    worst = np.abs(spec - ref).reshape(-1).max() / np.abs(ref).reshape(-1).max()
+    assert worst < 10 * SPEC_TOL  # no row out of its place, not one element
