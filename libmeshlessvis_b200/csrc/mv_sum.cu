@@ -47,6 +47,7 @@
 #include "mv_device.cuh"
 #include "mv_internal.h"
 #include "mv_row_order.h"
+#include "mv_split_rules.h"
 
 namespace mv {
 
@@ -833,11 +834,10 @@ int launch_plain_sum(const SumRequest& req, Workspace& ws, KernelTimer* timer) {
             }
         }
     }
-    // Each block of the branch part reads the run of a few h-bins, known on
-    // the device only and of very uneven length over the blocks (sorted by |k|):
-    // cut in 8, the longest runs no longer hold the launch (2.2 ms at 5% issue
-    // on 262,144 particles and 128^3 uncut).
-    if (amp == kAmpShell) splits = std::min<long long>(8, max_splits);
+    const size_t plane = fold ? (size_t)lat.nx * n_rest : (size_t)nxc * L * n_rest;
+    // folded form: the running FP64 sums of a split, 2 FY pairs per representative
+    const size_t split_sums = fold ? fold_l * (fold_y ? 4 : 2) * (size_t)blocks_f * kThreads * sizeof(double2) : 0;
+    if (amp == kAmpShell) splits = branch_cuts(max_splits, plane * sizeof(float2) + split_sums);
     // Equal runs: a run's last tile may be short.  Rounded up to whole tiles, the
     // last of 5 splits of 4,373 particles had a quarter of the others' work (450
     // us and 384 on 100 x 90 x 70).
@@ -859,13 +859,10 @@ int launch_plain_sum(const SumRequest& req, Workspace& ws, KernelTimer* timer) {
         if (req.kink) table_n = std::min(table_n, (int)std::llround(phi_branch_point(req.basis) / ds - 0.5) + 1);
     }
 
-    const size_t plane = fold ? (size_t)lat.nx * n_rest : (size_t)nxc * L * n_rest;
     const size_t part_bytes = (plane * splits * sizeof(float2) + 255) / 256 * 256;
     const size_t table_cells = (amp == kAmpTable || amp == kAmpShell) ? (size_t)table_n + 1 : 0;
     const size_t table_bytes = (table_cells * sizeof(float4) + 255) / 256 * 256;
-    // folded form: the running FP64 sums, 2 FY pairs per representative
-    const size_t sums_bytes =
-        fold ? (size_t)splits * fold_l * (fold_y ? 4 : 2) * (size_t)blocks_f * kThreads * sizeof(double2) : 0;
+    const size_t sums_bytes = (size_t)splits * split_sums;
     // Rows sorted by their distance from the x axis: a warp's 32 representatives
     // then have nearly the same |k| and read the same cell or two of the table,
     // where 32 rows along z read cells far apart, whose bank conflicts bound the
