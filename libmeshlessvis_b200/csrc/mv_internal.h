@@ -212,6 +212,7 @@ int tensor_sum_available(const SumRequest& req, int form);
 // per stage.
 struct TcJob {
     const unsigned char* blocks;  // the job's per-particle constants, 64-particle blocks
+    const float4* weights;        // the blocks' weights (put_weight)
     // Item results: each work item owns slot [local item * slot_stride ..] of
     // `slots`: per CTA of the item (rank r at r * 128 * 2 nc_tile elements)
     // its 128 rows of every accumulator column n.  A job whose items span at
@@ -389,9 +390,9 @@ struct TensorPlan {
     std::vector<int> nyq_job_of_group;  // the Nyquist-plane job (h-binned: the first bin's), or -1
     std::vector<int> face_job_of_group; // Gaussian groups: the b = -Ky/2 job, or -1
     std::vector<int> group_binned;      // index into binned, or -1
-    // per job: its particle constants (offset into the particles workspace),
+    // per job: its particle constants and weights (offsets into the particles workspace),
     // coefficient table (offset in floats into coef, SIZE_MAX for none)
-    std::vector<size_t> job_tp, job_coef, job_slot;  // job_slot: byte offset into slots
+    std::vector<size_t> job_tp, job_weights, job_coef, job_slot;  // job_slot: byte offset into slots
     std::vector<int> job_binned;                     // its binned group, or -1
     // the reduction: its parts by launch, their column blocks (job, order; job
     // -1: none) in fours, both in meta

@@ -35,9 +35,9 @@
 // TMEM accumulator (FP32, units of 2^24; 256 columns).  Every TcJob::flush
 // stages (a chain of 12 MMAs a stage) the MMA pauses while the flush warps add
 // the accumulator into an FP32 total in the other 256 TMEM columns, with the
-// mean of what the tensor core's truncation took from it (kChainGain: the
-// error then does not grow with the chain as it did, 4.1e-6 rel-L2 at 16
-// stages; now 0.4-1.5e-6 at the 8 and 16 stages in use).  A work item
+// mean of what the tensor core's truncation took from it (kChainGain: where the
+// error grew with the chain, to 4.1e-6 rel-L2 at 16 stages, it is 0.4 to 2.9e-6
+// at the 8 and 16 stages in use).  A work item
 // (one particle range of one tile) owns a slot of global memory: at its end
 // an item of at most kMaxItemChains chains stores its FP32 total there once,
 // and a longer item adds its FP32 total of every kMaxItemChains chains into
@@ -119,9 +119,18 @@ namespace mv {
 //   offa[64], offb[64]      u32 turns added to every row and column phase
 //   ry[64], rz[64]          float2 exp(-2 pi i Q / 2^32), accurate
 // Particles past the group's end (up to the block boundary) have amp = 0.
+// Behind all blocks of a set, for the flush warps (chain_particles), a float4 a
+// block: the sums of amp^2 of its halves, and 24 times the K steps (16
+// particles) of each that hold weight.
 constexpr int kBlockParticles = 64;
 constexpr int kFieldBytes = 4 * kBlockParticles;
 constexpr int kBlockBytes = 8 * kFieldBytes + 2 * 2 * kFieldBytes;  // 3072
+constexpr int kStepParticles = 16;  // particles of an MMA (K)
+
+// Bytes of a set of blocks with their weights.
+constexpr size_t block_set_bytes(size_t blocks) {
+    return blocks * kBlockBytes + (blocks * sizeof(float4) + 255) / 256 * 256;
+}
 constexpr int kOffQx = 0, kOffQy = kFieldBytes, kOffQz = 2 * kFieldBytes, kOffAmp = 3 * kFieldBytes,
               kOffGam = 4 * kFieldBytes, kOffRho2 = 5 * kFieldBytes, kOffOa = 6 * kFieldBytes,
               kOffOb = 7 * kFieldBytes, kOffRy = 8 * kFieldBytes, kOffRz = 10 * kFieldBytes;
@@ -147,19 +156,28 @@ constexpr float kOperandScale = 4096.f;                     // 2^12 per operand
 constexpr double kInvProductScale = 1.0 / (4096.0 * 4096.0);  // 2^-24
 // The tensor core's FP32 accumulation truncates toward zero, so a chain's total
 // comes out low by a part that grows with the chain: per 64 particles 2.1e-7
-// of the total where the terms' phases are random, up to 4.3e-7 where they
+// of the total where the terms' phases are random, up to 4.9e-7 where they
 // agree and the total approaches the number of particles (the spectrum near
 // its peak), measured against FP64 on 64^3 and 128^3 (uniform and clustered
-// sets of 2^12 to 2^18 particles, chains of 2 to 32 stages).  The flush adds
-// it back: a part kChainGain per particle, growing with |total| / (particles
-// x operand scale^2) up to kChainGainMost times that.  A unit column (the
-// frequency 0 of a Gaussian job's columns, whose factors are exactly 1, so
-// that many low bits are 0) loses 0.8e-7: kChainGainUnit.
+// sets of 2^12 to 2^18 particles, chains of 2 to 32 stages; a chain is no
+// longer than that).  The flush adds it back: a part kChainGain per particle
+// that counts (chain_particles), growing with |total| / (particles x operand
+// scale^2) up to kChainGainMost times that.  A unit column (the frequency 0 of
+// a Gaussian job's columns, whose factors are exactly 1, so that many low bits
+// are 0) loses 0.8e-7: kChainGainUnit.  What it leaves, rel-L2 on 405 sets (15
+// distributions of weights, sparse, zeroed and dominated by one among them; pure
+// phases, Gaussians and h-bins; 64^3, 64 x 64 x 256, 128^3): 0.8e-6 in the mean
+// (1.6e-6 without), 2.9e-6 at most where particles fill the box.  Sets at one
+// phase or a few (all in 0.002 of the box, or on the points of a 4^3 lattice) may
+// lose less than the mean, or nothing: up to 6.3e-6.
 constexpr float kChainGain = 2.1e-7f / 64, kChainAgree = 4.f, kChainGainMost = 2.f, kChainGainUnit = 0.4f;
 // What an item costs beside its stages (the pipeline's fill, the last flush
 // and its slot), and a flush of the single-accumulator tiles, in stages (about
 // 1 us each): 2 and 2, measured on the 256^3 set with chains of 4 to 16.
 constexpr int kItemCost = 2;
+// The longest accumulation chain, in stages: the flush reads a chain's weights
+// with a lane a stage.
+constexpr int kMaxChainStages = 32;
 // An FP32 total in TMEM sums at most this many accumulation chains (random-walk
 // rounding of about 2^-24 sqrt(64) of the total) before it goes to the item's
 // slot.
@@ -535,6 +553,41 @@ __device__ __forceinline__ float2 unit_phase(uint32_t q) {
     return make_float2(c, -s);
 }
 
+// Lanes a chain takes below (as its log2): its stages, at most kMaxChainStages.
+__device__ __forceinline__ int chain_width_log2(int flush) { return flush <= 8 ? 3 : flush <= 16 ? 4 : 5; }
+
+// The particles of a chain as the truncation counts them.  A K step costs a part
+// of the accumulator that stands then, and one of zeros costs nothing: with the
+// accumulator growing as the root of the summed w^2 (random phases), the 16
+// particles of a step count 3/2 sqrt(w^2 up to its stage / w^2 of the chain), and
+// equal weights count in full.  Counted by number alone, zeroed or sparse weights
+// took a correction of up to 3.4e-6 for truncations that were none (2.2e-6 rel-L2
+// where one particle in 64 has a weight, 0.7e-6 so), and a particle that
+// outweighs its chain took it wherever it stood (3.7e-6, 1.5e-6 so).
+//
+// A warp at once for as many chains from `weights` on (of `stages` left in the
+// item) as fit: each in 2^width_log2 lanes, which all return its count.  Not
+// inlined, so that the flush's loop keeps its registers: 2^20 Gaussians on 256^3
+// take 82.0 ms, 84.2 inlined, and 82.8 without any of this.
+__device__ __noinline__ float chain_particles(const float4* weights, int stages, int flush, int width_log2) {
+    const int lane = threadIdx.x & 31, width = 1 << width_log2;
+    const int stage = lane & (width - 1), at = (lane >> width_log2) * flush + stage;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (stage < flush && at < stages) v = weights[at];
+    const float own = v.x + v.y;
+    float upto = own;
+    for (int o = 1; o < width; o <<= 1) {
+        const float t = __shfl_up_sync(0xffffffffu, upto, o, width);
+        if (stage >= o) upto += t;
+    }
+    const float all = __shfl_sync(0xffffffffu, upto, width - 1, width);
+    // the accumulator at the middle of the stage (lanes past the chain count 0)
+    const float middle = fmaxf(fmaf(-0.5f, own, upto), 1e-30f);
+    float sum = all > 1e-24f ? (v.z + v.w) * rsqrtf(__fdividef(all, middle)) : 0.f;
+    for (int o = 1; o < width; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o, width);
+    return sum;
+}
+
 __device__ __forceinline__ uint32_t h2_bits(__half2 h) { return *reinterpret_cast<const uint32_t*>(&h); }
 
 // A producer's two particles as packed pairs: X = (Re z0, Re z1), Y = (Im z0,
@@ -831,18 +884,23 @@ __global__ void __launch_bounds__(kThreads, 1) tc_sum_kernel(TcArgs a) {
             // FP64 slot: columns n, n + 1 (n even) at [(n / 2) * 256 + row * 2]
             float* slot32 = static_cast<float*>(I.slot) + row * 4;
             double* slot64 = static_cast<double*>(I.slot) + row * 2;
+            float counts = 0.f;  // chain_particles of this chain and the next ones
             for (int kk = 0; kk < I.n_chunks; ++kk) {
                 const int k = C + kk;
                 const int b = k % kBufs, u = k / kBufs;
                 const uint32_t acc_col = lane_base + (uint32_t)(b * SH::kN);
+                // the chain's mean truncation, to be added back (kChainGain)
+                const int chain_n = min(I.flush * kKp, I.ke - I.kb - kk * I.flush * kKp);
+                const int width = chain_width_log2(I.flush), in_warp = kk & ((32 >> width) - 1);
+                if (in_warp == 0)
+                    counts = chain_particles(I.job->weights + I.kb / kBlockParticles + kk * I.flush,
+                                             I.n_stages - kk * I.flush, I.flush, width);
+                const float counted = __shfl_sync(0xffffffffu, counts, in_warp << width);
+                const float gain_n = kChainGain * counted;
+                const float agree = kChainAgree * gain_n / ((float)chain_n * kOperandScale * kOperandScale);
                 // warp-uniform outcome: the warp arrives as one below
                 if (!__all_sync(0xffffffffu, mbar_wait(&acc_full[b], u & 1, abort_flag, a.error_flag, a.wait_limit_ns, 4))) break;
                 tc_fence_after();
-                // the chain's total, with its mean truncation added back
-                // (kChainGain)
-                const int chain_n = min(I.flush * kKp, I.ke - I.kb - kk * I.flush * kKp);
-                const float gain_n = kChainGain * (float)chain_n;
-                const float agree = kChainAgree * kChainGain / (kOperandScale * kOperandScale);
                 auto chain_gain = [&](float v) {
                     return 1.f + fminf(fmaf(fabsf(v), agree, gain_n), kChainGainMost * gain_n);
                 };
@@ -1209,6 +1267,19 @@ __device__ __forceinline__ void put_constants(uint8_t* blk, int l, uint32_t qa, 
     reinterpret_cast<float2*>(blk + kOffRz)[l] = rc;
 }
 
+// The weights of a warp's half block (entries l = 0 .. 31 or 32 .. 63).
+__device__ __forceinline__ void put_weight(float4* weights, int l, float amp) {
+    const unsigned any = __ballot_sync(0xffffffffu, amp != 0.f);
+    float w2 = amp * amp;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) w2 += __shfl_xor_sync(0xffffffffu, w2, o);
+    if (l % 32 == 0) {
+        float* out = reinterpret_cast<float*>(weights) + l / 32;
+        out[0] = w2;
+        out[2] = 1.5f * kStepParticles * (float)(((any & 0xffffu) != 0u) + ((any >> 16) != 0u));
+    }
+}
+
 // Half of the row lattice's step (Qx + F Qy) / 2, in turns: the row phases of
 // a pure-phase job are taken about the middle of its lattice, (a, b) =
 // (-1/2, -F/2) (TcJob), and the columns take the offset back.  The odd half
@@ -1220,9 +1291,12 @@ __device__ __forceinline__ uint32_t half_steps(uint32_t qx, uint32_t qy, int fol
 __global__ void tc_prep_kernel(TcPrepArgs p) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     const int padded = (p.n + kBlockParticles - 1) / kBlockParticles * kBlockParticles;
-    if (j >= padded) return;
-    const size_t blk = (size_t)(j / kBlockParticles) * kBlockBytes;
-    const int l = j % kBlockParticles;
+    if (j >= padded) return;  // whole warps
+    const int block = j / kBlockParticles, l = j % kBlockParticles;
+    const size_t blk = (size_t)block * kBlockBytes;
+    auto weights = [&](uint8_t* set) {  // the block's, behind the set's blocks
+        return reinterpret_cast<float4*>(set + (size_t)(padded / kBlockParticles) * kBlockBytes) + block;
+    };
     uint32_t qx = 0, qy = 0, qz = 0;
     float amp = 0.f, gam = 0.f;
     if (j < p.n) {
@@ -1242,16 +1316,20 @@ __global__ void tc_prep_kernel(TcPrepArgs p) {
     const float2 ux = unit_phase(qx), uy = unit_phase(qy), uz = unit_phase(qz);
     const float2 ry = p.exch ? uz : p.fold > 1 ? unit_phase((uint32_t)p.fold * by) : uy;
     put_constants(p.out + blk, l, qx, by, bz, amp, gam, rho2, off, 0u - off, ry, p.exch ? uy : uz);
+    put_weight(weights(p.out), l, amp);
     // a fixed frequency f joins the column offsets and, for Gaussians, the weight
     auto fixed_amp = [&](int f) { return p.gauss ? amp * exp2f(gam * (float)(f * f)) : amp; };
     if (p.out_nyq) {
         const uint32_t o = p.gauss ? 0u : qy >> 1;
-        put_constants(p.out_nyq + blk, l, 0u, qy, qx, fixed_amp(p.half_z), gam, rho2, o, (uint32_t)p.half_z * qz - o,
-                      uy, ux);
+        const float w = fixed_amp(p.half_z);
+        put_constants(p.out_nyq + blk, l, 0u, qy, qx, w, gam, rho2, o, (uint32_t)p.half_z * qz - o, uy, ux);
+        put_weight(weights(p.out_nyq), l, w);
     }
-    if (p.out_face)
-        put_constants(p.out_face + blk, l, 0u, qx, qz, fixed_amp(p.half_y), gam, rho2, 0u,
-                      0u - (uint32_t)p.half_y * qy, ux, uz);
+    if (p.out_face) {
+        const float w = fixed_amp(p.half_y);
+        put_constants(p.out_face + blk, l, 0u, qx, qz, w, gam, rho2, 0u, 0u - (uint32_t)p.half_y * qy, ux, uz);
+        put_weight(weights(p.out_face), l, w);
+    }
 }
 
 // h-bins of a group whose Phi^ does not separate per axis (SPH, Wendland with
@@ -1336,6 +1414,21 @@ __global__ void tc_prep_binned_kernel(TcBinnedPrepArgs p) {
         const uint32_t o = qy >> 1;
         put_constants(p.out_nyq + blk_off, l, 0u, qy, qx, amp, t, 1.f, o, (uint32_t)p.half_z * qz - o, uy,
                       unit_phase(qx));
+    }
+}
+
+// The weights of the blocks that tc_prep_binned_kernel filled (its particles'
+// places are known when it has run): a warp a block, of the planes' blocks and
+// of the Nyquist plane's, whose weights are the same.
+__global__ void __launch_bounds__(256) tc_binned_weight_kernel(uint8_t* out, uint8_t* out_nyq, int blocks) {
+    const int b = blockIdx.x * 8 + threadIdx.x / 32, lane = threadIdx.x & 31;
+    if (b >= blocks) return;
+    const float* amp = reinterpret_cast<const float*>(out + (size_t)b * kBlockBytes + kOffAmp);
+    const size_t weights = (size_t)blocks * kBlockBytes + (size_t)b * sizeof(float4);
+#pragma unroll
+    for (int l = lane; l < kBlockParticles; l += 32) {
+        put_weight(reinterpret_cast<float4*>(out + weights), l, amp[l]);
+        if (out_nyq) put_weight(reinterpret_cast<float4*>(out_nyq + weights), l, amp[l]);
     }
 }
 
@@ -1844,15 +1937,17 @@ bool tc_pairs_enabled() {
 // and h-binned jobs take 8 stages of 64 particles, Gaussian jobs of the
 // single-accumulator tiles (kWide, kPair), which stall the MMA for every
 // flush, the tuned value (16: 84 ms on 2^20 particles and 256^3, 90 at 8),
-// and the narrow tiles at most 8.  MV_TC_FLUSH_STAGES (1..1024) overrides all.
+// and the narrow tiles at most 8.  MV_TC_FLUSH_STAGES (1..1024) overrides all;
+// no chain is longer than kMaxChainStages.
 int tc_flush_stages(int mode, bool gauss) {
     static const int env = [] {
         const char* e = std::getenv("MV_TC_FLUSH_STAGES");
         const int x = e ? std::atoi(e) : 0;
         return (x >= 1 && x <= 1024) ? x : 0;
     }();
-    if (env) return env;
-    return narrow_mode(mode) || !gauss ? std::min(8, active_tune().tc_flush) : active_tune().tc_flush;
+    if (env) return std::min(env, kMaxChainStages);
+    return narrow_mode(mode) || !gauss ? std::min(8, active_tune().tc_flush)
+                                       : std::min(kMaxChainStages, active_tune().tc_flush);
 }
 
 // B-operand images are made for jobs whose every image is copied by at
@@ -2134,7 +2229,8 @@ int tensor_plan(const std::vector<SumRequest>& groups, TensorPlan& plan) {
     double launch_terms = 1.0;
     for (const SumRequest& r : groups)
         launch_terms += (double)std::max(0, r.n) * r.lat.nx * r.lat.ny * std::max(1, r.lat.nz - 1);
-    auto add_job = [&](TcJob j, int mode, bool image_ok, size_t tp_offset, int cls, int part, size_t coef_offset) {
+    auto add_job = [&](TcJob j, int mode, bool image_ok, size_t tp_offset, size_t weights_offset, int cls, int part,
+                       size_t coef_offset) {
         // equal n-tiles of at most kNc c values: 192 planes -> 96 + 96 (two
         // N = 192 MMAs) rather than 128 + 64 (an N = 128 one, bound by its
         // shared-memory operand reads); multiples of 16 for kPair
@@ -2192,6 +2288,7 @@ int tensor_plan(const std::vector<SumRequest>& groups, TensorPlan& plan) {
         plan.jobs.push_back(j);
         plan.bimg_offset.push_back(img_off);
         plan.job_tp.push_back(tp_offset);
+        plan.job_weights.push_back(weights_offset);
         plan.job_coef.push_back(coef_offset);
         plan.job_binned.push_back(coef_offset == SIZE_MAX ? -1 : (int)plan.binned.size());
         plan.job_slot.push_back(plan.slot_bytes);
@@ -2317,7 +2414,8 @@ int tensor_plan(const std::vector<SumRequest>& groups, TensorPlan& plan) {
             bg.coef_stride = (bg.total_q + kCoefLine - 1) / kCoefLine * kCoefLine;  // the reduction reads whole lines
             bg.coef_count = (size_t)bg.coef_stride * bg.nsq;  // [n2][bin's blocks]
             plan.coef_bytes += (bg.coef_count * sizeof(float) + 255) / 256 * 256;
-            const size_t blocks_bytes = (size_t)blocks * kBlockBytes;
+            const size_t blocks_bytes = block_set_bytes((size_t)blocks);
+            auto weights_at = [&](size_t set, int block) { return set + (size_t)blocks * kBlockBytes + (size_t)block * sizeof(float4); };
             plan.tp_bytes += blocks_bytes;
             // the Nyquist plane as a transposed job needs whole 8-column
             // blocks of either sign of a
@@ -2348,7 +2446,8 @@ int tensor_plan(const std::vector<SumRequest>& groups, TensorPlan& plan) {
                 j.fold = bfold;
                 j.coef_stride = bg.coef_stride;
                 const size_t tp = plan.tp_offset.back() + (size_t)first_block[b] * kBlockBytes;
-                const int jm = add_job(j, mode_of(j.lz_tc, (long long)j.kx * j.ky), true, tp, cls, 0, coef_off);
+                const int jm = add_job(j, mode_of(j.lz_tc, (long long)j.kx * j.ky), true, tp,
+                                       weights_at(plan.tp_offset.back(), first_block[b]), cls, 0, coef_off);
                 if (first_job < 0) {
                     first_job = jm;
                     set_part(cls, 0, kPartPlanes, j, -1, -bfold, INT32_MIN, 1, 0);
@@ -2364,7 +2463,8 @@ int tensor_plan(const std::vector<SumRequest>& groups, TensorPlan& plan) {
                     t.b_base = 0;
                     t.c_base = -kx / 2;
                     const size_t tpn = plan.tp_nyq_offset.back() + (size_t)first_block[b] * kBlockBytes;
-                    const int jn = add_job(t, mode_of(t.lz_tc, t.ky), false, tpn, cls, 1, coef_off);
+                    const int jn = add_job(t, mode_of(t.lz_tc, t.ky), false, tpn,
+                                           weights_at(plan.tp_nyq_offset.back(), first_block[b]), cls, 1, coef_off);
                     if (first_nyq < 0) {
                         first_nyq = jn;
                         set_part(cls, 1, kPartNyquist, t, 0, -1, INT32_MIN, 1, lz_tc);
@@ -2378,8 +2478,8 @@ int tensor_plan(const std::vector<SumRequest>& groups, TensorPlan& plan) {
             continue;
         }
         // ------------------------------------------------ separable group
-        const size_t blocks_bytes =
-            (size_t)((std::max(0, r.n) + kBlockParticles - 1) / kBlockParticles) * kBlockBytes;
+        const size_t blocks = (size_t)((std::max(0, r.n) + kBlockParticles - 1) / kBlockParticles);
+        const size_t blocks_bytes = block_set_bytes(blocks), weights_at = blocks * kBlockBytes;
         plan.tp_bytes += blocks_bytes;
         // Row fold of a group whose terms are pure phases: the F of {1, 2, 4}
         // whose columns F lz_tc fill the MMAs best.  A CTA-pair (or narrow)
@@ -2411,7 +2511,7 @@ int tensor_plan(const std::vector<SumRequest>& groups, TensorPlan& plan) {
         j.exch = exch ? 1 : 0;
         j.unit_col = gauss ? 1 : 0;
         plan.job_of_group.push_back(add_job(j, mode_of(j.lz_tc, (long long)j.kx * j.ky), true, plan.tp_offset.back(),
-                                            cls, 0, SIZE_MAX));
+                                            plan.tp_offset.back() + weights_at, cls, 0, SIZE_MAX));
         // mirrors: pure phases in (-1/2, -F/2), every one; Gaussians in 0,
         // where a = 0 (exchanged: b = 0) is its own
         if (exch) set_part(cls, 0, kPartExchanged, j, 0, 0, 1, 1, 0);
@@ -2435,7 +2535,7 @@ int tensor_plan(const std::vector<SumRequest>& groups, TensorPlan& plan) {
             t.lz_tc = kx;
             t.c_base = -kx / 2;
             const size_t tpn = plan.tp_nyq_offset.back();
-            plan.nyq_job_of_group.back() = add_job(t, mode_of(kx, t.ky), false, tpn, cls, 1, SIZE_MAX);  // no reuse
+            plan.nyq_job_of_group.back() = add_job(t, mode_of(kx, t.ky), false, tpn, tpn + weights_at, cls, 1, SIZE_MAX);  // no reuse
             if (gauss) set_part(cls, 1, kPartNyquist, t, 0, 0, 1, 1, lz_tc);
             else set_part(cls, 1, kPartNyquist, t, 0, -1, INT32_MIN, 1, lz_tc);
         }
@@ -2447,7 +2547,7 @@ int tensor_plan(const std::vector<SumRequest>& groups, TensorPlan& plan) {
             t.ky = (kx / 2 + 1 + 7) / 8 * 8;
             t.lz_tc = lz_tc;
             t.c_base = 0;
-            plan.face_job_of_group.back() = add_job(t, mode_of(lz_tc, t.ky), false, tpf, cls, 2, SIZE_MAX);
+            plan.face_job_of_group.back() = add_job(t, mode_of(lz_tc, t.ky), false, tpf, tpf + weights_at, cls, 2, SIZE_MAX);
             set_part(cls, 2, kPartFace, t, 0, 0, 1, exch ? 1 : 0, -ky / 2);
         }
     }
@@ -2622,6 +2722,7 @@ int tensor_reserve_upload(TensorPlan& plan, TensorWorkspace& ws, cudaStream_t st
         job.bimg = plan.bimg_offset[j] == SIZE_MAX ? nullptr
                                                    : static_cast<const unsigned char*>(ws.bimg.ptr) + plan.bimg_offset[j];
         job.blocks = reinterpret_cast<const unsigned char*>(tp_base + plan.job_tp[j]);
+        job.weights = reinterpret_cast<const float4*>(tp_base + plan.job_weights[j]);
         job.slots = static_cast<char*>(ws.slots.ptr) + plan.job_slot[j];
         job.colmap = reinterpret_cast<const int4*>(static_cast<char*>(ws.meta.ptr) + plan.colmap_offset) +
                      plan.job_colmap[j];
@@ -2865,6 +2966,8 @@ int tensor_enqueue(const std::vector<SumRequest>& groups, const TensorPlan& plan
                 bp.order = index_out;
             }
             tc_prep_binned_kernel<<<(r.n + 255) / 256, 256, 0, stream>>>(bp);
+            count_launch();
+            tc_binned_weight_kernel<<<(unsigned)((blocks + 7) / 8), 256, 0, stream>>>(bp.out, bp.out_nyq, (int)blocks);
             count_launch();
             TcCoefArgs ca;
             ca.basis = r.basis;
