@@ -113,6 +113,8 @@ int launch_plain_sum(const SumRequest& req, Workspace& ws, KernelTimer* timer);
 double phi_table_cell(int basis);
 int phi_table_cells(int basis, double smax);
 void launch_phi_table(int basis, double ds, int n, float4* out, cudaStream_t stream);
+// Lets a kernel's launches take the largest table as dynamic shared memory.
+int allow_table_memory(const void* kernel);
 
 // One group's direct slice (mv_slice_sum.cu) into the C2R layout
 // float2[nx][ny/2+1]: every element written, or (req.accumulate) the samples

@@ -86,6 +86,7 @@ __device__ __forceinline__ void add_tile(double2* sums, size_t stride, const flo
 constexpr int kTile = 64, kStage = 32;
 constexpr int kFRow = kTile + 4;  // floats of a particle's 64 factors' re (or im), padded against bank conflicts
 constexpr size_t kGemmSmem = (size_t)kStage * 4 * kFRow * sizeof(float);
+static_assert(kGemmSmem + kThreads * (sizeof(uint4) + sizeof(float4)) <= 48 << 10, "within what a launch may take");
 
 template <bool GAUSS>
 __global__ void __launch_bounds__(kThreads, 2) slice_gemm_kernel(SliceSumArgs a) {
@@ -625,10 +626,10 @@ int launch_slice_sum(const SumRequest& req, int nx, int ny, Workspace& ws, Kerne
             kernel = threads == 32 * 4 ? slice_table_kernel<4> : slice_table_kernel<3>;
             smem = (size_t)(a.table_n + 1) * sizeof(float4);
         }
-        // beside the static shared memory (25 KB at most), over the 48 KB a launch may take by itself
-        if (smem > 20 * 1024) {
-            st = check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                            "cudaFuncSetAttribute");
+        // beside the static shared memory (25 KB at most; the product kernel's
+        // fits), over the 48 KB a launch may take by itself
+        if (by_table && smem > 20 * 1024) {
+            st = allow_table_memory(reinterpret_cast<const void*>(kernel));
             if (st != kOk) return st;
         }
         timer_begin(timer, 0, req.stream);

@@ -721,6 +721,15 @@ int shell_representatives(const Lattice& lat, int xp_count, int yrows, const uin
 
 double phi_table_cell(int basis) { return table_cell(basis); }
 
+// The limit belongs to the kernel, for all threads of the process: set to the
+// most a table takes, whatever this call's does, so that no thread lowers it
+// between another's call here and its launch.
+int allow_table_memory(const void* kernel) {
+    return check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (kMaxTable + 1) * (int)sizeof(float4)),
+                      "cudaFuncSetAttribute");
+}
+
 // Beyond kMaxTable cells (s > 63 for Wendland, > 60 for SPH) |Phi^| < 1e-11
 // and the zero cell stands in for it.
 int phi_table_cells(int basis, double smax) {
@@ -925,8 +934,7 @@ int launch_plain_sum(const SumRequest& req, Workspace& ws, KernelTimer* timer) {
                        : fold_l == 5  ? pick_fold<5, 2>(amp)
                                       : pick_fold<6, 2>(amp);
         if (dyn_smem > kSmemDefault - kSmemStatic) {
-            st = check_cuda(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn_smem),
-                            "cudaFuncSetAttribute");
+            st = allow_table_memory(reinterpret_cast<const void*>(k));
             if (st != kOk) return st;
         }
         timer_begin(timer, 0, req.stream);
@@ -937,8 +945,7 @@ int launch_plain_sum(const SumRequest& req, Workspace& ws, KernelTimer* timer) {
     } else {
         SumKernel k = (L == 8) ? pick<8>(req.basis, amp) : pick<1>(req.basis, amp);
         if (dyn_smem > kSmemDefault - kSmemStatic) {
-            st = check_cuda(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn_smem),
-                            "cudaFuncSetAttribute");
+            st = allow_table_memory(reinterpret_cast<const void*>(k));
             if (st != kOk) return st;
         }
         timer_begin(timer, 0, req.stream);
@@ -1103,8 +1110,7 @@ extern "C" int vis_fourier_slice_sum_noalloc(const Constraint* d_constraints, co
     SumKernel k = (L == 8) ? pick<8>(basis, amp) : pick<1>(basis, amp);
     const size_t dyn_smem = amp == kAmpTable ? (size_t)(table_n + 1) * sizeof(float4) : 0;
     if (dyn_smem > kSmemDefault - kSmemStatic) {
-        st = check_cuda(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn_smem),
-                        "cudaFuncSetAttribute");
+        st = allow_table_memory(reinterpret_cast<const void*>(k));
         if (st != kOk) return st;
     }
     k<<<dim3((unsigned)blocks_f, (unsigned)splits), kThreads, dyn_smem, stream>>>(a);
