@@ -769,39 +769,43 @@ void vis_register_meshless_dataset(VisConfig* c, MeshlessDataset* ds) {
     }
     const long long multiple = std::max(1LL, (long long)std::max(1, c->_number_of_partial_sums) * std::max(1, c->block_length));
     std::vector<Group*> large;
-    for (int g = 0; g < ds->number_of_groups; ++g) {
-        Group& grp = ds->groups[g];
+    auto copy_group = [&](Group& grp) {
         grp.d_constraints = nullptr;
         grp.d_radii = nullptr;
         grp.d_number_of_terms = 0;
         if (grp.number_of_terms < 0 || (grp.number_of_terms > 0 && !grp.h_constraints)) {
             set_error(kInvalidValue, "vis_register_meshless_dataset: group without host constraints");
-            return;
+            return false;
         }
         const long long padded = (grp.number_of_terms + multiple - 1) / multiple * multiple;
         if (padded > INT32_MAX) {
             set_error(kInvalidValue, "vis_register_meshless_dataset: too many terms");
-            return;
+            return false;
         }
         grp.d_number_of_terms = (int)padded;
-        if (padded == 0) continue;
-        if (registration_alloc(&grp.d_constraints, (size_t)padded, s->registrations, s->stream) != kOk) return;
+        if (padded == 0) return true;
+        if (registration_alloc(&grp.d_constraints, (size_t)padded, s->registrations, s->stream) != kOk) return false;
         const size_t n = (size_t)grp.number_of_terms, pad = (size_t)padded - n;
         cudaMemcpyAsync(grp.d_constraints, grp.h_constraints, sizeof(Constraint) * n, cudaMemcpyHostToDevice, s->stream);
         if (pad) cudaMemsetAsync(grp.d_constraints + n, 0, sizeof(Constraint) * pad, s->stream);
         if (grp.h_radii) {
-            if (registration_alloc(&grp.d_radii, (size_t)padded, s->registrations, s->stream) != kOk) return;
+            if (registration_alloc(&grp.d_radii, (size_t)padded, s->registrations, s->stream) != kOk) return false;
             cudaMemcpyAsync(grp.d_radii, grp.h_radii, sizeof(float) * n, cudaMemcpyHostToDevice, s->stream);
             if (pad) cudaMemsetAsync(grp.d_radii + n, 0, sizeof(float) * pad, s->stream);
         }
         if (grp.number_of_terms >= kDeviceStats) {
             large.push_back(&grp);
-            continue;
+            return true;
         }
         const GroupStats gs = host_statistics(grp);
         std::lock_guard<std::mutex> lock(g_stats_mu);
         g_stats[grp.d_constraints] = gs;
-    }
+        return true;
+    };
+    // a group that is refused ends the registration; the groups before it stay
+    // registered, statistics and all
+    for (int g = 0; g < ds->number_of_groups; ++g)
+        if (!copy_group(ds->groups[g])) break;
     std::vector<GroupStats> stats;
     if (device_statistics(large, s->post, s->stream, stats) != kOk) return;
     {
