@@ -180,6 +180,7 @@ GroupStats host_statistics(const Group& grp) {
         for (int k = 0; k < grp.number_of_terms; ++k) {
             gs.radius_min = std::min(gs.radius_min, grp.h_radii[k]);
             gs.radius_max = std::max(gs.radius_max, grp.h_radii[k]);
+            gs.radius_nan = gs.radius_nan || std::isnan(grp.h_radii[k]);
         }
     }
     if (wants_histogram(grp, gs)) {
@@ -232,6 +233,7 @@ int device_statistics(const std::vector<Group*>& groups, Workspace& scratch, cud
             const float r0 = groups[i]->h_radii[0];
             gs.radius_min = std::isnan(r0) ? r0 : register_value(ext[i].radius_min ? ~ext[i].radius_min : 0u, r0);
             gs.radius_max = std::isnan(r0) ? r0 : register_value(ext[i].radius_max, r0);
+            gs.radius_nan = ext[i].radius_nan != 0u;
         }
         if (!wants_histogram(*groups[i], gs)) continue;
         hist[i] = empty_histogram(gs);
@@ -883,6 +885,7 @@ void vis_fourier_volume_rendering(MeshlessDataset* ds, VisConfig* c) {
             r.radius_min = gs.radius_min;
             r.radius_max = gs.radius_max;
             r.weight_max = gs.weight_max;
+            r.radius_nan = gs.radius_nan;
         }
         r.error_flag = static_cast<int*>(s->error_word.ptr);
         r.n = grp.number_of_terms;
@@ -1009,6 +1012,7 @@ SumRequest spectrum_request(const VisSpectrum* sp, const Group& grp, ConfigState
     r.radius_min = gs.radius_min;
     r.radius_max = gs.radius_max;
     r.weight_max = gs.weight_max;
+    r.radius_nan = gs.radius_nan;
     r.hbins = gs.hbins.get();  // kept alive by the registration table until unregistered
     r.n = grp.number_of_terms;
     r.basis = (int)grp.basis_function_id;

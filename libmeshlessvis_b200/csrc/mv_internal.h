@@ -72,6 +72,7 @@ struct SumRequest {
     float radius_min;         // smallest / largest radius and largest |weight|
     float radius_max;         //   when known (registration), else < 0
     float weight_max;
+    bool radius_nan;          // some radius is a NaN, which the extremes pass over
     const HBinStats* hbins;   // smoothing-length histogram (registration), or null
     int n;
     int basis;
@@ -507,15 +508,16 @@ TuneParams tuned_params(int kx, int ky, int kz, long long n_total, int n_groups,
 // and keyed by the group's device particle pointer; all -1 if unknown.
 struct GroupStats {
     float radius_min = -1.f, radius_max = -1.f, weight_max = -1.f;
+    bool radius_nan = false;  // some radius is a NaN (the extremes pass over it)
     std::shared_ptr<const HBinStats> hbins;  // SPH / Wendland groups with varying radii
 };
 GroupStats registered_group_stats(const void* d_constraints);
 
 // Registration statistics on the device (mv_register.cu): extremes as ordered
-// integers, the minimum's complement (0: none seen), and a histogram of kHBinFine counts and largest
-// |weight|s.
+// integers, the minimum's complement (0: none seen), whether a radius is a NaN,
+// and a histogram of kHBinFine counts and largest |weight|s.
 struct RegisterStats {
-    uint32_t weight_max, radius_min, radius_max;
+    uint32_t weight_max, radius_min, radius_max, radius_nan;
 };
 float register_value(uint32_t ordered, float none);
 int launch_register_extremes_clear(RegisterStats* d, int n, cudaStream_t stream);

@@ -24,6 +24,7 @@ __global__ void __launch_bounds__(256) register_extremes_kernel(const float4* __
                                                                 const float* __restrict__ radii, int n,
                                                                 RegisterStats* out) {
     uint32_t w = 0u, lo = 0u, hi = 0u;
+    bool nan = false;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const float a = fabsf(particles[i].w);
         if (a >= 0.f) w = max(w, ordered_bits(__float_as_uint(a)));
@@ -33,16 +34,20 @@ __global__ void __launch_bounds__(256) register_extremes_kernel(const float4* __
                 const uint32_t o = ordered_bits(__float_as_uint(r));
                 lo = max(lo, ~o);
                 hi = max(hi, o);
+            } else {
+                nan = true;
             }
         }
     }
     w = __reduce_max_sync(0xffffffffu, w);
     lo = __reduce_max_sync(0xffffffffu, lo);
     hi = __reduce_max_sync(0xffffffffu, hi);
+    nan = __any_sync(0xffffffffu, nan);
     if ((threadIdx.x & 31) == 0) {
         if (w) atomicMax(&out->weight_max, w);
         if (lo) atomicMax(&out->radius_min, lo);
         if (hi) atomicMax(&out->radius_max, hi);
+        if (nan) atomicMax(&out->radius_nan, 1u);
     }
 }
 

@@ -232,10 +232,11 @@ __global__ void __launch_bounds__(kThreads, 2) slice_gemm_kernel(SliceSumArgs a)
 // x Qy} for the second -- and keeps them packed in shared memory; the loop over
 // particles rotates them once, and takes the next particle's sines at y while it
 // sums one.  No one pipe binds it: shared memory, the packed operations' FMA
-// pipe and issue are each about half busy.  Indices past the table, of negative
-// radii and of NaNs read its last, all-zero cell; a tile whose radii all lie in
-// the table's range (a group's usually do: the table reaches its largest radius)
-// uses the index as it is.
+// pipe and issue are each about half busy.  Indices past the table and of
+// negative radii read its last, all-zero cell (a NaN radius reads it too, but its
+// offset in the cell is a NaN, and so are its terms); a tile whose radii all lie
+// in the table's range (a group's usually do: the table reaches its largest
+// radius) uses the index as it is.
 constexpr int kL = 4;
 constexpr int kTableResident = 24;  // warps an SM, of 80 registers
 constexpr int kXRow = kL / 2;      // float4 of a particle's x factors
@@ -543,7 +544,8 @@ int launch_slice_sum(const SumRequest& req, int nx, int ny, Workspace& ws, Kerne
     if (req.n < 0) return set_error(kInvalidValue, "negative number of terms");
     if (req.n > 0 && req.particles == nullptr) return set_error(kInvalidValue, "dataset group has no device particles");
     const bool known = req.radii && req.radius_min >= 0.f && std::isfinite(req.radius_max);
-    const bool uniform = known && req.radius_min == req.radius_max;
+    // one radius for all: a NaN among equal radii makes its particle's terms NaNs
+    const bool uniform = known && !req.radius_nan && req.radius_min == req.radius_max;
     const bool factored = !req.radii || uniform;
     const bool gauss = !factored && known && (req.basis == kGaussian || req.basis == kGaussianDecaying);
     const bool table = !factored && (req.basis == kSph || req.basis == kWendland) && lat.kx == lat.ky &&

@@ -70,3 +70,14 @@ def test_radii_past_the_table_and_zero_radii():
     h[::7] = 5.0
     h[3::11] = 0.0
     _check([(c, h, b)], (32, 32), (64, 64))
+
+
+@pytest.mark.parametrize("basis", [M.SPH, M.WENDLAND_D3_C2, M.GAUSSIAN_DECAYING])
+@pytest.mark.parametrize("n", [300, 8192])  # statistics from the host, from the device
+@pytest.mark.parametrize("cutoff", [(16, 16), (16, 40)])
+def test_a_nan_among_equal_radii_shows(basis, n, cutoff):
+    """The particle's terms are NaNs, and so is every pixel: not the image of the
+    radius that the others have."""
+    c, h, b = _group(np.random.default_rng(5), n, basis, "uniform", 0.05)
+    h[n // 2] = np.nan
+    assert np.isnan(render_direct([(c, h, b)], (1.0, 1.0), cutoff, U, V, (2 * cutoff[0], 2 * cutoff[1]))).all()
