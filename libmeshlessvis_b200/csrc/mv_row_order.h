@@ -11,6 +11,26 @@
 
 namespace mv {
 
+// Whether a sum of n particles is worth the order.  `cells`: the cells of Phi^'s
+// table that one step of k spans at the largest radius (negative: not known).
+// Sorted rows save bank conflicts, a part of a particle's time that grows with
+// the cells between the lanes' rows, and the order costs 2 to 6 us, so small sums
+// and those of few cells lose by it.  us a group of 8, rows as they lie and
+// sorted:
+//   cells      1.2                  5.8                  23
+//   62         34.3  40.6           34.3  42.0           38.4  42.6   100 x 90 x 70
+//   250        73.4  80.5           77.4  81.5           86.7  81.6
+//   2000       186   194            191   195            229   196
+//   4000       349   358            359   358            429   362
+//   250        71.3  75.5           75.5  76.1           84.7  77.5   92 x 76 x 58
+//   2000       122   127            131   127            151   128
+// The line, n cells^2 = 45,000, is within 3% of the better one in all of these.
+constexpr double kRowOrderWorth = 45000.0;
+
+MV_HD bool rows_worth_sorting(long long n, double cells) {
+    return cells < 0.0 || (double)n * cells * cells >= kRowOrderWorth;
+}
+
 // The rows (yp, z) of a folded lattice sorted by their distance from the x
 // axis (ties by yp, then z): a row's place is the number of rows before it,
 // found for each yp by bisection over z >= 0, along which the distance grows.

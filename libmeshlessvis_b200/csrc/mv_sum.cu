@@ -877,10 +877,14 @@ int launch_plain_sum(const SumRequest& req, Workspace& ws, KernelTimer* timer) {
     // where 32 rows along z read cells far apart, whose bank conflicts bound the
     // kernel wherever h dk spans several cells: 20,011 SPH particles on 100 x 90
     // x 70, 2182 us and 1666 with radii of 0.1 to 0.4 (a cell is h k = 0.017),
-    // 1663 and 1654 with 0.01 to 0.1.  The order costs 5 us, beside the table.
+    // 1663 and 1654 with 0.01 to 0.1.  Small sums and small radii lose by the
+    // order (rows_worth_sorting).
     const long long rows = (long long)yrows * lat.nz;
+    const double cells = req.radius_max >= 0.f
+                             ? (double)req.radius_max * std::max(std::fabs(lat.ky), std::fabs(lat.kz)) / ds
+                             : -1.0;
     const bool sorted = fold_y && amp == kAmpTable && lat.nz > 1 && lat.z0 >= 0 && std::isfinite(lat.ky * lat.ky) &&
-                        std::isfinite(lat.kz * lat.kz);
+                        std::isfinite(lat.kz * lat.kz) && rows_worth_sorting(req.n, cells);
     const size_t rows_bytes = sorted ? (size_t)rows * sizeof(int) : 0;
     int st = ws.reserve(part_bytes + table_bytes + sums_bytes + rows_bytes);
     if (st != kOk) return st;

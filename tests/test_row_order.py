@@ -49,3 +49,18 @@ def test_places_are_a_permutation(tmp_path, flags):
     exe = tmp_path / "check"
     subprocess.run(["g++", "-std=c++17", *flags, f"-I{CSRC}", str(src), "-o", str(exe)], check=True)
     assert int(subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout) == 0
+
+
+def test_small_sums_and_radii_take_the_rows_as_they_lie(tmp_path):
+    """An order that costs more than it saves is not made; particles and table
+    cells a step of k, on both sides of the line, and without a known radius."""
+    src = tmp_path / "check.cpp"
+    src.write_text('#include <cstdio>\n#include "mv_row_order.h"\nint main() {\n'
+                   + "".join(f'std::printf("%d ", mv::rows_worth_sorting({n}, {c}));\n'
+                             for n, c in ((62, 5.8), (62, 23.0), (4000, 1.2), (500, 5.8), (250, 23.0), (20011, 5.8),
+                                          (1, 300.0), (62, -1.0)))
+                   + "}\n")
+    exe = tmp_path / "check"
+    subprocess.run(["g++", "-std=c++17", f"-I{CSRC}", str(src), "-o", str(exe)], check=True)
+    out = subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout.split()
+    assert out == ["0", "0", "0", "0", "1", "1", "1", "1"]
