@@ -19,12 +19,12 @@
 // All image batches are float[images][Nx][Ny] with x slow, as vis_copy_to_host
 // returns them; RGB outputs are float[images][Nx][Ny][3].
 #include <algorithm>
-#include <cfloat>
 #include <cmath>
 #include <cstdio>
 #include <vector>
 
 #include "meshless_vis_b200.h"
+#include "mv_divide.h"
 #include "mv_internal.h"
 
 namespace mv {
@@ -136,14 +136,6 @@ __host__ __device__ inline Knots color_knots(int map) {
                                {{0, 0, 0}, {0.f, 0.004f, 0.686f}, {0.f, 0.42f, 1.f}, {0.f, 0.518f, 1.f}, {1, 1, 1}}};
     return Knots{{0.f, 0.475f, 0.694f, 0.745f, 1.f},
                  {{0, 0, 0}, {0.686f, 0.004f, 0.f}, {1.f, 0.42f, 0.f}, {1.f, 0.518f, 0.f}, {1, 1, 1}}};
-}
-
-// x / c where r = 1 / c, correctly rounded: x r, corrected by its remainder
-// (Markstein's division step), which gives the rounded quotient; infinities and
-// NaNs as x r has them.  c and r have to be normal numbers.
-__device__ __forceinline__ float divide_by(float x, float c, float r) {
-    const float q = x * r, q1 = fmaf(fmaf(-q, c, x), r, q);
-    return fabsf(q1) <= FLT_MAX ? q1 : q;
 }
 
 // The colour map's segments and colours come from shared memory (indexed by

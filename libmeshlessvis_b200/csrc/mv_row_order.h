@@ -3,10 +3,12 @@
 #pragma once
 #include <cmath>
 
+#ifndef MV_HD
 #ifdef __CUDACC__
 #define MV_HD __host__ __device__ __forceinline__
 #else
 #define MV_HD inline
+#endif
 #endif
 
 namespace mv {

@@ -45,3 +45,32 @@ def test_post_at_odd_sizes(count, nx, ny, offset):
                                        d_rgb.data_ptr()) == 0
         np.testing.assert_allclose(rgb(), O.colormap(imgs, -1.0, 9.0, log_scale, color_map), rtol=2e-5, atol=2e-5)
     cfg.close()
+
+
+def _rgb(cfg, call, imgs, *args):
+    import torch
+
+    d_img = torch.from_numpy(imgs).cuda()
+    d_rgb = torch.empty(imgs.shape + (3,), dtype=torch.float32, device="cuda")
+    torch.cuda.synchronize()
+    assert call(cfg.ptr, d_img.data_ptr(), len(imgs), L.int2(*imgs.shape[1:]), *args, d_rgb.data_ptr()) == 0
+    cfg.synchronize()
+    return d_rgb.cpu().numpy()
+
+
+@pytest.mark.parametrize("log_scale,color_map", [(0, 1), (1, 2), (0, 3)])
+@pytest.mark.parametrize("scale", [1.0, 1e-29])
+def test_colormap_of_infinities_nans_and_small_ranges(log_scale, color_map, scale):
+    """Intensities below the range, and NaNs, take the first colour, those above
+    it the last; a range as small as 1e-29 keeps its quotients."""
+    rng = np.random.default_rng(color_map)
+    imgs = (rng.uniform(-1.0, 4.0, (2, 33, 31)) * scale).astype(np.float32)
+    imgs[0, 0, :3] = np.inf, -np.inf, np.nan
+    imgs[1, 32, 30] = np.nan
+    lo, hi = np.float32(0.0), np.float32(3.0 * scale)
+    cfg = M.Config(step=(1.0, 1.0), cutoff=(8, 4), samples=(16, 16), block_length=64)
+    got = _rgb(cfg, M.lib().vis_images_colormap, imgs, float(lo), float(hi), log_scale, color_map)
+    cfg.close()
+    finite = np.where(np.isnan(imgs) | (imgs == -np.inf), np.float32(-1.0 * scale), imgs)
+    finite = np.where(imgs == np.inf, np.float32(9.0 * scale), finite)
+    np.testing.assert_allclose(got, O.colormap(finite, float(lo), float(hi), log_scale, color_map), rtol=2e-5, atol=2e-5)
