@@ -40,7 +40,9 @@ __device__ __forceinline__ float unordered(unsigned int u) {
 }
 
 // One image per blockIdx.y, 16 bytes a load between its unaligned ends; fmaxf
-// passes over NaNs, from the first sample, as the reference's scan does.
+// passes over NaNs, from the first sample, as the reference's scan does.  A block
+// that has none but NaNs (the first sample where it has no pixels of its own) adds
+// nothing; an image of NaNs keeps the start value, which is one.
 __global__ void __launch_bounds__(256) image_max_kernel(const float* __restrict__ img, long long per_image,
                                                         unsigned int* out_max) {
     const float* p = img + (size_t)blockIdx.y * per_image;
@@ -63,7 +65,7 @@ __global__ void __launch_bounds__(256) image_max_kernel(const float* __restrict_
     if (threadIdx.x < 32) {
         float v = threadIdx.x < (blockDim.x >> 5) ? wm[threadIdx.x] : p[0];
         for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-        if (threadIdx.x == 0) atomicMax(out_max + blockIdx.y, ordered(v));
+        if (threadIdx.x == 0 && v == v) atomicMax(out_max + blockIdx.y, ordered(v));
     }
 }
 

@@ -74,3 +74,29 @@ def test_colormap_of_infinities_nans_and_small_ranges(log_scale, color_map, scal
     finite = np.where(np.isnan(imgs) | (imgs == -np.inf), np.float32(-1.0 * scale), imgs)
     finite = np.where(imgs == np.inf, np.float32(9.0 * scale), finite)
     np.testing.assert_allclose(got, O.colormap(finite, float(lo), float(hi), log_scale, color_map), rtol=2e-5, atol=2e-5)
+
+
+@pytest.mark.parametrize("shape", [(2, 25, 41), (1, 3, 683), (2, 64, 64), (3, 5, 7)])
+@pytest.mark.parametrize("where", ["first", "first rows", "all", "infinite"])
+def test_maximum_passes_over_nans(shape, where):
+    """The scan from the first sample on passes over NaNs, also where a block has
+    no pixels but the first sample (1025 and 2049 of them); an image of NaNs has
+    none other, and an infinite maximum leaves zeros."""
+    rng = np.random.default_rng(shape[2])
+    imgs = rng.uniform(-1.0, 9.0, shape).astype(np.float32)
+    if where == "first":
+        imgs[:, 0, 0] = np.nan
+    elif where == "first rows":
+        imgs[:, :2] = np.nan
+    elif where == "all":
+        imgs[-1] = np.nan
+    else:
+        imgs[:, -1, -1] = np.inf
+    cfg = M.Config(step=(1.0, 1.0), cutoff=(8, 4), samples=(16, 16), block_length=64)
+    got = _rgb(cfg, M.lib().vis_images_normalize_to_rgb, imgs)
+    cfg.close()
+    expected = np.empty(shape)
+    for e, img in zip(expected, imgs.astype(np.float64)):
+        m = np.nan if np.isnan(img).all() else np.nanmax(img)
+        e[:] = np.divide(np.maximum(img, 0.0), m, out=np.full(img.shape, np.nan), where=img < np.inf)
+    np.testing.assert_allclose(got, np.repeat(expected[..., None], 3, axis=3), rtol=1e-6, atol=1e-7)
