@@ -23,6 +23,8 @@
 // 384 x 384 from 384^3, turning about y: 412 us with a thread an element in
 // output order and every corner read, 302 with two lanes a sample (the corners
 // at l and at l + 1; fewer lookups, more instructions), 266 us so.
+#include <algorithm>
+
 #include "mv_internal.h"
 
 namespace mv {
@@ -101,11 +103,13 @@ __device__ __forceinline__ void slice_tile(const SliceAt& s, int tile_x, int til
         if (x0 + tx < nx && y0 + ty < h) out[(size_t)(x0 + tx) * h + y0 + ty] = s_tile[ty][tx];
 }
 
-__global__ void __launch_bounds__(kThreads) slice_extract_kernel(SliceRequest r) {
+// Tiles from (first_x, first_y) on.
+__global__ void __launch_bounds__(kThreads) slice_extract_kernel(SliceRequest r, int first_x, int first_y) {
     const int view = blockIdx.x;
     const float* v = r.views + 8 * view;
     const SliceAt s = {r.spectrum, r.gx, r.gy, r.gz / 2 + 1, r.inv_step, v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7]};
-    slice_tile(s, blockIdx.z, blockIdx.y, r.cx, r.cy, r.nx, r.ny, r.arranged + (size_t)view * r.nx * (r.ny / 2 + 1));
+    slice_tile(s, first_x + blockIdx.z, first_y + blockIdx.y, r.cx, r.cy, r.nx, r.ny,
+               r.arranged + (size_t)view * r.nx * (r.ny / 2 + 1));
 }
 
 // Batched form: every view has its own spectrum and image size; a block finds
@@ -145,10 +149,17 @@ int launch_slice_extract_batch(const SliceView* d_views, int number_of_views, lo
 int launch_slice_extract(const SliceRequest& req, KernelTimer* timer) {
     const int tiles_x = (req.nx + kTileX - 1) / kTileX, tiles_y = (req.ny / 2 + 1 + kTileY - 1) / kTileY;
     if (req.number_of_views <= 0 || tiles_x <= 0 || tiles_y <= 0) return kOk;
-    if (tiles_x > 65535 || tiles_y > 65535) return set_error(kInvalidValue, "too many slice samples");
+    if ((long long)req.nx * (req.ny / 2 + 1) * req.number_of_views > (1LL << 40))
+        return set_error(kInvalidValue, "too many slice samples");
     timer_begin(timer, 1, req.stream);
-    slice_extract_kernel<<<dim3((unsigned)req.number_of_views, tiles_y, tiles_x), kThreads, 0, req.stream>>>(req);
-    count_launch();
+    // one launch; images of more tiles than a grid's y or z holds take several
+    constexpr int kMost = 65535;
+    for (int x = 0; x < tiles_x; x += kMost)
+        for (int y = 0; y < tiles_y; y += kMost) {
+            const dim3 grid((unsigned)req.number_of_views, std::min(kMost, tiles_y - y), std::min(kMost, tiles_x - x));
+            slice_extract_kernel<<<grid, kThreads, 0, req.stream>>>(req, x, y);
+            count_launch();
+        }
     timer_end(timer, 1, req.stream);
     return check_cuda(cudaGetLastError(), "slice_extract_kernel launch");
 }
