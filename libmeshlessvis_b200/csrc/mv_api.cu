@@ -199,21 +199,24 @@ GroupStats host_statistics(const Group& grp) {
 
 // The same from the device copies, for groups of at least kDeviceStats terms:
 // registering 30,011 particles with radii took 340 us, most of it one host
-// thread's passes over them.  `scratch` holds a RegisterStats and a histogram.
+// thread's passes over them.  `scratch` holds a RegisterStats and a histogram a
+// group.
 constexpr int kDeviceStats = 8192;
 
-int device_statistics(const std::vector<Group*>& groups, Workspace& scratch, cudaStream_t stream,
+size_t statistics_extremes_bytes(size_t groups) { return (groups * sizeof(RegisterStats) + 255) / 256 * 256; }
+size_t statistics_bytes(size_t groups) {
+    return statistics_extremes_bytes(groups) + groups * register_histogram_bytes();
+}
+
+int device_statistics(const std::vector<Group*>& groups, void* scratch, cudaStream_t stream,
                       std::vector<GroupStats>& out) {
     const size_t n = groups.size();
     out.assign(n, GroupStats{});
     if (n == 0) return kOk;
-    const size_t extremes_bytes = (n * sizeof(RegisterStats) + 255) / 256 * 256;
-    int st = scratch.reserve(extremes_bytes + n * register_histogram_bytes());
-    if (st != kOk) return st;
-    RegisterStats* d_ext = static_cast<RegisterStats*>(scratch.ptr);
-    char* d_hist = static_cast<char*>(scratch.ptr) + extremes_bytes;
+    RegisterStats* d_ext = static_cast<RegisterStats*>(scratch);
+    char* d_hist = static_cast<char*>(scratch) + statistics_extremes_bytes(n);
     std::vector<RegisterStats> ext(n);
-    st = launch_register_extremes_clear(d_ext, (int)n, stream);
+    int st = launch_register_extremes_clear(d_ext, (int)n, stream);
     for (size_t i = 0; i < n && st == kOk; ++i)
         st = launch_register_extremes(reinterpret_cast<const float4*>(groups[i]->d_constraints), groups[i]->d_radii,
                                       groups[i]->number_of_terms, d_ext + i, stream);
@@ -305,6 +308,8 @@ int registration_pool(cudaMemPool_t* pool) {
 struct RegistrationCache {
     std::map<size_t, std::deque<void*>> blocks;
     size_t held = 0, live = 0, peak = 0;
+    void* scratch = nullptr;  // of the statistics, kept for the next registration
+    size_t scratch_bytes = 0;
 
     void* take(size_t bytes) {
         auto it = blocks.find(bytes);
@@ -341,10 +346,25 @@ struct RegistrationCache {
             for (void* p : kv.second) cudaFreeAsync(p, stream);
         blocks.clear();
         held = live = peak = 0;
+        if (scratch) cudaFreeAsync(scratch, stream);
+        scratch = nullptr;
+        scratch_bytes = 0;
     }
 };
 
 namespace {
+int pool_alloc(void** p, size_t bytes, cudaStream_t stream) {
+    *p = nullptr;
+    cudaMemPool_t pool;
+    const int st = registration_pool(&pool);
+    if (st != kOk) return st;
+    const cudaError_t e = cudaMallocFromPoolAsync(p, bytes, pool, stream);
+    if (e == cudaSuccess) return kOk;
+    *p = nullptr;
+    cudaGetLastError();
+    return check_cuda(e, "cudaMallocFromPoolAsync");
+}
+
 template <typename T>
 int registration_alloc(T** p, size_t count, RegistrationCache& cache, cudaStream_t stream) {
     *p = nullptr;
@@ -355,17 +375,23 @@ int registration_alloc(T** p, size_t count, RegistrationCache& cache, cudaStream
         cache.registered(bytes, stream);
         return kOk;
     }
-    cudaMemPool_t pool;
-    int st = registration_pool(&pool);
+    void* q = nullptr;
+    const int st = pool_alloc(&q, bytes, stream);
     if (st != kOk) return st;
-    cudaError_t e = cudaMallocFromPoolAsync((void**)p, bytes, pool, stream);
-    if (e != cudaSuccess) {
-        *p = nullptr;
-        cudaGetLastError();
-        return check_cuda(e, "cudaMallocFromPoolAsync");
-    }
+    *p = static_cast<T*>(q);
     cache.registered(bytes, stream);
     return kOk;
+}
+
+// The statistics' scratch: from the pool too, so that a config's first
+// registration waits for no cudaMalloc of its own.
+int registration_scratch(RegistrationCache& cache, size_t bytes, cudaStream_t stream) {
+    if (bytes <= cache.scratch_bytes) return kOk;
+    if (cache.scratch) cudaFreeAsync(cache.scratch, stream);
+    cache.scratch_bytes = 0;
+    const int st = pool_alloc(&cache.scratch, bytes, stream);
+    if (st == kOk) cache.scratch_bytes = bytes;
+    return st;
 }
 }  // namespace
 
@@ -809,7 +835,9 @@ void vis_register_meshless_dataset(VisConfig* c, MeshlessDataset* ds) {
     for (int g = 0; g < ds->number_of_groups; ++g)
         if (!copy_group(ds->groups[g])) break;
     std::vector<GroupStats> stats;
-    if (device_statistics(large, s->post, s->stream, stats) != kOk) return;
+    if (registration_scratch(s->registrations, statistics_bytes(large.size()), s->stream) != kOk ||
+        device_statistics(large, s->registrations.scratch, s->stream, stats) != kOk)
+        return;
     {
         std::lock_guard<std::mutex> lock(g_stats_mu);
         for (size_t i = 0; i < large.size(); ++i) g_stats[large[i]->d_constraints] = stats[i];

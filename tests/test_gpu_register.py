@@ -59,3 +59,62 @@ def test_groups_before_a_refused_one_keep_their_statistics(n):
     assert cfg.kernel_time(3)[1] > 0  # launches of the tensor kernel
     sp.close()
     cfg.close()
+
+
+def test_a_new_config_registers_without_mapping_memory():
+    """Registered blocks and the statistics' scratch come from the library's
+    pool, which keeps what an earlier config gave back: registering the same
+    sizes again maps none."""
+    import torch
+
+    rng = np.random.default_rng(3)
+    n = 8192
+    cons = constraints(rng.random((n, 3), dtype=np.float32), rng.standard_normal(n).astype(np.float32))
+    radii = rng.uniform(0.01, 0.05, n).astype(np.float32)
+
+    def mapped():
+        cfgs = [M.Config(cutoff=(8, 8), samples=(16, 16), block_length=64) for _ in range(8)]
+        sets = [M.Dataset([(cons, radii, M.WENDLAND_D3_C2)]) for _ in cfgs]
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        for cfg, ds in zip(cfgs, sets):
+            cfg.register(ds)
+        torch.cuda.synchronize()
+        used = before - torch.cuda.mem_get_info()[0]
+        for cfg, ds in zip(cfgs, sets):
+            cfg.unregister(ds)
+            cfg.close()
+        return used
+
+    mapped()
+    assert mapped() == 0
+
+
+@pytest.mark.parametrize("what", ["weight", "first radius", "radius", "infinite radius", "infinite weight"])
+def test_host_and_device_statistics_agree_on_nans_and_infinities(what):
+    """A set of 8191 terms (host) and the same with one of weight zero more
+    (device) take the same route: the same elements are no numbers, or both are
+    refused alike."""
+    rng = np.random.default_rng(11)
+    n = 8192
+    weights = rng.standard_normal(n).astype(np.float32)
+    radii = np.exp(rng.uniform(np.log(0.01), np.log(0.05), n)).astype(np.float32)
+    weights[n - 1] = 0.0
+    {"weight": weights, "first radius": radii, "radius": radii, "infinite radius": radii, "infinite weight": weights}[what][
+        0 if what == "first radius" else 4000] = np.inf if "infinite" in what else np.nan
+    points = rng.random((n, 3), dtype=np.float32)
+
+    def outcome(count):
+        cons = constraints(points[:count], weights[:count])
+        try:
+            spec, images = spectrum_and_views([(cons, radii[:count], M.WENDLAND_D3_C2)], (32, 32, 32), 1.0, (1.0, 1.0),
+                                              (16, 16), (32, 32), [((1, 0, 0), (0, 1, 0))], M.FORM_AUTO)
+            return np.isfinite(spec), np.isfinite(images)
+        except M.VisError as e:
+            return str(e)
+
+    host, device = outcome(n - 1), outcome(n)
+    if isinstance(host, str) or isinstance(device, str):
+        assert host == device
+    else:
+        assert all(np.array_equal(h, d) for h, d in zip(host, device))
