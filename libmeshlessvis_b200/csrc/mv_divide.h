@@ -15,16 +15,23 @@
 namespace mv {
 
 // x / c where r = 1 / c, correctly rounded: x r, corrected by its remainder
-// (Markstein's division step), which gives the rounded quotient; infinities and
-// NaNs as x r has them.  c and r have to be normal numbers.  The remainder has
-// to be exact: below 2^-80, where it may lie between the least subnormal
-// numbers (x from 2^-108 down at c = 1e-29 gave other quotients), and for
-// quotients that small, the division itself.
-MV_HD float divide_by(float x, float c, float r) {
+// (Markstein's division step), which gives the rounded quotient.  c and r have to
+// be normal numbers, the quotient finite and the remainder exact: x = 0 or |x| and
+// |x / c| at least 2^-80 (from 2^-108 down it may lie between the least subnormal
+// numbers, and the quotient be another).
+MV_HD float divide_finite(float x, float c, float r) {
     const float q = x * r;
-    if (fminf(fabsf(x), fabsf(q)) < 0x1p-80f && x != 0.f) return x / c;
-    const float q1 = fmaf(fmaf(-q, c, x), r, q);
-    return fabsf(q1) <= FLT_MAX ? q1 : q;
+    return fmaf(fmaf(-q, c, x), r, q);
 }
+
+// The same of any x; infinities and NaNs as x r has them.
+MV_HD float divide_by(float x, float c, float r) {
+    const float q = divide_finite(x, c, r);
+    return fabsf(q) <= FLT_MAX ? q : x * r;
+}
+
+// From which x on divide_by(x, c, 1 / c) holds, 0 < c < 1e30, and for its
+// quotient as x again, c then from 2^-20 to 1.
+MV_HD float divide_by_least(float c) { return fmaxf(0x1p-80f, c * 0x1p-79f); }
 
 }  // namespace mv

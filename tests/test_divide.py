@@ -1,7 +1,7 @@
 """Division by a shared divisor (csrc/mv_divide.h) has the bits of the division
-itself: its own code, compiled for the host, over mantissas, exponents, signs,
-zeros, infinities and NaNs, for the colour map's divisors and ranges of images
-from 1e-29 to 1e29."""
+itself where the colour map uses it: its own code, compiled for the host, for
+ranges of images from 1e-29 to 1e29 and the map's own divisors after them, over
+mantissas, exponents, infinities and NaNs."""
 import subprocess
 from pathlib import Path
 
@@ -22,24 +22,30 @@ static float number(uint32_t u) { float f; std::memcpy(&f, &u, 4); return f; }
 static bool same(float a, float b) { return a == b || (a != a && b != b); }
 
 int main() {
-    const float colour[] = {0.25f, 0.475f, 0.694f - 0.475f, 0.745f - 0.694f, 1.f - 0.745f,
-                            std::log(0.011f) - std::log(1e-3f)};
+    const float colour[] = {0.25f, 0.475f, 0.694f - 0.475f, 0.745f - 0.694f, 1.f - 0.745f};
     uint32_t seed = 1;
     auto random = [&seed] { return seed = seed * 1664525u + 1013904223u, seed >> 9; };
     long long wrong = 0;
-    auto check = [&wrong](float x, float c) {
-        for (float s : {x, -x}) wrong += !same(mv::divide_by(s, c, 1.f / c), s / c);
-    };
-    const float inf = std::numeric_limits<float>::infinity();
-    auto divisor = [&](float c) {
-        for (int e = -149; e <= 127; ++e)
-            for (int i = 0; i < 2000; ++i) check(std::ldexp(number(0x3f800000u | random()), e), c);
-        for (float x : {0.f, inf, std::numeric_limits<float>::quiet_NaN(), 1e-45f, 1e-38f, 3e38f}) check(x, c);
-    };
-    for (float c : colour) divisor(c);
-    for (int e = -96; e <= 96; e += 4) divisor(std::ldexp(number(0x3f800000u | random()), e));
+    auto check = [&wrong](float x, float c) { wrong += !same(mv::divide_by(x, c, 1.f / c), x / c); };
+    auto weight = [&wrong](float x, float c) { wrong += !same(mv::divide_finite(x, c, 1.f / c), x / c); };
+    const float inf = std::numeric_limits<float>::infinity(), log_range = std::log(0.011f) - std::log(1e-3f);
+    for (int e = -96; e <= 96; ++e) {
+        const float range = std::ldexp(number(0x3f800000u | random()), e), least = mv::divide_by_least(range);
+        for (float x : {0.f, least, 3e38f, inf, std::numeric_limits<float>::quiet_NaN()}) check(x, range);
+        for (int f = -149; f <= 127; ++f)
+            for (int i = 0; i < 1000; ++i) {
+                const float x = std::ldexp(number(0x3f800000u | random()), f);
+                if (x < least) continue;
+                check(x, range);
+                const float a = x / range;
+                if (a > 1.f) continue;
+                for (float c : colour) weight(a, c);
+            }
+    }
     for (float c : colour)  // every mantissa
-        for (uint32_t m = 0; m < 1u << 23; ++m) check(number(0x3f800000u | m), c);
+        for (uint32_t m = 0; m < 1u << 23; ++m) weight(number(0x3f800000u | m), c);
+    for (uint32_t m = 0; m < 1u << 23; ++m)
+        for (float x : {number(0x3f800000u | m), std::ldexp(number(0x3f800000u | m), -22)}) check(x, log_range);
     std::printf("%lld\n", wrong);
     return 0;
 }
