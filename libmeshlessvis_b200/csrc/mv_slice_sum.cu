@@ -32,6 +32,7 @@
 
 #include "mv_device.cuh"
 #include "mv_internal.h"
+#include "mv_split_rules.h"
 
 namespace mv {
 namespace {
@@ -505,36 +506,6 @@ __global__ void __launch_bounds__(32 * kFinalWarps) slice_finalize_kernel(SliceF
     }
 }
 
-// Particles a split, in units of 64; more than a tile (4 units) in whole tiles.
-// The least of the blocks' work an SM (which 60% of its resident blocks keep
-// busy), half a block's time for the last wave, a block's start (half a unit)
-// and the splits' partial sums to write and reduce (0.005 units a block of
-// them, 5 us a unit).
-// A set of few tiles is so cut to fill the chip: 4096 particles on 64 x 64 took
-// 43 us in 16 blocks of a tile, 5 in 64; 100,003 on 256 x 128 took 1.21 ms in
-// one wave of 833 blocks of 8 tiles, whose SMs held 5 or 6.
-int split_chunk(int n, long long blocks, size_t plane, int resident) {
-    constexpr int kUnit = 64, kUnits = kThreads / kUnit;
-    constexpr double kMostPartial = 256e6;  // bytes of partial sums
-    const double sms = device_sm_count();
-    const long long units = std::max<long long>(1, ((long long)n + kUnit - 1) / kUnit);
-    const long long most = (units + kUnits - 1) / kUnits * kUnits;  // one split
-    long long chosen = most;
-    double best_cost = 1e300;
-    for (long long per = 1; per <= most; per += per < kUnits ? 1 : std::max<long long>(kUnits, per / 4 / kUnits * kUnits)) {
-        const long long splits = (units + per - 1) / per;
-        if (splits > 65535 || (splits > 1 && (double)splits * (double)plane * sizeof(float2) > kMostPartial)) continue;
-        const double an_sm = (double)blocks * (double)splits / sms;
-        const double cost = std::max(an_sm, 0.6 * resident) * ((double)per + 0.5) +
-                            0.5 * (double)per * std::min<double>(resident, an_sm) + 0.005 * (double)(blocks * splits);
-        if (cost < best_cost) {
-            best_cost = cost;
-            chosen = per;
-        }
-    }
-    return (int)(chosen * kUnit);
-}
-
 }  // namespace
 
 int launch_slice_sum(const SumRequest& req, int nx, int ny, Workspace& ws, KernelTimer* timer) {
@@ -607,13 +578,14 @@ int launch_slice_sum(const SumRequest& req, int nx, int ny, Workspace& ws, Kerne
             }
         }
         if (blocks > INT32_MAX) return set_error(kInvalidValue, "slice too large");
-        a.chunk = split_chunk(req.n, blocks, a.plane, resident);
+        const size_t partial_bytes = a.plane * sizeof(float2);  // of a split
+        const size_t split_sums = (size_t)(by_table ? 4 * kL : 32) * (size_t)blocks * threads * sizeof(double2);
+        a.chunk = slice_chunk(req.n, kThreads, blocks, partial_bytes, split_sums, resident, device_sm_count());
         splits = (int)(((long long)req.n + a.chunk - 1) / a.chunk);
         if (splits > 65535) return set_error(kInvalidValue, "slice sum: too many splits");
-        const size_t part_bytes = (a.plane * splits * sizeof(float2) + 255) / 256 * 256;
+        const size_t part_bytes = (splits * partial_bytes + 255) / 256 * 256;
         const size_t table_bytes = by_table ? ((size_t)(a.table_n + 1) * sizeof(float4) + 255) / 256 * 256 : 0;
-        const size_t sums_bytes =
-            a.chunk > kThreads ? (size_t)splits * (by_table ? 4 * kL : 32) * (size_t)blocks * threads * sizeof(double2) : 0;
+        const size_t sums_bytes = a.chunk > kThreads ? splits * split_sums : 0;
         st = ws.reserve(part_bytes + table_bytes + sums_bytes);
         if (st != kOk) return st;
         char* base = static_cast<char*>(ws.ptr);
