@@ -67,8 +67,8 @@ def sum_terms_split(w):
 
 # DRAM bytes (read + write) per launch of the dominant kernel, from ncu
 # captures of dram__bytes_read.sum + dram__bytes_write.sum of the full-size
-# launch (profiles/tc_sum_kernel_c3_dram.md names the capture and its
-# command); None where no capture exists.
+# launch, taken on 2^20 Gaussians and 256^3 with a one-pass ncu run of this
+# benchmark; None where no capture exists.
 DRAM_TRAFFIC_PER_LAUNCH = {("C3", "tc_sum_kernel"): 14.08e9 + 1.43e9}
 
 

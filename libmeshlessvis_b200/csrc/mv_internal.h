@@ -488,8 +488,8 @@ enum TileShape : int {
 struct TuneParams {
     int plain_waves = 6;  // plain form: split-K until the grid holds ~plain_waves blocks per SM
     int tc_waves = 4;     // tensor form: particle splits until the items make ~tc_waves waves
-    int tc_flush = 16;    // tensor form, single-accumulator tiles: stages per TMEM chain (8 or 16;
-                          // the double-buffered 128x128 tile uses at most 8)
+    int tc_flush = 16;    // tensor form, Gaussian jobs of more than 64 columns: stages per TMEM chain
+                          // (8 or 16; other jobs and the tiles of 64 columns use at most 8)
     int hbin_job_cost = 1024;  // h-binned groups: cost of one more bin (a job), in particle x n-tile units
     int hbin_block_cost = 0;  // h-binned groups: cost of one more Chebyshev block (the reduction), same units
     int tc_shapes = kTileAll;  // tensor form: the tile shapes the planner may use (TileShape bits)

@@ -147,13 +147,14 @@ __host__ __device__ inline Knots color_knots(int map) {
 // for 360 images of 384 x 384, where their bytes take 0.13).  The divisors are
 // the same for all pixels, their reciprocals are taken once a thread: with four
 // full divisions a pixel the instructions bounded the kernel: 413 us with the
-// normalisation of the same images, 395 so (the colour map 203).  Pixels too near
-// the range's start for that are divided: 208 us, at 8 blocks an SM (225 at the 40
-// registers that it would take without the bound; a factor on all numbers in
-// place of the test, 209, or 197 without the logarithm, where the test takes 192).
+// normalisation of the same images, 380 so (the colour map alone 203).  Pixels
+// too near the range's start for that are divided: 208 us, at 8 blocks an SM (225
+// at the 40 registers that it would take without the bound; a factor on all
+// numbers in place of the test, 209, or 197 without the logarithm, where the test
+// takes 192).
 __global__ void __launch_bounds__(kRgbThreads, 8) colormap_kernel(const float* __restrict__ img, long long count,
-                                                               float imin, float imax, int log_scale, Knots k,
-                                                               float* __restrict__ rgb) {
+                                                                  float imin, float imax, int log_scale, Knots k,
+                                                                  float* __restrict__ rgb) {
     __shared__ float4 s_out[3 * kRgbThreads];
     __shared__ float4 s_x[8];     // segment up to knot i: its ends, length, 1 / length
     __shared__ float4 s_c[8];     // colours of the knots

@@ -22,7 +22,9 @@
 // through shared memory as 64-byte pieces of the y-fast layout.  360 views of
 // 384 x 384 from 384^3, turning about y: 412 us with a thread an element in
 // output order and every corner read, 302 with two lanes a sample (the corners
-// at l and at l + 1; fewer lookups, more instructions), 266 us so.
+// at l and at l + 1; fewer lookups, more instructions), 242 us so.  Turning about
+// y half of the corners have weight 0; about a tilted axis it was 405 us and is
+// 338, at random attitudes 395 and 366.
 #include <algorithm>
 
 #include "mv_internal.h"

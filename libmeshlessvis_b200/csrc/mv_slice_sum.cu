@@ -21,10 +21,10 @@
 // Other slices (SPH or Wendland with varying radii, cx != cy or two steps) take
 // the folded plain form.
 //
-// Both split the particles over blocks until the chip is full, down to one
-// 256-particle tile a block (the plain form's four leave a small slice on a few
-// SMs); a tile is summed in FP32 registers, tiles in FP64 running sums in global
-// scratch (none for blocks of one tile), splits in FP64 by the finalize.
+// Both split the particles over blocks until the chip is full, down to 64 a block
+// (the plain form's four tiles of 256 leave a small slice on a few SMs); a tile is
+// summed in FP32 registers, tiles in FP64 running sums in global scratch (none
+// for blocks of one tile), splits in FP64 by the finalize.
 #include <algorithm>
 #include <cmath>
 #include <string>

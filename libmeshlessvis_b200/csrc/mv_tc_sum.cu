@@ -37,7 +37,8 @@
 // the accumulator into an FP32 total in the other 256 TMEM columns, with the
 // mean of what the tensor core's truncation took from it (kChainGain: where the
 // error grew with the chain, to 4.1e-6 rel-L2 at 16 stages, it is 0.4 to 2.9e-6
-// at the 8 and 16 stages in use).  A work item
+// at the 8 and 16 stages in use on sets of up to 2^20 particles; 4.1e-6 on 2^24
+// and 384^3).  A work item
 // (one particle range of one tile) owns a slot of global memory: at its end
 // an item of at most kMaxItemChains chains stores its FP32 total there once,
 // and a longer item adds its FP32 total of every kMaxItemChains chains into
@@ -1437,7 +1438,7 @@ struct TcCoefArgs {
     double step;
     int nbins;
     int nsq;               // |k|^2 / step^2 = 0 .. nsq - 1
-    int coef_stride;       // floats per |k|^2: the group's Chebyshev blocks over all bins, padded to fours
+    int coef_stride;       // floats per |k|^2: the group's Chebyshev blocks over all bins, padded to whole lines of 32
     const int4* bins;      // (first block, capacity, first Chebyshev block, order)
     const float4* spans;   // (lo, hi, ...)
     const float* edges;    // the bins' classification edges
@@ -2163,8 +2164,9 @@ bool binned_group(const SumRequest& r) {
 }
 
 // The automatic choice takes the h-binned tensor form while its work (terms x
-// mean Chebyshev order) stays below what the plain form costs, which does
-// about a tenth of the tensor form's terms per second.
+// mean Chebyshev order) stays well below what the plain form costs, which does
+// about a twentieth of the tensor form's terms per second (4,990 and 109,935
+// GTerms/s on 2^20 Gaussians and 256^3).
 constexpr double kHBinAutoMaxCost = 6.0;
 
 }  // namespace
@@ -2209,8 +2211,8 @@ struct ClassKey {
 int tensor_plan(const std::vector<SumRequest>& groups, TensorPlan& plan) {
     plan = TensorPlan{};
     std::vector<ClassKey> keys;
-    // (tile mode, cost, item): kNarrow items first, then kPair, then kWide;
-    // each mode longest first
+    // (tile mode, cost, item); mode by mode, each longest first (a launch a
+    // mode, the launches by their units' load)
     struct Item {
         int mode;
         long long cost;
@@ -2552,8 +2554,8 @@ int tensor_plan(const std::vector<SumRequest>& groups, TensorPlan& plan) {
         }
     }
     if (items.size() > (size_t)INT32_MAX) return set_error(kInvalidValue, "tensor sum: too many work items");
-    // Per tile mode, longest first (round-robin over the persistent CTAs /
-    // pairs), in cost classes 5% wide.  Within a class, items run in blocks of
+    // Per tile mode, longest first (each to the unit with the least to do,
+    // below), in cost classes 5% wide.  Within a class, items lie in blocks of
     // as many m-tiles as there are resident units: one wave takes one (job,
     // split) over distinct m-tiles, all of them reading the same B-operand
     // stages (images) at about the same time, and the next waves the other
